@@ -113,7 +113,8 @@ def draw(rng):
     if family == "batch":
         return {"family": family, "instances": round(_log(rng, 20, 160)), "mix": rng.randint(100, 9999)}
     if family == "komega":
-        return {"family": family, "sensors": _smooth(rng, 64, 4096), "samples": _smooth(rng, 256, 8192, even=True)}
+        return {"family": family, "sensors": 4096 if rng.random() < 0.1 else _smooth(rng, 64, 2560),
+                "samples": _smooth(rng, 256, 8192, even=True)}
     length = _smooth(rng, 64, 4096)
     return {"family": family, "count": _count(rng, length, 1 << 13, 1 << 21), "length": length, "dir": way}
 
