@@ -105,10 +105,12 @@ struct Job {
     const void *twg = nullptr;    // per-pass twiddle tables of the general kernel's schedule
     const void *pc = nullptr;     // per-pass constants of that schedule (PassConst)
     const void *twdd = nullptr;   // per-pass double-float twiddles of the FP64 form (or null)
+    const struct DifTab *dif = nullptr;  // schedule and tables of the in-place mixed-radix kernel (or null)
     int npass = 0;
     int radix[40];
     int form = 0;        // JVSIP_FORM_* of the plan
     bool no_fast = false;      // JVSIP_GPU_NO_FAST at plan creation: general kernels only
+    bool no_dif = false;       // the plan's tuned schedule or shape belongs to the shared-memory kernel
     bool no_pipeline = false;  // JVSIP_GPU_NO_PIPELINE at plan creation: one staging copy each way
     int tuned_vpb = 0, tuned_emax = 0;  // the plan's tuned shared-memory kernel shape (0: automatic)
     int tma_columns = -1;      // JVSIP_GPU_TMA_COLUMNS at plan creation: 1 / 0 force TMA-staged
@@ -179,6 +181,25 @@ constexpr long kLongFewMin = 8192;
 // mixed (2187 x 1024: 1.07x, 2560 x 1024: 0.91x, 2400 x 512: 0.70x).
 constexpr long kColStepsMin = 3000;
 
+// Schedule and device tables of the in-place mixed-radix kernel for one length
+// and precision, shared by the plans of the length (jv_dif.cu).
+struct DifTab {
+    long N = 0;
+    int prec = P_F32;
+    int cls = 0;              // 0: c2c, 1: R2C, 2: C2R (the pair pass bounds a radix)
+    std::vector<int> radix;   // in pass order
+    long P1 = 0;              // shared-memory pitch of a first-pass block
+    std::vector<int> two;     // start of each pass's twiddle table
+    void *d_tw = nullptr;
+    long vpb = 1;             // CTA shape of row calls: transforms, threads
+    int nthr = 128;
+    int refs = 0;
+};
+const DifTab *dif_acquire(long N, int prec, int cls);  // nullptr: no schedule for N (or no memory)
+void dif_release(const DifTab *t);
+bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1);
+bool launch_dif_f32(const Job &j, cudaStream_t s);  // false when the call does not qualify
+
 // Kernel entry points (defined in the kernel translation units).
 bool launch_smem_f32(const Job &j, cudaStream_t s);
 bool launch_smem_f64(const Job &j, cudaStream_t s);
@@ -231,6 +252,7 @@ struct Plan {
     int hint = 0;
     int form = 0;             // JVSIP_FORM_*
     bool no_fast = false;     // environment switches read once at creation
+    bool no_dif = false;      // tuned schedule or CTA shape of the shared-memory kernel
     bool no_pipeline = false;
     int tma_columns = -1;
     int tuned_vpb = 0;        // tuned transforms per CTA of the shared-memory kernel (0: heuristic)
@@ -244,6 +266,7 @@ struct Plan {
     void *d_twg = nullptr;    // per-pass [r][m] twiddle tables of the general kernel's schedule
     void *d_pc = nullptr;     // per-pass constants of that schedule (PassConst, one per pass)
     void *d_twdd = nullptr;   // per-pass double-float tables of the FP64 form (built by setform_d)
+    const DifTab *dif = nullptr;  // the in-place mixed-radix kernel's schedule and tables (or null)
     std::vector<unsigned long> jofk;  // reference digit-reversal map (kept for parity checks)
     std::vector<CallGraph> graphs;    // captured calls (ntimes == 0), most recent last
     bool single = false;      // a single-FFT plan (vsip_fft_*: one row, vector views)

@@ -1,0 +1,388 @@
+// jv_dif.cu -- host side of the in-place mixed-radix kernel (jv_dif.cuh): the
+// radix schedule and shared-memory pitch of a length (dif_shape), its twiddle
+// tables (shared by all plans of the length) and the launchers.
+#include <math.h>
+#include <stdio.h>
+#include <stdlib.h>
+#include <string.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <tuple>
+
+#include "jv_dif.cuh"
+
+namespace jv {
+
+// arithmetic instructions per point of a codelet, R = 0..16
+static const double kDifCost[17] = {0,   0,    2.0,  4.0,  4.0,  7.2,  7.3, 9.4, 7.0,
+                                    9.8, 10.8, 13.6, 10.0, 15.7, 13.1, 13.3, 10.0};
+
+// Cost of a radix-R pass in issue slots per point: the butterfly, and beside
+// it the shared-memory accesses, addresses and twiddles (single precision) or
+// the twiddles alone (double precision, bound by its FP64 pipe); per butterfly
+// the index arithmetic.
+static double pass_cost(int R, int prec) {
+    return prec == P_F32 ? kDifCost[R] + 10.0 + 20.0 / R : kDifCost[R] + 4.5;
+}
+
+// multisets of codelet radices (descending) with product n
+static void multisets(long n, int maxr, std::vector<int> &cur, std::vector<std::vector<int>> &out) {
+    if (n == 1) {
+        if (cur.size() >= 2 && (int)cur.size() <= kDifMaxPass) out.push_back(cur);
+        return;
+    }
+    if ((int)cur.size() >= kDifMaxPass) return;
+    for (int R = std::min<long>(maxr, n); R >= 2; R--) {
+        if (n % R) continue;
+        cur.push_back(R);
+        multisets(n / R, R, cur, out);
+        cur.pop_back();
+    }
+}
+
+// shared-memory wavefronts of the middle (read and write) and last passes of
+// schedule r with block pitch P1, sampled over groups of W lanes (W slots of
+// one element each make a wavefront)
+static long bank_waves(const std::vector<int> &r, long N, long P1, int W) {
+    const int np = (int)r.size();
+    long waves = 0;
+    long M = N / r[0];
+    for (int p = 1; p < np; p++) {
+        const bool last = p == np - 1;
+        const long S = last ? 1 : M / r[p], NR = N / r[p], NB1 = N / r[0] / r[p];
+        const long ngr = (NR + W - 1) / W, take = std::min<long>(ngr, 12);
+        for (long g = 0; g < take; g++) {
+            const long b0 = g * ngr / take * W;
+            int hit[16] = {0};
+            int worst = 0;
+            for (long b = b0; b < std::min(b0 + W, NR); b++) {
+                long pos;
+                if (last) {
+                    long rem = b / r[0];
+                    pos = (b % r[0]) * P1;
+                    long Sq = N / r[0];
+                    for (int i = 1; i + 1 < np; i++) {
+                        Sq /= r[i];
+                        pos += (rem % r[i]) * Sq;
+                        rem /= r[i];
+                    }
+                } else {
+                    const long k1 = b / NB1, u = b % NB1;
+                    pos = k1 * P1 + u + (u / S) * (M - S);
+                }
+                worst = std::max(worst, ++hit[pos % W]);
+            }
+            waves += (last ? 1 : 2) * worst * ngr / take * r[p];
+        }
+        M = S;
+    }
+    return waves;
+}
+
+// The schedule of length N: the multiset of radices of least cost, in the
+// order and with the block pitch of the fewest shared-memory wavefronts
+// (larger first radices on ties).  Real transforms' pair pass (the last of
+// R2C, the first of C2R) takes a radix of at most kDifPairMax.  False when N
+// has a prime above 13 or fewer than two codelet factors.
+bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1) {
+    std::vector<std::vector<int>> sets;
+    std::vector<int> cur;
+    if (N < 4 || N > 32768) return false;
+    multisets(N, 16, cur, sets);
+    if (sets.empty()) return false;
+    double best = 1e30;
+    std::vector<int> pick;
+    for (const std::vector<int> &m : sets) {
+        if (cls && m.back() > kDifPairMax) continue;
+        double c = 0;
+        for (int R : m) c += pass_cost(R, prec);
+        if (c < best) {
+            best = c;
+            pick = m;
+        }
+    }
+    if (pick.empty()) return false;
+    const int W = prec == P_F32 ? 16 : 8;
+    long bw = -1;
+    std::vector<int> q = pick;
+    std::sort(q.begin(), q.end());
+    int tried = 0;
+    do {
+        if (cls && (cls == 1 ? q.back() : q.front()) > kDifPairMax) continue;
+        const long S1 = N / q[0];
+        for (int pad = 0; pad < W; pad++) {
+            const long w = bank_waves(q, N, S1 + pad, W);
+            if (bw < 0 || w < bw || (w == bw && q[0] > rad[0])) {
+                bw = w;
+                rad = q;
+                *P1 = S1 + pad;
+            }
+        }
+    } while (++tried < 60 && std::next_permutation(q.begin(), q.end()));
+    return true;
+}
+
+// ---------------------------------------------------------------- tables
+static std::mutex g_dif_mu;
+static std::map<std::tuple<long, int, int>, DifTab> g_dif;
+
+static void root(long m, long N, double *c, double *s) {  // exp(-2 pi i m/N)
+    bool flip = false;
+    if (2 * m > N) {
+        m = N - m;
+        flip = true;
+    }
+    const double a = 2.0 * 3.14159265358979323846264338327950288 * ((double)m / (double)N);
+    *c = cos(a);
+    *s = flip ? sin(a) : -sin(a);
+}
+
+template <typename T> static void *upload_tables(const std::vector<int> &rad, long N, std::vector<int> &two) {
+    std::vector<T> tw;
+    long M = N;
+    for (size_t p = 0; p + 1 < rad.size(); p++) {
+        const long R = rad[p], S = M / R;
+        two.push_back((int)(tw.size() / 2));
+        for (long k = 0; k < R; k++)
+            for (long n = 0; n < S; n++) {
+                double c, s;
+                root(k * n % M, M, &c, &s);
+                tw.push_back((T)c);
+                tw.push_back((T)s);
+            }
+        M = S;
+    }
+    two.push_back(0);
+    void *d = dmalloc(tw.size() * sizeof(T));
+    if (!d) return nullptr;
+    if (!cuda_ok(cudaMemcpy(d, tw.data(), tw.size() * sizeof(T), cudaMemcpyHostToDevice), "twiddle upload")) {
+        dfree(d);
+        return nullptr;
+    }
+    return d;
+}
+
+// CTA shape of row calls: vpb transforms in nthr threads, chosen by the idle
+// thread slots of the passes' last rounds, the threads and points an SM then
+// holds, and the CTA's size.  Small CTAs (1200 to 2400 points) are in
+// different phases and end the last wave sooner; the weights are fitted to
+// sweeps of 51 lengths on 2^24 points, of which the rule's choice is 2 % off
+// the best on average (us, transforms x threads): 100 points 12 x 128 45.3, 24
+// x 256 49.3, 32 x 192 49.3; 1200: 2 x 128 60.5, 4 x 256 62.6, 6 x 320 63.5;
+// 2400: 1 x 160 62.1, 2 x 320 67.8, 3 x 512 70.1.
+static void row_shape(DifTab &t, int cls) {
+    const long esz = t.prec == P_F32 ? 8 : 16, regs = t.prec == P_F32 ? 64 : 128, maxt = 65536 / regs;
+    const long ldb = t.radix[0] * t.P1 * esz, unit = t.prec == P_F32 ? 1200 : 600;
+    const size_t np = t.radix.size();
+    double best = 1e30;
+    t.vpb = 1;
+    t.nthr = 96;
+    for (long v = 1; v == 1 || v * t.N <= 2 * unit; v++) {
+        for (long th = 96; th <= maxt; th += 32) {
+            double slots = 0;
+            for (size_t i = 0; i < np; i++) {
+                const int R = t.radix[i];
+                const bool pair = (cls == 1 && i + 1 == np) || (cls == 2 && i == 0);
+                const long per = t.N / R, nb = v * (pair ? per / 2 + 1 : per);
+                slots += (double)((nb + th - 1) / th) * pass_cost(R, t.prec) * R * (pair ? 2.0 : 1.0);
+            }
+            slots = slots * th / (double)(v * t.N);
+            const long ctas = std::min({32L, maxt / th, 227L * 1024 / (v * ldb + 1024)});
+            if (ctas < 1) continue;
+            const double act = (double)ctas * th, want = 0.9 * maxt, pts = (double)ctas * v * t.N;
+            if (act < want) slots *= sqrt(want / act);
+            if (pts < 10.0 * unit) slots *= 10.0 * unit / pts;
+            if (v > 1 && v * t.N > unit) slots *= pow((double)(v * t.N) / unit, 0.4);
+            if (slots < best) {
+                best = slots;
+                t.vpb = v;
+                t.nthr = (int)th;
+            }
+        }
+    }
+}
+
+const DifTab *dif_acquire(long N, int prec, int cls) {
+    if (prec != P_F32 || N > 16384) return nullptr;
+    std::lock_guard<std::mutex> lk(g_dif_mu);
+    auto key = std::make_tuple(N, prec, cls);
+    auto it = g_dif.find(key);
+    if (it != g_dif.end()) {
+        it->second.refs++;
+        return &it->second;
+    }
+    DifTab t;
+    if (!dif_schedule(N, prec, cls, t.radix, &t.P1)) return nullptr;
+    t.N = N;
+    t.prec = prec;
+    t.cls = cls;
+    const int err0 = jvsip_gpu_last_error();
+    t.d_tw = prec == P_F32 ? upload_tables<float>(t.radix, N, t.two) : upload_tables<double>(t.radix, N, t.two);
+    if (!t.d_tw) {  // the general kernels take the plan's calls
+        if (!err0 && jvsip_gpu_last_error()) jvsip_gpu_clear_error();
+        return nullptr;
+    }
+    row_shape(t, cls);
+    t.refs = 1;
+    auto &slot = g_dif[key];
+    slot = t;
+    return &slot;
+}
+
+void dif_release(const DifTab *t) {
+    if (!t) return;
+    std::lock_guard<std::mutex> lk(g_dif_mu);
+    auto it = g_dif.find(std::make_tuple(t->N, t->prec, t->cls));
+    if (it == g_dif.end() || --it->second.refs > 0) return;
+    dfree(it->second.d_tw);
+    g_dif.erase(it);
+}
+
+// ---------------------------------------------------------------- launch
+template <typename T> static bool interleaved_c(const CView &v) {
+    return v.cst == 2 && (const T *)v.im == (const T *)v.re + 1 && (uintptr_t)v.re % (2 * sizeof(T)) == 0;
+}
+// rows of len elements that do not overlap
+static bool apart(long vs, long len, long nvec) { return nvec <= 1 || labs(vs) >= len; }
+// real rows of unit stride, even offset and pitch: x_2n, x_2n+1 one complex element
+template <typename T> static bool real_pairs(const RView &r, long len, long nvec) {
+    return r.rst == 1 && r.es == 1 && r.off % 2 == 0 && (nvec <= 1 || (r.vs % 2 == 0 && labs(r.vs) >= len)) &&
+           (uintptr_t)r.a % (2 * sizeof(T)) == 0;
+}
+
+template <typename T>
+static bool launch_dif_t(const Job &j, cudaStream_t st) {
+    typedef typename cplx_t<T>::t C;
+    const DifTab *t = j.dif;
+    if (!t || j.no_fast || j.no_dif || j.nvec <= 0 || j.nbatch > 1 || j.tw_lo || j.gram || j.taper_n) return false;
+    const CView &ci = j.cin, &co = j.cout;
+    DifArgs<T> a;
+    memset(&a, 0, sizeof a);
+    bool rows = true, split = false;
+    if (j.kind == K_C2C) {
+        split = ci.cst == 1 && co.cst == 1;
+        if (!split && (!interleaved_c<T>(ci) || !interleaved_c<T>(co))) return false;
+        rows = ci.es == 1 && co.es == 1;
+        if (rows) {
+            if (!apart(ci.vs, j.N, j.nvec) || !apart(co.vs, j.N, j.nvec)) return false;
+        } else {
+            // adjacent transforms, their elements at least the whole set apart
+            if (labs(ci.vs) != 1 || labs(co.vs) != 1 || j.nvec < 2 || labs(ci.es) < j.nvec || labs(co.es) < j.nvec ||
+                j.tma_columns == 1)
+                return false;
+        }
+        if (split) {
+            a.in_re = (const T *)ci.re + ci.off;
+            a.in_im = (const T *)ci.im + ci.off;
+            a.out_re = (T *)co.re + co.off;
+            a.out_im = (T *)co.im + co.off;
+        } else {
+            a.in = (const C *)ci.re + ci.off;
+            a.out = (C *)co.re + co.off;
+        }
+        a.es_in = ci.es;
+        a.vs_in = ci.vs;
+        a.es_out = co.es;
+        a.vs_out = co.vs;
+        a.smask_in = a.smask_out = j.inv ? 0x80000000u : 0u;
+    } else if (sizeof(T) != 4 || !j.thalf) {
+        return false;
+    } else if (j.kind == K_R2C) {
+        if (!real_pairs<T>(j.rin, 2 * j.N, j.nvec) || !interleaved_c<T>(co)) return false;
+        // spectrum rows apart, or interleaved element by element (a column-major spectrum)
+        if (co.es == 1 ? !apart(co.vs, j.N + 1, j.nvec)
+                       : (co.es == 0 || co.vs == 0 || labs(co.vs) * j.nvec > labs(co.es)))
+            return false;
+        a.in = (const C *)j.rin.a + j.rin.off / 2;
+        a.vs_in = j.rin.vs / 2;
+        a.es_in = 1;
+        a.out = (C *)co.re + co.off;
+        a.es_out = co.es;
+        a.vs_out = co.vs;
+        a.thalf = (const C *)j.thalf;
+    } else {
+        if (!interleaved_c<T>(ci) || ci.es != 1 || !apart(ci.vs, j.N + 1, j.nvec) ||
+            !real_pairs<T>(j.rout, 2 * j.N, j.nvec))
+            return false;
+        a.in = (const C *)ci.re + ci.off;
+        a.vs_in = ci.vs;
+        a.es_in = 1;
+        a.out = (C *)j.rout.a + j.rout.off / 2;
+        a.vs_out = j.rout.vs / 2;
+        a.es_out = 1;
+        a.smask_out = 0x80000000u;
+        a.thalf = (const C *)j.thalf;
+    }
+    a.nvec = j.nvec;
+    a.N = (int)j.N;
+    a.np = (int)t->radix.size();
+    a.P1 = (int)t->P1;
+    a.LD = (int)(t->radix[0] * t->P1);
+    a.has_scale = j.has_scale;
+    a.scale = j.has_scale ? (T)j.scale : (T)1;
+    a.tw = (const C *)t->d_tw;
+    long M = j.N;
+    for (int i = 0; i < a.np; i++) {
+        DifPass &p = a.p[i];
+        p.R = t->radix[i];
+        p.S = (int)(M / p.R);
+        p.NR = (int)(j.N / p.R);
+        p.mstep = (int)M - p.S;
+        p.NB1 = (int)(j.N / t->radix[0] / p.R);
+        p.two = t->two[i];
+        p.mNR = magic_host((unsigned long)p.NR);
+        p.mNB1 = magic_host((unsigned long)p.NB1);
+        p.mS = magic_host((unsigned long)p.S);
+        p.mR = magic_host((unsigned long)p.R);
+        M = p.S;
+    }
+    if (j.kind == K_R2C) a.mH = magic_host((unsigned long)(a.p[a.np - 1].NR / 2 + 1));
+    if (j.kind == K_C2R) a.mH = magic_host((unsigned long)(a.p[0].S / 2 + 1));
+    const size_t cap = device()->smem_optin;
+    long vpb, nthr;
+    if (rows) {
+        vpb = t->vpb;
+        nthr = t->nthr;
+        // few transforms: smaller CTAs, so that more SMs work on them
+        while (vpb > 1 && (j.nvec + vpb - 1) / vpb < 2L * device()->sms) {
+            vpb = (vpb + 1) / 2;
+            nthr = std::max(64L, (vpb * j.N / 16 + 31) / 32 * 32);
+        }
+    } else {
+        // Column tiles, 64 KB or less: 16 adjacent transforms (128-byte rows of
+        // the tile) up to 256 points, 8 up to 1200, 4 beyond, about 16 points
+        // per thread.  Measured on 2^23 points (us; transforms x threads): 256
+        // points 16 x 256 29.2, 32 x 512 31.5, 4 x 64 34.8; 640: 8 x 320 40.3,
+        // 16 x 512 41.2, 4 x 160 45.4; 1200: 8 x 512 43.2, 4 x 320 45.0; 1500:
+        // 4 x 320 43.2, 8 x 640 50.2; 3000: 4 x 512 53.6, 8 x 1024 59.9.
+        const long pts = sizeof(T) == 4 ? 9600 : 4800;
+        a.lgv = sizeof(T) == 4 ? 4 : 3;
+        while (a.lgv > 1 && ((1L << a.lgv) * j.N > (a.lgv == 4 ? 4096 : pts))) a.lgv--;
+        if (a.lgv < 2 && sizeof(T) == 4) a.lgv = 2;
+        while (a.lgv > 0 && ((size_t)a.LD << a.lgv) * sizeof(C) > cap) a.lgv--;
+        vpb = 1L << a.lgv;
+        nthr = std::max(64L, (vpb * j.N / 16 + 31) / 32 * 32);
+        const long maxt = sizeof(T) == 4 ? 1024 : 512;
+        if (nthr > maxt) nthr = maxt;
+        if (sizeof(T) == 4 && nthr > 512 && vpb * j.N <= 16384) nthr = 512;
+    }
+    a.vpb = (int)vpb;
+    const size_t smem = (size_t)a.LD * vpb * sizeof(C);
+    if (smem > cap) return false;
+    if constexpr (sizeof(T) == 4) {
+        if (j.kind == K_R2C) return dif_go<T, DIF_R2C, false>(a, (int)nthr, smem, st);
+        if (j.kind == K_C2R) return dif_go<T, DIF_C2R, false>(a, (int)nthr, smem, st);
+        if (split)
+            return rows ? dif_go<T, DIF_SPLIT, false>(a, (int)nthr, smem, st)
+                        : dif_go<T, DIF_SPLIT, true>(a, (int)nthr, smem, st);
+    } else if (split) {
+        return false;
+    }
+    return rows ? dif_go<T, DIF_C2C, false>(a, (int)nthr, smem, st) : dif_go<T, DIF_C2C, true>(a, (int)nthr, smem, st);
+}
+
+bool launch_dif_f32(const Job &j, cudaStream_t st) { return launch_dif_t<float>(j, st); }
+
+}  // namespace jv

@@ -1,0 +1,380 @@
+// jv_dif.cuh -- the in-place mixed-radix kernel: whole transforms of any
+// length N = R1*R2*...*Rp (codelets 2..16) in shared memory, decimated in
+// frequency.
+//
+// Pass 1 reads the view: the butterfly of n' (< S1 = N/R1) takes elements
+// n' + r*S1, multiplies output k1 by exp(-2 pi i k1 n'/N) and stores it at
+// k1*P1 + n'.  Pass p transforms the R_p sub-blocks of S_p elements inside
+// every block of M_p = R_p*S_p = S_(p-1) elements, twiddles output k_p by
+// exp(-2 pi i k_p n/M_p) and puts it back where it came from.  The last pass
+// (S = 1) writes the view: butterfly q = k1 + R1*(k2 + R2*(k3 ...)) holds
+// outputs q + r*N/R_last.
+//
+// Every butterfly reads and writes the same R places, so a pass is a plain
+// loop over butterflies with one barrier after it (the self-sorting passes of
+// k_smem hold every butterfly of a thread in registers between two barriers),
+// a butterfly's addresses are computed once, and any thread count serves any
+// radix.  The pitch P1 of the k1 blocks is the one of 16 paddings whose
+// accesses collide least in the shared-memory banks (dif_shape).
+#pragma once
+
+#include "jv_kernels.cuh"
+
+namespace jv {
+
+constexpr int kDifMaxPass = 8;
+
+struct DifPass {
+    int R, S;            // radix; distance of a butterfly's elements inside a k1 block
+    int NR, mstep;       // butterflies per transform N/R; M - S
+    int NB1, two;        // butterflies per k1 block; start of the pass's twiddle table
+    unsigned mNR, mNB1;  // multiply-high magic of NR, NB1
+    unsigned mS, mR;     // of S, R
+};
+
+template <typename T> struct DifArgs {
+    typedef typename cplx_t<T>::t C;
+    // transform v starts at in + v*vs_in; element n follows at n*es_in (es 1 for rows)
+    const C *in;
+    C *out;
+    const T *in_re, *in_im;  // split complex views
+    T *out_re, *out_im;
+    long es_in, vs_in, es_out, vs_out, nvec;
+    int N, np, vpb, lgv;     // transforms per CTA (2^lgv for column tiles)
+    int P1, LD;              // pitch of a k1 block; of a transform (rows)
+    unsigned smask_in, smask_out;  // 0x80000000: conjugate on load / store
+    int has_scale;
+    T scale;
+    const C *tw;             // per-pass tables: pass p at p.two, entry k*S + n = exp(-2 pi i k n/M)
+    const C *thalf;          // real transforms: exp(-+ i pi k/N), k <= N
+    unsigned mH;             // and the magic of the pair passes' work items per transform
+    DifPass p[kDifMaxPass];
+};
+
+enum DifKind { DIF_C2C = 0, DIF_SPLIT = 1, DIF_R2C = 2, DIF_C2R = 3 };
+
+template <int KIND, typename T>
+__device__ __forceinline__ typename cplx_t<T>::t dif_in(const DifArgs<T> &a, long e) {
+    typedef typename cplx_t<T>::t C;
+    if constexpr (KIND == DIF_SPLIT) return mk<C>(a.in_re[e], a.in_im[e]);
+    else return a.in[e];
+}
+template <int KIND, typename T>
+__device__ __forceinline__ void dif_out(const DifArgs<T> &a, long e, typename cplx_t<T>::t c) {
+    if constexpr (KIND == DIF_SPLIT) {
+        a.out_re[e] = c.x;
+        a.out_im[e] = c.y;
+    } else {
+        a.out[e] = c;
+    }
+}
+
+// First pass.  Rows: consecutive threads on consecutive n' of one transform;
+// column tiles: on adjacent transforms (element i of transform t at i*vpb + t).
+template <int KIND, bool COLS, int R, typename T>
+__device__ __forceinline__ void dif_first(const DifArgs<T> &a, typename cplx_t<T>::t *s, int nt, long v0) {
+    typedef typename cplx_t<T>::t C;
+    const DifPass &p = a.p[0];
+    const int S = p.S, V = COLS ? a.vpb : 1;
+    const int nb = COLS ? S : nt * S;
+    const int step = COLS ? (int)blockDim.x >> a.lgv : (int)blockDim.x;
+    const int ct = COLS ? ((int)threadIdx.x & (V - 1)) : 0;
+    const int sp = a.P1 * V;
+    if (COLS && ct >= nt) return;
+    for (int b = COLS ? (int)threadIdx.x >> a.lgv : (int)threadIdx.x; b < nb; b += step) {
+        int t = ct, j = b;
+        if (!COLS && a.vpb > 1) {
+            t = mdiv(b, p.mNR);
+            j = b - t * S;
+        }
+        const long e0 = (v0 + t) * a.vs_in + (COLS ? (long)j * a.es_in : (long)j);
+        C v[R];
+        if constexpr (COLS) {
+            const long st = (long)S * a.es_in;
+#pragma unroll
+            for (int r = 0; r < R; r++) v[r] = dif_in<KIND>(a, e0 + r * st);
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++) v[r] = dif_in<KIND>(a, e0 + r * S);
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r].y = flip_sign(v[r].y, a.smask_in);
+        Dft<C, R>::run(v);
+        const C *w = a.tw + j;
+#pragma unroll
+        for (int r = 1; r < R; r++) v[r] = cmul(v[r], __ldg(w + r * S));
+        C *d = COLS ? s + (j * V + t) : s + (t * a.LD + j);
+#pragma unroll
+        for (int r = 0; r < R; r++) d[r * sp] = v[r];
+    }
+}
+
+// Middle pass.
+template <bool COLS, int R, typename T>
+__device__ __forceinline__ void dif_mid(const DifArgs<T> &a, const DifPass &p, typename cplx_t<T>::t *s, int nt) {
+    typedef typename cplx_t<T>::t C;
+    const int S = p.S, V = COLS ? a.vpb : 1;
+    const int nb = COLS ? p.NR : nt * p.NR;
+    const int step = COLS ? (int)blockDim.x >> a.lgv : (int)blockDim.x;
+    const int ct = COLS ? ((int)threadIdx.x & (V - 1)) : 0;
+    const int sp = S * V;
+    if (COLS && ct >= nt) return;
+    for (int b = COLS ? (int)threadIdx.x >> a.lgv : (int)threadIdx.x; b < nb; b += step) {
+        int t = ct, j = b;
+        if (!COLS && a.vpb > 1) {
+            t = mdiv(b, p.mNR);
+            j = b - t * p.NR;
+        }
+        const int k1 = mdiv(j, p.mNB1), u = j - k1 * p.NB1;
+        const int c = mdiv(u, p.mS), n = u - c * S;
+        const int pos = k1 * a.P1 + u + c * p.mstep;
+        C *d = COLS ? s + (pos * V + t) : s + (t * a.LD + pos);
+        C v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = d[r * sp];
+        Dft<C, R>::run(v);
+        const C *w = a.tw + (p.two + n);
+#pragma unroll
+        for (int r = 1; r < R; r++) v[r] = cmul(v[r], __ldg(w + r * S));
+#pragma unroll
+        for (int r = 0; r < R; r++) d[r * sp] = v[r];
+    }
+}
+
+// position of butterfly q = k1 + R1*(k2 + R2*(...)) of the last pass
+template <typename T> __device__ __forceinline__ int dif_pos(const DifArgs<T> &a, int q) {
+    int rem = mdiv(q, a.p[0].mR);
+    int pos = (q - rem * a.p[0].R) * a.P1;
+    for (int i = 1; i + 1 < a.np; i++) {
+        const int n = mdiv(rem, a.p[i].mR);
+        pos += (rem - n * a.p[i].R) * a.p[i].S;
+        rem = n;
+    }
+    return pos;
+}
+
+// Last pass: to the view.
+template <int KIND, bool COLS, int R, typename T>
+__device__ __forceinline__ void dif_last(const DifArgs<T> &a, const typename cplx_t<T>::t *s, int nt, long v0) {
+    typedef typename cplx_t<T>::t C;
+    const DifPass &p = a.p[a.np - 1];
+    const int Q = p.NR, V = COLS ? a.vpb : 1;
+    const int nb = COLS ? Q : nt * Q;
+    const int step = COLS ? (int)blockDim.x >> a.lgv : (int)blockDim.x;
+    const int ct = COLS ? ((int)threadIdx.x & (V - 1)) : 0;
+    if (COLS && ct >= nt) return;
+    for (int b = COLS ? (int)threadIdx.x >> a.lgv : (int)threadIdx.x; b < nb; b += step) {
+        int t = ct, q = b;
+        if (!COLS && a.vpb > 1) {
+            t = mdiv(b, p.mNR);
+            q = b - t * Q;
+        }
+        const int pos = dif_pos(a, q);
+        const C *d = COLS ? s + (pos * V + t) : s + (t * a.LD + pos);
+        C v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = COLS ? d[r * V] : d[r];
+        Dft<C, R>::run(v);
+        const long e0 = (v0 + t) * a.vs_out + (COLS ? (long)q * a.es_out : (long)q);
+        const long st = COLS ? (long)Q * a.es_out : (long)Q;
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            dif_out<KIND>(a, e0 + r * st, out_value(v[r], a.smask_out, a.has_scale != 0, a.scale));
+    }
+}
+
+// First pass of C2R rows: Y_n = X_n + conj X_{N-n} + i w_n (X_n - conj X_{N-n}),
+// w_n = exp(+i pi n/N) (c_VSIP_src/VI_crfftmop_f_def.h:58-110), conjugated for
+// the forward passes.  A thread takes the butterflies of n' and S - n' (one of
+// them for n' = 0 and S/2), which hold each other's partners X_{N-n}, so every
+// spectrum element is loaded once; w_{N-n} = -conj w_n.
+template <int R, typename T>
+__device__ __forceinline__ void dif_first_c2r(const DifArgs<T> &a, typename cplx_t<T>::t *s, int nt, long v0) {
+    typedef typename cplx_t<T>::t C;
+    const DifPass &p = a.p[0];
+    const int S = p.S, H = S / 2 + 1;
+    for (int b = threadIdx.x; b < nt * H; b += blockDim.x) {
+        const int t = mdiv(b, a.mH), j = b - t * H;
+        const C *x = a.in + (v0 + t) * a.vs_in;
+        const C *xu = x + j, *xw = x + (S - j), *h = a.thalf + j;
+        C u[R], w[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) u[r] = xu[r * S];
+#pragma unroll
+        for (int r = 0; r < R; r++) w[r] = xw[r * S];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const C f = u[r], g = w[R - 1 - r], c = __ldg(h + r * S);
+            const C d = mk<C>(g.x - f.x, f.y + g.y);
+            u[r] = mk<C>(f.x + g.x + c.y * d.x - c.x * d.y, -(f.y - g.y - c.y * d.y - c.x * d.x));
+            w[R - 1 - r] = mk<C>(f.x + g.x - c.y * d.x + c.x * d.y, -(g.y - f.y - c.y * d.y - c.x * d.x));
+        }
+        C *d = s + (t * a.LD + j);
+        Dft<C, R>::run(u);
+        const C *tu = a.tw + j;
+#pragma unroll
+        for (int r = 1; r < R; r++) u[r] = cmul(u[r], __ldg(tu + r * S));
+#pragma unroll
+        for (int r = 0; r < R; r++) d[r * a.P1] = u[r];
+        if (j != 0 && 2 * j != S) {
+            d += S - 2 * j;
+            Dft<C, R>::run(w);
+            const C *tw = a.tw + (S - j);
+#pragma unroll
+            for (int r = 1; r < R; r++) w[r] = cmul(w[r], __ldg(tw + r * S));
+#pragma unroll
+            for (int r = 0; r < R; r++) d[r * a.P1] = w[r];
+        }
+    }
+}
+
+// Last pass of R2C rows: Z from two butterflies q and Q - q (Q = N/R), which
+// hold each other's partners Z_{N-k}, then X_k = ((Z_k + conj Z_{N-k}) - i w_k
+// (Z_k - conj Z_{N-k}))/2, w_k = exp(-i pi k/N), Z_N = Z_0, the scale applied
+// to Z first (c_VSIP_src/VI_rcfftmop_f_def.h:79-118): the spectrum leaves from
+// registers, without another trip through shared memory.
+template <int R, typename T>
+__device__ __forceinline__ void dif_last_r2c(const DifArgs<T> &a, const typename cplx_t<T>::t *s, int nt, long v0) {
+    typedef typename cplx_t<T>::t C;
+    const DifPass &p = a.p[a.np - 1];
+    const int Q = p.NR, H = Q / 2 + 1;
+    for (int b = threadIdx.x; b < nt * H; b += blockDim.x) {
+        const int t = mdiv(b, a.mH), q = b - t * H;
+        const C *su = s + (t * a.LD + dif_pos(a, q)), *sw = s + (t * a.LD + dif_pos(a, q ? Q - q : 0));
+        C u[R], w[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) u[r] = su[r];
+#pragma unroll
+        for (int r = 0; r < R; r++) w[r] = sw[r];
+        Dft<C, R>::run(u);
+        Dft<C, R>::run(w);
+        if (a.has_scale) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                u[r] = cscale(u[r], a.scale);
+                w[r] = cscale(w[r], a.scale);
+            }
+        }
+        const C *h = a.thalf + q;
+        C *o = a.out + (v0 + t) * a.vs_out;
+        const bool both = q != 0 && 2 * q != Q;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int k = q + r * Q;
+            const C z = u[r], c = __ldg(h + r * Q);
+            C n = w[R - 1 - r];
+            if (q == 0) n = w[(R - r) % R];
+            const C sm = mk<C>(z.x + n.x, z.y + n.y), df = mk<C>(z.x - n.x, z.y - n.y);
+            o[(long)k * a.es_out] =
+                mk<C>((T)0.5 * (sm.x + c.x * sm.y + c.y * df.x), (T)0.5 * (df.y - c.x * df.x + c.y * sm.y));
+            if (both || (r == 0 && q == 0))
+                o[(long)(a.N - k) * a.es_out] =
+                    mk<C>((T)0.5 * (sm.x - c.x * sm.y - c.y * df.x), (T)0.5 * (-df.y - c.x * df.x + c.y * sm.y));
+        }
+    }
+}
+
+#define JV_DIF_SWITCH(RAD, CALL)     \
+    switch (RAD) {                   \
+        case 16: CALL(16); break;    \
+        case 15: CALL(15); break;    \
+        case 14: CALL(14); break;    \
+        case 13: CALL(13); break;    \
+        case 12: CALL(12); break;    \
+        case 11: CALL(11); break;    \
+        case 10: CALL(10); break;    \
+        case 9: CALL(9); break;      \
+        case 8: CALL(8); break;      \
+        case 7: CALL(7); break;      \
+        case 6: CALL(6); break;      \
+        case 5: CALL(5); break;      \
+        case 4: CALL(4); break;      \
+        case 3: CALL(3); break;      \
+        default: CALL(2); break;     \
+    }
+
+// the pair passes hold two butterflies, of at most this radix
+constexpr int kDifPairMax = 10;
+#define JV_DIF_PAIR_SWITCH(RAD, CALL) \
+    switch (RAD) {                    \
+        case 10: CALL(10); break;     \
+        case 9: CALL(9); break;       \
+        case 8: CALL(8); break;       \
+        case 7: CALL(7); break;       \
+        case 6: CALL(6); break;       \
+        case 5: CALL(5); break;       \
+        case 4: CALL(4); break;       \
+        case 3: CALL(3); break;       \
+        default: CALL(2); break;      \
+    }
+
+template <typename T, int KIND, bool COLS>
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_dif(const __grid_constant__ DifArgs<T> a) {
+    typedef typename cplx_t<T>::t C;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    C *s = reinterpret_cast<C *>(smem_raw);
+    const long v0 = (long)blockIdx.x * a.vpb;
+    const int nt = (int)min((long)a.vpb, a.nvec - v0);
+    if constexpr (KIND == DIF_C2R) {
+#define JV_DIF_FIRST(R) (dif_first_c2r<R, T>(a, s, nt, v0))
+        JV_DIF_PAIR_SWITCH(a.p[0].R, JV_DIF_FIRST)
+#undef JV_DIF_FIRST
+    } else {
+#define JV_DIF_FIRST(R) (dif_first<KIND, COLS, R, T>(a, s, nt, v0))
+        JV_DIF_SWITCH(a.p[0].R, JV_DIF_FIRST)
+#undef JV_DIF_FIRST
+    }
+    __syncthreads();
+    for (int i = 1; i + 1 < a.np; i++) {
+#define JV_DIF_MID(R) (dif_mid<COLS, R, T>(a, a.p[i], s, nt))
+        JV_DIF_SWITCH(a.p[i].R, JV_DIF_MID)
+#undef JV_DIF_MID
+        __syncthreads();
+    }
+    if constexpr (KIND == DIF_R2C) {
+#define JV_DIF_LAST(R) (dif_last_r2c<R, T>(a, s, nt, v0))
+        JV_DIF_PAIR_SWITCH(a.p[a.np - 1].R, JV_DIF_LAST)
+#undef JV_DIF_LAST
+    } else {
+#define JV_DIF_LAST(R) (dif_last<KIND, COLS, R, T>(a, s, nt, v0))
+        JV_DIF_SWITCH(a.p[a.np - 1].R, JV_DIF_LAST)
+#undef JV_DIF_LAST
+    }
+}
+
+// Launches (nvec + vpb - 1)/vpb CTAs of nthr threads; instances in jv_dif*.cu.
+template <typename T, int KIND, bool COLS>
+bool dif_go(const DifArgs<T> &a, int nthr, size_t smem, cudaStream_t st);
+
+template <typename T, int KIND, bool COLS>
+inline bool dif_launch(const DifArgs<T> &a, int nthr, size_t smem, cudaStream_t st) {
+    static std::atomic<bool> attr{false};  // set once; concurrent first calls both set it
+    if (!attr) {
+        if (!cuda_ok(cudaFuncSetAttribute(k_dif<T, KIND, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)device()->smem_optin),
+                     "cudaFuncSetAttribute"))
+            return false;
+        attr = true;
+    }
+    const long grid = (a.nvec + a.vpb - 1) / a.vpb;
+    if (grid > 0x7fffffffL) return false;
+    k_dif<T, KIND, COLS><<<(unsigned)grid, (unsigned)nthr, smem, st>>>(a);
+    count_launch();
+    return cuda_ok(cudaGetLastError(), "k_dif launch");
+}
+#define JV_DIF_INSTANCE(T, KIND, COLS)                                                        \
+    template <>                                                                               \
+    bool dif_go<T, KIND, COLS>(const DifArgs<T> &a, int nthr, size_t smem, cudaStream_t st) { \
+        return dif_launch<T, KIND, COLS>(a, nthr, smem, st);                                  \
+    }
+#define JV_DIF_DECLARE(T, KIND, COLS) \
+    template <>                       \
+    bool dif_go<T, KIND, COLS>(const DifArgs<T> &a, int nthr, size_t smem, cudaStream_t st);
+JV_DIF_DECLARE(float, DIF_C2C, false)
+JV_DIF_DECLARE(float, DIF_C2C, true)
+JV_DIF_DECLARE(float, DIF_SPLIT, false)
+JV_DIF_DECLARE(float, DIF_SPLIT, true)
+JV_DIF_DECLARE(float, DIF_R2C, false)
+JV_DIF_DECLARE(float, DIF_C2R, false)
+
+}  // namespace jv

@@ -1,0 +1,7 @@
+// jv_dif_f32.cu -- single-precision c2c instances of the in-place mixed-radix kernel (jv_dif.cuh).
+#include "jv_dif.cuh"
+
+namespace jv {
+JV_DIF_INSTANCE(float, DIF_C2C, false)
+JV_DIF_INSTANCE(float, DIF_C2C, true)
+}  // namespace jv

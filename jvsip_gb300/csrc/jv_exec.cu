@@ -557,6 +557,19 @@ static bool run_long(Job &j, cudaStream_t st, bool *handled) {
     return j.prec == P_F32 ? launch_c2r_unpack_f32(j, ys, st) : launch_c2r_unpack_f64(j, ys, st);
 }
 
+// One launch over whole transforms: the register-resident kernel at its
+// lengths, the in-place mixed-radix kernel at the others (lengths with factors
+// 11 and 13 among them) and where it is the faster one -- rows of 64 and 1000
+// points that fill the GPU (2^24 points: 43.1 us against 49.2, and 60 against
+// 70; 40 rows of 1000: 6.9 against 6.2).  False when neither takes the call.
+static bool run_tiles(const Job &j, cudaStream_t st) {
+    if (j.prec != P_F32) return false;
+    const bool dif_first = (j.N == 64 || j.N == 1000) && j.kind == K_C2C && j.cin.cst == 2 && j.cin.es == 1 &&
+                           j.cout.es == 1 && j.nvec * j.N >= 4096L * device()->sms;
+    if (dif_first && launch_dif_f32(j, st)) return true;
+    return launch_fast_f32(j, st) || launch_dif_f32(j, st);
+}
+
 static bool run_job(Job &j, cudaStream_t st) {
     if (j.nvec <= 0 || j.N <= 0) return true;
     if (j.form == JVSIP_FORM_SPLIT_BF16 || j.form == JVSIP_FORM_SPLIT_FP16) {
@@ -568,23 +581,15 @@ static bool run_job(Job &j, cudaStream_t st) {
     // columns take the two steps when the plan's scratch can be had, the
     // tile kernels otherwise
     const bool two = long_few(j) || (long_columns(j) && long_scratch(j.lp, long_scratch_need(j), true));
-    if (job_in_smem(j) && !two) {
-        if (j.prec == P_F32) {
-            if (launch_fast_f32(j, st)) return true;
-            return launch_smem_f32(j, st);
-        }
-        return launch_smem_f64(j, st);
-    }
-    if (j.lp) {
+    if (!two && run_tiles(j, st)) return true;
+    if (j.lp && (two || !job_in_smem(j))) {
         bool handled = false;
         const bool ok = run_long(j, st, &handled);
         if (handled) return ok;
+        if (two && run_tiles(j, st)) return true;
     }
     if (job_in_smem(j)) {
-        if (j.prec == P_F32) {
-            if (launch_fast_f32(j, st)) return true;
-            return launch_smem_f32(j, st);
-        }
+        if (j.prec == P_F32) return launch_smem_f32(j, st);
         return launch_smem_f64(j, st);
     }
     return j.prec == P_F32 ? launch_global_f32(j, st) : launch_global_f64(j, st);
@@ -693,6 +698,8 @@ static void fill_job(Job &j, const Plan *p, int kind) {
     j.twg = p->d_twg;
     j.pc = p->d_pc;
     j.twdd = p->d_twdd;
+    j.dif = p->dif;
+    j.no_dif = p->no_dif;
     j.form = p->form;
     j.no_fast = p->no_fast;
     j.no_pipeline = p->no_pipeline;

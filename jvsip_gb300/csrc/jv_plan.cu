@@ -277,9 +277,11 @@ static bool make_tables(Plan *p) {
         p->d_twp = it->second.twp;
         p->d_twg = it->second.twg;
         p->d_pc = it->second.pc;
+        p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type));
         return true;
     }
     if (!build_tables<T>(p)) return false;
+    p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type));
     TableSet ts;
     ts.tw = p->d_tw;
     ts.thalf = p->d_thalf;
@@ -292,6 +294,8 @@ static bool make_tables(Plan *p) {
 }
 
 static void release_tables(Plan *p) {
+    dif_release(p->dif);
+    p->dif = nullptr;
     std::lock_guard<std::mutex> lk(g_tab_mu);
     auto key = std::make_tuple(p->MN, p->prec, table_kind(p->type), sched_key(p->radix));
     auto it = g_tabs.find(key);
@@ -637,8 +641,12 @@ static Plan *new_plan(int type, vsip_length M, vsip_length N, double scale, int 
         PlainTune t;
         if ((type == JV_CCFFTOP || type == JV_CCFFTIP) && p->smooth &&
             plain_tuned(p->MN, p->prec, p->major, &t)) {
-            if (schedule_valid(t.radix, p->MN, maxt)) p->radix = t.radix;
+            if (schedule_valid(t.radix, p->MN, maxt) && t.radix != p->radix) {
+                p->radix = t.radix;
+                p->no_dif = true;
+            }
             if (t.res == 1) p->no_fast = true;
+            if (t.vpb > 0 || t.emax > 0) p->no_dif = true;
             p->tuned_vpb = t.vpb;
             p->tuned_emax = t.emax;
             p->tuned = true;
