@@ -3,18 +3,19 @@
 // majors) in one launch per CTA-size class, fed by a device queue of tile
 // descriptors.
 //
-// The host cuts every call into tiles of transforms (FFTs per tile from the
-// autotuner's cache, or a heuristic), gives each tile the smallest CTA size
-// (256, 512 or 1024 threads) whose threads cover its passes, and uploads one
-// descriptor queue per size, largest tiles first.  One launch per size
-// consumes its queue, one descriptor per CTA -- no CTA ever waits on another
-// -- running the general kernel's fused c2c passes on each tile; the launches
-// run side by side on forked streams.  Each CTA first asks L2 for the input
-// of the descriptor one resident wave further down its queue (the CTA that
-// will take this SM slot later), so later tiles' DRAM reads overlap earlier
-// tiles' passes.  Columns of 8192 points or more (adjacent, more than one) go
-// through the plain calls' two steps instead, on four more streams.  A
-// captured batch (jvsip_fftm_batch_create_f) records the launches in a CUDA
+// The host cuts every call on row-contiguous or adjacent transforms into tiles
+// of the in-place mixed-radix kernel (jv_dif.cuh, k_dif_batch): one queue per
+// block size, largest tiles first, one tile per CTA -- no CTA ever waits on
+// another -- whose arguments (the call's) the CTA copies into shared memory.
+// Columns from kColStepsMin points (adjacent, more than one) go through the
+// plain calls' two steps on eight streams of their own.  Other layouts, and
+// lengths without a schedule of two codelets, keep the general kernel's fused
+// c2c passes in CTAs of 256, 512 or 1024 threads (k_batch), each CTA asking L2
+// for the input of the descriptor one resident wave further down its queue.
+// The launches run side by side on forked streams.  160 instances of 64-16384
+// points (0.58 GB per buffer) on GB300: 0.60 ms against 0.79 with every tile
+// on the general kernel's passes and only columns from 8192 points in steps.
+// A captured batch (jvsip_fftm_batch_create_f) records the launches in a CUDA
 // graph once; jvsip_fftm_batch_run_f replays it.
 //
 // No reference counterpart: VSIPL has no multi-plan call; the reference can
@@ -23,12 +24,14 @@
 #include <string.h>
 
 #include <algorithm>
+#include <map>
 #include <mutex>
 #include <new>
 #include <vector>
 
 #include <cooperative_groups.h>
 
+#include "jv_dif.cuh"
 #include "jv_launch.cuh"
 
 namespace jv {
@@ -229,18 +232,26 @@ __global__ void __cluster_dims__(kColCluster, 1, 1) __launch_bounds__(BT, 1)
 
 // ---------------------------------------------------------------- host side
 // A call the batch runs through the plain path instead of tiles: single-
-// precision c2c columns (adjacent vectors on both sides) of 8192 points or
-// more, which the plain calls take as two steps (on the register-resident
-// column tiles or the shared-memory kernel, the groups along the grid's y).
-// Measured on the 2 GB batch: its columns of 8192-16384 points 1.052 ms this
-// way against 1.185 ms on the column clusters; columns of 3000-8191 points
-// were slower this way than as tiles (0.94 against 0.72 ms).
+// precision c2c columns (adjacent vectors on both sides) that the plain calls
+// take as two steps, the groups along the grid's y.  Measured on the 160
+// instances above: 0.60 ms with all of them in steps, 0.64 with columns of
+// 3000-8191 points as tiles of 4 columns.
 struct StepCall {
     Plan *p;
     const vsip_cmview_f *x, *y;
 };
 
+// Tiles of the in-place mixed-radix kernel of one block size, rows or columns.
+struct DifGroup {
+    bool cols = false;
+    int nthr = 0;
+    size_t smem = 0;
+    std::vector<DifTile> tiles;
+};
+
 struct BatchBuild {
+    std::vector<DifArgs<float>> calls;   // of the groups' tiles
+    std::vector<DifGroup> groups;
     std::vector<TileDesc> tiles[kClasses];
     size_t smem[kClasses] = {0, 0, 0, 0};
     std::vector<StepCall> steps;
@@ -255,6 +266,54 @@ static long tile_ld(long N, bool vf) {
 
 // FFTs per tile for length N (transforms adjacent in memory or not).
 long batch_fft_per_tile(long N, bool vf, long rows);
+long batch_tuned_per_tile(long N, bool vf);  // the autotuner's entry, 0: none
+
+// Cuts a call into tiles of the in-place mixed-radix kernel; false when its
+// views or length are not for it.
+static bool dif_tiles(const Plan *p, const TileDesc &t, long nv, BatchBuild &bb) {
+    Job j;
+    j.kind = K_C2C;
+    j.prec = P_F32;
+    j.N = t.N;
+    j.nvec = nv;
+    j.inv = t.inv;
+    j.has_scale = t.has_scale;
+    j.scale = t.scale;
+    j.dif = p->dif;
+    j.no_fast = p->no_fast;
+    j.no_dif = p->no_dif;
+    j.cin.re = const_cast<float *>(t.in);
+    j.cin.im = const_cast<float *>(t.in) + 1;
+    j.cin.off = t.in_off;
+    j.cin.es = t.in_es;
+    j.cin.vs = t.in_vs;
+    j.cout.re = t.out;
+    j.cout.im = t.out + 1;
+    j.cout.off = t.out_off;
+    j.cout.es = t.out_es;
+    j.cout.vs = t.out_vs;
+    DifArgs<float> a;
+    DifCta c;
+    if (!dif_tile_args(j, batch_tuned_per_tile(t.N, t.vec_fast != 0), a, c) ||
+        c.smem > device()->smem_optin - kStaticArgs)
+        return false;
+    // block sizes in steps of 64, so that one launch takes tiles of many lengths
+    c.nthr = (c.nthr + 63) / 64 * 64;
+    DifGroup *g = nullptr;
+    for (DifGroup &h : bb.groups)
+        if (h.cols == !c.rows && h.nthr == c.nthr) g = &h;
+    if (!g) {
+        bb.groups.emplace_back();
+        g = &bb.groups.back();
+        g->cols = !c.rows;
+        g->nthr = c.nthr;
+    }
+    g->smem = std::max(g->smem, c.smem);
+    for (long v0 = 0; v0 < nv; v0 += a.vpb)
+        g->tiles.push_back(DifTile{(int)bb.calls.size(), (int)std::min((long)a.vpb, nv - v0), v0});
+    bb.calls.push_back(a);
+    return true;
+}
 
 static bool build_tiles(size_t n, const vsip_fftm_f *const plans[], const vsip_cmview_f *const in[],
                         const vsip_cmview_f *const out[], BatchBuild &bb) {
@@ -336,8 +395,12 @@ static bool build_tiles(size_t n, const vsip_fftm_f *const plans[], const vsip_c
         bool vf_out = labs(t.out_vs) == 1 && labs(t.out_es) != 1;
         t.vec_fast = (vf_in || vf_out) ? 1 : 0;
         t.ld = (int)tile_ld(N, t.vec_fast);
-        if (N >= kLongFewMin && resident_long_columns_f(p, x, y)) {
+        if (resident_long_columns_f(p, x, y)) {
             bb.steps.push_back(StepCall{p, x, y});
+            bb.bytes += 16.0 * N * nv;
+            continue;
+        }
+        if (dif_tiles(p, t, nv, bb)) {
             bb.bytes += 16.0 * N * nv;
             continue;
         }
@@ -389,6 +452,12 @@ static bool build_tiles(size_t n, const vsip_fftm_f *const plans[], const vsip_c
         std::stable_sort(bb.tiles[c].begin(), bb.tiles[c].end(), [](const TileDesc &a, const TileDesc &b) {
             return (long)a.N * a.nt > (long)b.N * b.nt;
         });
+    for (DifGroup &g : bb.groups)
+        std::stable_sort(g.tiles.begin(), g.tiles.end(), [&](const DifTile &a, const DifTile &b) {
+            return (long)bb.calls[a.call].N * a.nt > (long)bb.calls[b.call].N * b.nt;
+        });
+    // the groups of the largest CTAs are launched first
+    std::stable_sort(bb.groups.begin(), bb.groups.end(), [](const DifGroup &a, const DifGroup &b) { return a.smem > b.smem; });
     return true;
 }
 
@@ -399,6 +468,14 @@ struct DevBatch {
     size_t smem[kClasses] = {0, 0, 0, 0};
     int total = 0;
     std::vector<StepCall> steps;      // calls run through the plain path
+    struct Group {
+        bool cols;
+        int nthr, first, n;
+        size_t smem;
+    };
+    DifArgs<float> *calls = nullptr;  // the in-place mixed-radix kernel's calls and tiles
+    DifTile *tiles = nullptr;
+    std::vector<Group> groups;
 };
 
 static bool upload(const BatchBuild &bb, DevBatch &db) {
@@ -422,7 +499,21 @@ static bool upload(const BatchBuild &bb, DevBatch &db) {
                                                  cudaMemcpyHostToDevice, d->stream),
                                  "batch queue upload"))
         return false;
-    return true;
+    if (bb.groups.empty()) return true;
+    std::vector<DifTile> tiles;
+    for (const DifGroup &g : bb.groups) {
+        db.groups.push_back({g.cols, g.nthr, (int)tiles.size(), (int)g.tiles.size(), g.smem});
+        tiles.insert(tiles.end(), g.tiles.begin(), g.tiles.end());
+    }
+    db.calls = (DifArgs<float> *)dmalloc(bb.calls.size() * sizeof(DifArgs<float>));
+    db.tiles = (DifTile *)dmalloc(tiles.size() * sizeof(DifTile));
+    return db.calls && db.tiles &&
+           cuda_ok(cudaMemcpyAsync(db.calls, bb.calls.data(), bb.calls.size() * sizeof(DifArgs<float>),
+                                   cudaMemcpyHostToDevice, d->stream),
+                   "batch queue upload") &&
+           cuda_ok(cudaMemcpyAsync(db.tiles, tiles.data(), tiles.size() * sizeof(DifTile), cudaMemcpyHostToDevice,
+                                   d->stream),
+                   "batch queue upload");
 }
 
 template <int CBT>
@@ -475,10 +566,12 @@ static bool launch_one(const DevBatch &db, int c, cudaStream_t st) {
 
 // Streams and events the classes run on side by side (forked from and joined
 // back to the caller's stream; the same pattern is recorded into the graph).
-constexpr int kStepStreams = 4;  // streams of the calls run through the plain path
+constexpr int kStepStreams = 8;  // streams of the calls run through the plain path
+constexpr int kDifStreams = 8;   // streams of the in-place mixed-radix kernel's groups
+constexpr int kBatchStreams = kClasses + kStepStreams + kDifStreams;
 struct BatchStreams {
-    cudaStream_t s[kClasses + kStepStreams] = {};  // the classes', then the plain-path calls'
-    cudaEvent_t fork = nullptr, join[kClasses + kStepStreams] = {};
+    cudaStream_t s[kBatchStreams] = {};  // the classes', the plain-path calls', the groups'
+    cudaEvent_t fork = nullptr, join[kBatchStreams] = {};
     bool ready = false;
 };
 static BatchStreams g_bs;
@@ -488,32 +581,37 @@ static bool batch_streams() {
     std::lock_guard<std::mutex> lk(g_bs_mu);
     if (g_bs.ready) return true;
     bool ok = cuda_ok(cudaEventCreateWithFlags(&g_bs.fork, cudaEventDisableTiming), "batch event");
-    for (int c = 0; c < kClasses + kStepStreams && ok; c++)
+    for (int c = 0; c < kBatchStreams && ok; c++)
         ok = cuda_ok(cudaStreamCreateWithFlags(&g_bs.s[c], cudaStreamNonBlocking), "batch stream") &&
              cuda_ok(cudaEventCreateWithFlags(&g_bs.join[c], cudaEventDisableTiming), "batch event");
     g_bs.ready = ok;
     return ok;
 }
 
-// the plain-path calls on their streams; calls of one plan share its scratch,
-// so they all go to one stream, in order
-static int step_stream(const StepCall &c) { return (int)(((uintptr_t)c.p >> 6) % kStepStreams); }
+
+
+static bool launch_group(const DevBatch &db, const DevBatch::Group &g, cudaStream_t st) {
+    return dif_batch_go(g.cols, db.calls, db.tiles + g.first, g.n, g.nthr, g.smem, st);
+}
 
 static bool launch(const DevBatch &db, cudaStream_t st) {
-    if (db.total == 0 && db.steps.empty()) return true;
+    if (db.total == 0 && db.steps.empty() && db.groups.empty()) return true;
+    if (db.total == 0 && db.steps.empty() && db.groups.size() == 1) return launch_group(db, db.groups[0], st);
     int used = 0, only = 0;
     for (int c = 0; c < kClasses; c++)
         if (db.n[c]) {
             used++;
             only = c;
         }
-    if (used == 1 && db.steps.empty()) return launch_one(db, only, st);
+    if (used == 1 && db.steps.empty() && db.groups.empty()) return launch_one(db, only, st);
     if (!batch_streams()) return false;
     bool ok = cuda_ok(cudaEventRecord(g_bs.fork, st), "batch fork");
     if (!db.steps.empty()) {
+        // calls of one plan share its scratch, so they all go to one stream, in order
         bool on[kStepStreams] = {};
+        std::map<const Plan *, int> stream_of;
         for (const StepCall &c : db.steps) {
-            const int k = step_stream(c);
+            const int k = stream_of.emplace(c.p, (int)stream_of.size() % kStepStreams).first->second;
             cudaStream_t sl = g_bs.s[kClasses + k];
             if (!on[k]) ok = ok && cuda_ok(cudaStreamWaitEvent(sl, g_bs.fork, 0), "batch fork");
             on[k] = true;
@@ -531,12 +629,25 @@ static bool launch(const DevBatch &db, cudaStream_t st) {
              cuda_ok(cudaEventRecord(g_bs.join[c], g_bs.s[c]), "batch join") &&
              cuda_ok(cudaStreamWaitEvent(st, g_bs.join[c], 0), "batch join");
     }
+    const int base = kClasses + kStepStreams, ng = (int)db.groups.size();
+    for (int i = 0; i < ng && ok; i++) {
+        cudaStream_t sg = g_bs.s[base + i % kDifStreams];
+        if (i < kDifStreams) ok = cuda_ok(cudaStreamWaitEvent(sg, g_bs.fork, 0), "batch fork");
+        ok = ok && launch_group(db, db.groups[i], sg);
+    }
+    for (int i = 0; i < std::min(ng, kDifStreams) && ok; i++)
+        ok = cuda_ok(cudaEventRecord(g_bs.join[base + i], g_bs.s[base + i]), "batch join") &&
+             cuda_ok(cudaStreamWaitEvent(st, g_bs.join[base + i], 0), "batch join");
     return ok;
 }
 
 static void free_dev(DevBatch &db) {
     dfree(db.q);
+    dfree(db.calls);
+    dfree(db.tiles);
     db.q = nullptr;
+    db.calls = nullptr;
+    db.tiles = nullptr;
 }
 
 }  // namespace jv
@@ -628,7 +739,7 @@ int jvsip_fftm_batch_run_f(jvsip_fftm_batchplan_f *b) {
     if (!b) return E_ARG;
     Device *d = device();
     if (!d) return E_NODEVICE;
-    if (b->db.total == 0 && b->db.steps.empty()) return 0;
+    if (b->db.total == 0 && b->db.steps.empty() && b->db.groups.empty()) return 0;
     if (!cuda_ok(cudaGraphLaunch(b->exec, d->stream), "batch graph launch")) return E_CUDA;
     count_launch();
     for (const void *blk : b->blocks) {

@@ -175,10 +175,10 @@ struct LongPlan {
 constexpr long kLongFewMin = 8192;
 // Shortest length whose single-precision c2c columns (adjacent vectors) run as
 // two steps whatever their count, unless the register-resident column tiles
-// take the length (fast_step_len: powers of two up to 4096 and 1000).
-// Measured on columns of 3000-7776 points (128-1024 of them): 1.1-1.7x the
-// shared-memory kernel's column tiles; 8192-16384 points: 1.1-3.0x; below,
-// mixed (2187 x 1024: 1.07x, 2560 x 1024: 0.91x, 2400 x 512: 0.70x).
+// take the length (fast_step_len: powers of two up to 4096 and 1000).  Below,
+// one launch of 4- or 8-column tiles is the faster way (2400 x 3495: 52 us
+// against 76 for the shared-memory kernel's tiles); above, the steps
+// (long_columns).
 constexpr long kColStepsMin = 3000;
 
 // Schedule and device tables of the in-place mixed-radix kernel for one length
@@ -199,6 +199,7 @@ const DifTab *dif_acquire(long N, int prec, int cls);  // nullptr: no schedule f
 void dif_release(const DifTab *t);
 bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1);
 bool launch_dif_f32(const Job &j, cudaStream_t s);  // false when the call does not qualify
+bool launch_dif_step_f32(const Job &j, cudaStream_t s);  // a step of a long transform's adjacent vectors
 
 // Kernel entry points (defined in the kernel translation units).
 bool launch_smem_f32(const Job &j, cudaStream_t s);

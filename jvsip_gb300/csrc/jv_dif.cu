@@ -252,13 +252,15 @@ template <typename T> static bool real_pairs(const RView &r, long len, long nvec
            (uintptr_t)r.a % (2 * sizeof(T)) == 0;
 }
 
+// The kernel's arguments for a call and its CTA: tuned > 0 asks for that many
+// transforms (a power of two for column tiles).  False when the call does not
+// qualify.
 template <typename T>
-static bool launch_dif_t(const Job &j, cudaStream_t st) {
+static bool dif_args(const Job &j, long tuned, DifArgs<T> &a, DifCta &cta) {
     typedef typename cplx_t<T>::t C;
     const DifTab *t = j.dif;
-    if (!t || j.no_fast || j.no_dif || j.nvec <= 0 || j.nbatch > 1 || j.tw_lo || j.gram || j.taper_n) return false;
+    if (!t || j.no_fast || j.no_dif || j.nvec <= 0 || j.gram || j.taper_n) return false;
     const CView &ci = j.cin, &co = j.cout;
-    DifArgs<T> a;
     memset(&a, 0, sizeof a);
     bool rows = true, split = false;
     if (j.kind == K_C2C) {
@@ -286,7 +288,8 @@ static bool launch_dif_t(const Job &j, cudaStream_t st) {
         a.vs_in = ci.vs;
         a.es_out = co.es;
         a.vs_out = co.vs;
-        a.smask_in = a.smask_out = j.inv ? 0x80000000u : 0u;
+        a.smask_in = (j.conj_in < 0 ? j.inv : j.conj_in) ? 0x80000000u : 0u;
+        a.smask_out = (j.conj_out < 0 ? j.inv : j.conj_out) ? 0x80000000u : 0u;
     } else if (sizeof(T) != 4 || !j.thalf) {
         return false;
     } else if (j.kind == K_R2C) {
@@ -345,10 +348,15 @@ static bool launch_dif_t(const Job &j, cudaStream_t st) {
     if (rows) {
         vpb = t->vpb;
         nthr = t->nthr;
-        // few transforms: smaller CTAs, so that more SMs work on them
-        while (vpb > 1 && (j.nvec + vpb - 1) / vpb < 2L * device()->sms) {
-            vpb = (vpb + 1) / 2;
-            nthr = std::max(64L, (vpb * j.N / 16 + 31) / 32 * 32);
+        if (tuned > 0 && tuned != vpb) {
+            vpb = std::max(1L, std::min(tuned, (long)(cap / (a.LD * sizeof(C)))));
+            nthr = std::min(512L, std::max(64L, (vpb * j.N / 16 + 31) / 32 * 32));
+        } else if (tuned <= 0) {
+            // few transforms: smaller CTAs, so that more SMs work on them
+            while (vpb > 1 && (j.nvec + vpb - 1) / vpb < 2L * device()->sms) {
+                vpb = (vpb + 1) / 2;
+                nthr = std::max(64L, (vpb * j.N / 16 + 31) / 32 * 32);
+            }
         }
     } else {
         // Column tiles, 64 KB or less: 16 adjacent transforms (128-byte rows of
@@ -359,28 +367,60 @@ static bool launch_dif_t(const Job &j, cudaStream_t st) {
         // 4 x 320 43.2, 8 x 640 50.2; 3000: 4 x 512 53.6, 8 x 1024 59.9.
         const long pts = sizeof(T) == 4 ? 9600 : 4800;
         a.lgv = sizeof(T) == 4 ? 4 : 3;
-        while (a.lgv > 1 && ((1L << a.lgv) * j.N > (a.lgv == 4 ? 4096 : pts))) a.lgv--;
-        if (a.lgv < 2 && sizeof(T) == 4) a.lgv = 2;
+        while (a.lgv > 2 && (j.N << a.lgv) > (a.lgv == 4 ? 4096 : pts)) a.lgv--;
+        if (tuned > 0)
+            for (a.lgv = 0; (2L << a.lgv) <= tuned; a.lgv++) {
+            }
         while (a.lgv > 0 && ((size_t)a.LD << a.lgv) * sizeof(C) > cap) a.lgv--;
         vpb = 1L << a.lgv;
         nthr = std::max(64L, (vpb * j.N / 16 + 31) / 32 * 32);
-        const long maxt = sizeof(T) == 4 ? 1024 : 512;
-        if (nthr > maxt) nthr = maxt;
-        if (sizeof(T) == 4 && nthr > 512 && vpb * j.N <= 16384) nthr = 512;
+        if (nthr > 512) nthr = (sizeof(T) == 4 && vpb * j.N > 16384) ? std::min(1024L, nthr) : 512;
     }
     a.vpb = (int)vpb;
-    const size_t smem = (size_t)a.LD * vpb * sizeof(C);
-    if (smem > cap) return false;
+    cta.nthr = (int)nthr;
+    cta.smem = (size_t)a.LD * vpb * sizeof(C);
+    cta.rows = rows;
+    cta.split = split;
+    return cta.smem <= cap;
+}
+
+template <typename T>
+static bool launch_dif_t(const Job &j, cudaStream_t st) {
+    DifArgs<T> a;
+    DifCta c;
+    if (j.nbatch > 1 || j.tw_lo || !dif_args<T>(j, 0, a, c)) return false;
     if constexpr (sizeof(T) == 4) {
-        if (j.kind == K_R2C) return dif_go<T, DIF_R2C, false>(a, (int)nthr, smem, st);
-        if (j.kind == K_C2R) return dif_go<T, DIF_C2R, false>(a, (int)nthr, smem, st);
-        if (split)
-            return rows ? dif_go<T, DIF_SPLIT, false>(a, (int)nthr, smem, st)
-                        : dif_go<T, DIF_SPLIT, true>(a, (int)nthr, smem, st);
-    } else if (split) {
+        if (j.kind == K_R2C) return dif_go<T, DIF_R2C, false>(a, c.nthr, c.smem, st);
+        if (j.kind == K_C2R) return dif_go<T, DIF_C2R, false>(a, c.nthr, c.smem, st);
+        if (c.split)
+            return c.rows ? dif_go<T, DIF_SPLIT, false>(a, c.nthr, c.smem, st)
+                          : dif_go<T, DIF_SPLIT, true>(a, c.nthr, c.smem, st);
+    } else if (c.split) {
         return false;
     }
-    return rows ? dif_go<T, DIF_C2C, false>(a, (int)nthr, smem, st) : dif_go<T, DIF_C2C, true>(a, (int)nthr, smem, st);
+    return c.rows ? dif_go<T, DIF_C2C, false>(a, c.nthr, c.smem, st) : dif_go<T, DIF_C2C, true>(a, c.nthr, c.smem, st);
+}
+
+// A step of a long transform of several adjacent vectors: column tiles, a
+// group per grid row.
+bool launch_dif_step_f32(const Job &j, cudaStream_t st) {
+    DifArgs<float> a;
+    DifCta c;
+    if (j.kind != K_C2C || j.nbatch < 1 || j.nbatch > 65535 || !dif_args<float>(j, 0, a, c) || c.rows || c.split)
+        return false;
+    a.bvs_in = j.bvs_in;
+    a.bvs_out = j.bvs_out;
+    a.tw_lo = (const float2 *)j.tw_lo;
+    a.tw_hi = (const float2 *)j.tw_hi;
+    a.tw_mask = j.tw_mask;
+    a.tw_sh = j.tw_sh;
+    a.tw_ts = j.tw_ts;
+    a.tw_ys = j.tw_ys;
+    return dif_step_go(a, c.nthr, c.smem, st, (unsigned)j.nbatch);
+}
+
+bool dif_tile_args(const Job &j, long tuned, DifArgs<float> &a, DifCta &c) {
+    return j.kind == K_C2C && dif_args<float>(j, tuned, a, c) && !c.split;
 }
 
 bool launch_dif_f32(const Job &j, cudaStream_t st) { return launch_dif_t<float>(j, st); }

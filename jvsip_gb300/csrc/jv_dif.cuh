@@ -46,12 +46,19 @@ template <typename T> struct DifArgs {
     int has_scale;
     T scale;
     const C *tw;             // per-pass tables: pass p at p.two, entry k*S + n = exp(-2 pi i k n/M)
+    // the steps of a long transform (DIF_STEP): group y of the grid starts
+    // y*bvs_in / y*bvs_out elements on, and output k of its transform t is
+    // multiplied by W^(g*k), g = t*tw_ts + y*tw_ys (none when tw_lo is null),
+    // W^m = tw_lo[m & tw_mask] * tw_hi[m >> tw_sh]
+    long bvs_in, bvs_out;
+    const C *tw_lo, *tw_hi;
+    unsigned tw_mask, tw_sh, tw_ts, tw_ys;
     const C *thalf;          // real transforms: exp(-+ i pi k/N), k <= N
     unsigned mH;             // and the magic of the pair passes' work items per transform
     DifPass p[kDifMaxPass];
 };
 
-enum DifKind { DIF_C2C = 0, DIF_SPLIT = 1, DIF_R2C = 2, DIF_C2R = 3 };
+enum DifKind { DIF_C2C = 0, DIF_SPLIT = 1, DIF_R2C = 2, DIF_C2R = 3, DIF_STEP = 4 };
 
 template <int KIND, typename T>
 __device__ __forceinline__ typename cplx_t<T>::t dif_in(const DifArgs<T> &a, long e) {
@@ -87,7 +94,8 @@ __device__ __forceinline__ void dif_first(const DifArgs<T> &a, typename cplx_t<T
             t = mdiv(b, p.mNR);
             j = b - t * S;
         }
-        const long e0 = (v0 + t) * a.vs_in + (COLS ? (long)j * a.es_in : (long)j);
+        long e0 = (v0 + t) * a.vs_in + (COLS ? (long)j * a.es_in : (long)j);
+        if constexpr (KIND == DIF_STEP) e0 += blockIdx.y * a.bvs_in;
         C v[R];
         if constexpr (COLS) {
             const long st = (long)S * a.es_in;
@@ -175,8 +183,17 @@ __device__ __forceinline__ void dif_last(const DifArgs<T> &a, const typename cpl
 #pragma unroll
         for (int r = 0; r < R; r++) v[r] = COLS ? d[r * V] : d[r];
         Dft<C, R>::run(v);
-        const long e0 = (v0 + t) * a.vs_out + (COLS ? (long)q * a.es_out : (long)q);
+        long e0 = (v0 + t) * a.vs_out + (COLS ? (long)q * a.es_out : (long)q);
         const long st = COLS ? (long)Q * a.es_out : (long)Q;
+        if constexpr (KIND == DIF_STEP) {
+            e0 += blockIdx.y * a.bvs_out;
+            if (a.tw_lo) {
+                const unsigned g = (unsigned)(v0 + t) * a.tw_ts + blockIdx.y * a.tw_ys;
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    v[r] = cmul(v[r], tw_two_level(a.tw_lo, a.tw_hi, a.tw_mask, a.tw_sh, g * (unsigned)(q + r * Q)));
+            }
+        }
 #pragma unroll
         for (int r = 0; r < R; r++)
             dif_out<KIND>(a, e0 + r * st, out_value(v[r], a.smask_out, a.has_scale != 0, a.scale));
@@ -342,12 +359,61 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_dif(const __gri
     }
 }
 
+// One tile of a batch of calls: nt transforms from v0 of call `call`.
+struct DifTile {
+    int call, nt;
+    long v0;
+};
+
+// The batching form's kernel: CTA b takes tile b of the queue, its call's
+// arguments copied into shared memory.
+template <bool COLS>
+__global__ void __launch_bounds__(1024) k_dif_batch(const DifArgs<float> *__restrict__ calls,
+                                                    const DifTile *__restrict__ q) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ __align__(16) DifArgs<float> a;
+    float2 *s = reinterpret_cast<float2 *>(smem_raw);
+    const DifTile d = q[blockIdx.x];
+    static_assert(sizeof(DifArgs<float>) % 8 == 0, "copied by 8 bytes");
+    for (int i = threadIdx.x; i < (int)(sizeof(a) / 8); i += blockDim.x)
+        reinterpret_cast<unsigned long long *>(&a)[i] =
+            __ldg(reinterpret_cast<const unsigned long long *>(&calls[d.call]) + i);
+    __syncthreads();
+#define JV_DIF_FIRST(R) (dif_first<DIF_C2C, COLS, R, float>(a, s, d.nt, d.v0))
+    JV_DIF_SWITCH(a.p[0].R, JV_DIF_FIRST)
+#undef JV_DIF_FIRST
+    __syncthreads();
+    for (int i = 1; i + 1 < a.np; i++) {
+#define JV_DIF_MID(R) (dif_mid<COLS, R, float>(a, a.p[i], s, d.nt))
+        JV_DIF_SWITCH(a.p[i].R, JV_DIF_MID)
+#undef JV_DIF_MID
+        __syncthreads();
+    }
+#define JV_DIF_LAST(R) (dif_last<DIF_C2C, COLS, R, float>(a, s, d.nt, d.v0))
+    JV_DIF_SWITCH(a.p[a.np - 1].R, JV_DIF_LAST)
+#undef JV_DIF_LAST
+}
+
+// static shared memory of k_dif_batch (the copied arguments), rounded up
+constexpr size_t kStaticArgs = 1024;
+static_assert(sizeof(DifArgs<float>) <= kStaticArgs, "arguments fit");
+
+// CTA shape of a call
+struct DifCta {
+    int nthr = 0;
+    size_t smem = 0;
+    bool rows = true, split = false;
+};
+bool dif_tile_args(const Job &j, long tuned, DifArgs<float> &a, DifCta &c);  // batch tiles; false: not for k_dif
+bool dif_batch_go(bool cols, const DifArgs<float> *calls, const DifTile *q, int ntiles, int nthr, size_t smem,
+                  cudaStream_t st);
+
 // Launches (nvec + vpb - 1)/vpb CTAs of nthr threads; instances in jv_dif*.cu.
 template <typename T, int KIND, bool COLS>
 bool dif_go(const DifArgs<T> &a, int nthr, size_t smem, cudaStream_t st);
 
 template <typename T, int KIND, bool COLS>
-inline bool dif_launch(const DifArgs<T> &a, int nthr, size_t smem, cudaStream_t st) {
+inline bool dif_launch(const DifArgs<T> &a, int nthr, size_t smem, cudaStream_t st, unsigned gy = 1) {
     static std::atomic<bool> attr{false};  // set once; concurrent first calls both set it
     if (!attr) {
         if (!cuda_ok(cudaFuncSetAttribute(k_dif<T, KIND, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -358,7 +424,7 @@ inline bool dif_launch(const DifArgs<T> &a, int nthr, size_t smem, cudaStream_t 
     }
     const long grid = (a.nvec + a.vpb - 1) / a.vpb;
     if (grid > 0x7fffffffL) return false;
-    k_dif<T, KIND, COLS><<<(unsigned)grid, (unsigned)nthr, smem, st>>>(a);
+    k_dif<T, KIND, COLS><<<dim3((unsigned)grid, gy), (unsigned)nthr, smem, st>>>(a);
     count_launch();
     return cuda_ok(cudaGetLastError(), "k_dif launch");
 }
@@ -376,5 +442,6 @@ JV_DIF_DECLARE(float, DIF_SPLIT, false)
 JV_DIF_DECLARE(float, DIF_SPLIT, true)
 JV_DIF_DECLARE(float, DIF_R2C, false)
 JV_DIF_DECLARE(float, DIF_C2R, false)
+bool dif_step_go(const DifArgs<float> &a, int nthr, size_t smem, cudaStream_t st, unsigned groups);
 
 }  // namespace jv

@@ -274,6 +274,8 @@ static bool step_job(Job &q, const Job &j, const Plan *sp) {
     q.thalf = nullptr;
     q.form = 0;
     q.no_fast = true;
+    q.dif = j.no_fast ? nullptr : sp->dif;
+    q.no_dif = false;
     q.tma_columns = j.tma_columns;
     q.npass = (int)sp->radix.size();
     if (q.npass > 40) return false;
@@ -281,6 +283,18 @@ static bool step_job(Job &q, const Job &j, const Plan *sp) {
     q.inplace = 0;
     q.lp = nullptr;
     return true;
+}
+
+// One step: on the register-resident kernel's column tiles at its lengths
+// (groups along the grid's y), else on the in-place mixed-radix kernel's
+// (adjacent vectors), else on the shared-memory kernel.
+static bool long_step_f32(Job &q, cudaStream_t st) {
+    if (launch_fast_step_f32(q, st)) return true;
+    if (jvsip_gpu_last_error()) return false;
+    q.no_fast = false;
+    if (launch_dif_step_f32(q, st)) return true;
+    q.no_fast = true;
+    return !jvsip_gpu_last_error() && launch_smem_f32(q, st);
 }
 
 // The two steps of one c2c transform family: N-point transforms of the view
@@ -366,14 +380,7 @@ static bool two_steps(const Job &j, LongPlan *lp, const CView &in, const CView &
         b.bvs_out = out.es;
     }
     if (j.prec == P_F32) {
-        // steps of lengths the register-resident kernel takes as column tiles
-        // (groups along the grid's y)
-        const bool fa = launch_fast_step_f32(a, st);
-        if (!fa && jvsip_gpu_last_error()) return false;
-        if (!fa && !launch_smem_f32(a, st)) return false;
-        const bool fb = launch_fast_step_f32(b, st);
-        if (!fb && jvsip_gpu_last_error()) return false;
-        return fb || launch_smem_f32(b, st);
+        return long_step_f32(a, st) && long_step_f32(b, st);
     }
     return launch_smem_f64(a, st) && launch_smem_f64(b, st);
 }
@@ -492,12 +499,13 @@ static bool long_few(const Job &j) {
 }
 // single-precision c2c columns (adjacent vectors on both sides) of a length
 // with a decomposition from kColStepsMin points, not taken by the
-// register-resident column tiles: two steps whatever their count.  Measured
-// against the shared-memory kernel's column tiles: 16384 x 1024: 3001 against
-// 1013 GB/s (1799 before the steps ran on the register-resident column tiles);
-// 10000 x 1024: 1840 against 917; 8192 x 2048: 2980 against 1436; 7000 x 512:
-// 1319 against 782; 3000 x 1024: 1164 against 874 (and slower than the
-// register-resident tiles themselves: 4096 x 1024: 1457 against 2283).
+// register-resident column tiles: two steps whatever their count.  Measured on
+// 1000 columns (us), the steps on the in-place mixed-radix kernel against the
+// shared-memory kernel's: 3000 points 27.4 against 36.5, 6000: 45.2 against
+// 57.1, 12000: 83.5 against 112.5; steps of lengths that the register-resident
+// tiles take run there (16384 x 1000: 88).  One launch of the in-place
+// kernel's 4-column tiles instead: 3000 points 26.8, 3125: 36.9 (34.8 in the
+// steps), 4000 and longer slower.
 static bool long_columns(const Job &j) {
     return j.lp && j.kind == K_C2C && j.prec == P_F32 && j.nvec > 1 && j.N >= kColStepsMin && !fast_step_len(j.N) &&
            labs(j.cin.vs) == 1 && labs(j.cout.vs) == 1;
