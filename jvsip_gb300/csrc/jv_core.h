@@ -160,15 +160,29 @@ void count_launch_undo(unsigned long long n);  // launches recorded by a capture
 struct LongPlan {
     long N1 = 0, N2 = 0;
     struct Plan *p1 = nullptr, *p2 = nullptr;  // c2c plans of N1 and N2 points (schedules, tables)
-    // single vectors of 2^k points (f32): passes of radix sp_radix[i] (64..2048)
-    // in the register-resident kernel's column tiles, plans of those lengths
+    // single vectors of 2^13..2^20 points (f32): passes of radix sp_radix[i]
+    // (64..1024) in the register-resident kernel's column tiles, plans of those lengths
     std::vector<long> sp_radix;
     std::vector<struct Plan *> sp_plans;
+    struct VecPlan *vec = nullptr;             // single vectors (f32): the passes of launch_vec_f32
     void *d_lo = nullptr, *d_hi = nullptr;     // two-level table of W_N^m: lo[m & mask] * hi[m >> sh]
     unsigned mask = 0, sh = 0;
     void *scratch = nullptr;                   // nvec * N complex, allocated at the first call
     size_t scratch_bytes = 0;
 };
+
+// A single vector of N = f[0]*f[1]*f[2] points (f[1] = 1: two passes) on the
+// in-place mixed-radix kernel: tables of its passes (jv_dif.cu).
+struct VecPlan {
+    long f[3] = {0, 0, 0};
+    const DifTab *tab[3] = {nullptr, nullptr, nullptr};
+    void *d_t1 = nullptr, *d_t2 = nullptr;
+};
+VecPlan *vec_acquire(long N);
+void vec_release(VecPlan *v);
+bool launch_vec_f32(const VecPlan &v, const float2 *in, float2 *out, float2 *scratch, const float2 *lo, const float2 *hi,
+                    unsigned mask, unsigned sh, int conj_in, int conj_out, int has_scale, float scale, cudaStream_t st);
+constexpr long kVecTwoMax = 1L << 20;  // longest vector taken in two passes
 
 // Shortest length run as two steps when a plan has fewer transforms than half
 // the SMs (one CTA per transform would leave most of the GPU idle).

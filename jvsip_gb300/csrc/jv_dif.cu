@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <new>
 #include <tuple>
 
 #include "jv_dif.cuh"
@@ -252,6 +253,30 @@ template <typename T> static bool real_pairs(const RView &r, long len, long nvec
            (uintptr_t)r.a % (2 * sizeof(T)) == 0;
 }
 
+// the schedule's part of the kernel's arguments
+template <typename T> static void dif_fill(DifArgs<T> &a, const DifTab &t) {
+    a.N = (int)t.N;
+    a.np = (int)t.radix.size();
+    a.P1 = (int)t.P1;
+    a.LD = (int)(t.radix[0] * t.P1);
+    a.tw = (const typename cplx_t<T>::t *)t.d_tw;
+    long M = t.N;
+    for (int i = 0; i < a.np; i++) {
+        DifPass &p = a.p[i];
+        p.R = t.radix[i];
+        p.S = (int)(M / p.R);
+        p.NR = (int)(t.N / p.R);
+        p.mstep = (int)M - p.S;
+        p.NB1 = (int)(t.N / t.radix[0] / p.R);
+        p.two = t.two[i];
+        p.mNR = magic_host((unsigned long)p.NR);
+        p.mNB1 = magic_host((unsigned long)p.NB1);
+        p.mS = magic_host((unsigned long)p.S);
+        p.mR = magic_host((unsigned long)p.R);
+        M = p.S;
+    }
+}
+
 // The kernel's arguments for a call and its CTA: tuned > 0 asks for that many
 // transforms (a power of two for column tiles).  False when the call does not
 // qualify.
@@ -319,28 +344,9 @@ static bool dif_args(const Job &j, long tuned, DifArgs<T> &a, DifCta &cta) {
         a.thalf = (const C *)j.thalf;
     }
     a.nvec = j.nvec;
-    a.N = (int)j.N;
-    a.np = (int)t->radix.size();
-    a.P1 = (int)t->P1;
-    a.LD = (int)(t->radix[0] * t->P1);
     a.has_scale = j.has_scale;
     a.scale = j.has_scale ? (T)j.scale : (T)1;
-    a.tw = (const C *)t->d_tw;
-    long M = j.N;
-    for (int i = 0; i < a.np; i++) {
-        DifPass &p = a.p[i];
-        p.R = t->radix[i];
-        p.S = (int)(M / p.R);
-        p.NR = (int)(j.N / p.R);
-        p.mstep = (int)M - p.S;
-        p.NB1 = (int)(j.N / t->radix[0] / p.R);
-        p.two = t->two[i];
-        p.mNR = magic_host((unsigned long)p.NR);
-        p.mNB1 = magic_host((unsigned long)p.NB1);
-        p.mS = magic_host((unsigned long)p.S);
-        p.mR = magic_host((unsigned long)p.R);
-        M = p.S;
-    }
+    dif_fill(a, *t);
     if (j.kind == K_R2C) a.mH = magic_host((unsigned long)(a.p[a.np - 1].NR / 2 + 1));
     if (j.kind == K_C2R) a.mH = magic_host((unsigned long)(a.p[0].S / 2 + 1));
     const size_t cap = device()->smem_optin;
@@ -417,6 +423,164 @@ bool launch_dif_step_f32(const Job &j, cudaStream_t st) {
     a.tw_ts = j.tw_ts;
     a.tw_ys = j.tw_ys;
     return dif_step_go(a, c.nthr, c.smem, st, (unsigned)j.nbatch);
+}
+
+// ---------------------------------------------------------------- single long vectors
+// N = A*B*C (or A*C, B = 1) points of one vector: with n = n1*BC + r and k =
+// k1 + A*(k2 + B*k3), pass 1 transforms over n1 (A points BC apart, 16
+// adjacent r per tile) and twiddles by W_N^(k1 r) into scratch[k1*BC + r];
+// pass 2 does the same inside every block of BC over n2 (twiddle W_BC^(k2 n3),
+// in place); the last pass transforms rows of C points and stores output k3 of
+// 16 adjacent k1 side by side at y[k1 + A*(k2 + B*k3)].  Every pass reads and
+// writes segments of 128 bytes or more, and every twiddle is a coalesced table
+// load (pass 1: W_N^(k1 r0) of the tile's first r, computed once per tile, times
+// W_N^(k1 t); pass 2: the whole table of BC entries), where the Stockham passes
+// before took two gathers per point.
+static double vec_cost(long n) {
+    std::vector<int> r;
+    long P1;
+    if (n < 16 || n > 1024 || !dif_schedule(n, P_F32, 0, r, &P1)) return 1e30;
+    double c = 25;  // global accesses and the pass's own twiddle
+    for (int R : r) c += pass_cost(R, P_F32);
+    return n > 512 ? c * 1.3 : c;  // tiles of 8 transforms
+}
+
+// Two factors up to kVecTwoMax points where there are two, by cost otherwise
+// (2^20 points measured the same in two passes of 1024 and in three).
+bool vec_factors(long N, long f[3]) {
+    double best = 1e29;
+    f[0] = f[1] = f[2] = 0;
+    std::vector<long> d;
+    std::map<long, double> cost;
+    for (long a = 16; a <= 1024; a++)
+        if (N % a == 0 && vec_cost(a) < 1e29) {
+            d.push_back(a);
+            cost[a] = vec_cost(a);
+        }
+    for (long a : d) {
+        const long m = N / a;
+        if (cost.count(m) && N <= kVecTwoMax && cost[a] + cost[m] < best) {
+            best = cost[a] + cost[m];
+            f[0] = a;
+            f[1] = 1;
+            f[2] = m;
+        }
+        if (N <= kVecTwoMax && f[1] == 1) continue;
+        for (long b : d)
+            if (m % b == 0 && cost.count(m / b) && cost[a] + cost[b] + cost[m / b] < best) {
+                best = cost[a] + cost[b] + cost[m / b];
+                f[0] = a;
+                f[1] = b;
+                f[2] = m / b;
+            }
+    }
+    return f[0] != 0;
+}
+
+template <typename F> static void *upload_roots(long n, F exponent, long N) {
+    std::vector<float> t(2 * n);
+    for (long i = 0; i < n; i++) {
+        double c, s;
+        root(exponent(i) % N, N, &c, &s);
+        t[2 * i] = (float)c;
+        t[2 * i + 1] = (float)s;
+    }
+    void *d = dmalloc(t.size() * sizeof(float));
+    if (d && !cuda_ok(cudaMemcpy(d, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice), "twiddle upload")) {
+        dfree(d);
+        d = nullptr;
+    }
+    return d;
+}
+
+// adjacent transforms per tile: 128-byte segments, fewer while they leave SMs idle
+static long vec_tile(long n, long N) {
+    long v = n > 512 ? 8 : 16;
+    while (v > 4 && N / n / v < 2L * device()->sms) v /= 2;
+    return v;
+}
+
+void vec_release(VecPlan *v) {
+    if (!v) return;
+    for (const DifTab *t : v->tab) dif_release(t);
+    dfree(v->d_t1);
+    dfree(v->d_t2);
+    delete v;
+}
+
+// nullptr when N does not factor so, or without memory (the other paths take
+// the vector).
+VecPlan *vec_acquire(long N) {
+    long f[3];
+    if (N >= (1L << 31) || !vec_factors(N, f)) return nullptr;
+    const int err0 = jvsip_gpu_last_error();
+    VecPlan *v = new (std::nothrow) VecPlan();
+    if (!v) return nullptr;
+    const long V = vec_tile(f[0], N), BC = f[1] * f[2];
+    bool ok = true;
+    for (int i = 0; i < 3; i++) {
+        v->f[i] = f[i];
+        if (f[i] > 1) ok = ok && (v->tab[i] = dif_acquire(f[i], P_F32, 0)) != nullptr;
+    }
+    ok = ok && (v->d_t1 = upload_roots(f[0] * V, [&](long i) { return (i / V) * (i % V); }, N)) != nullptr;
+    const long C = f[2];
+    if (ok && f[1] > 1) ok = (v->d_t2 = upload_roots(BC, [&](long i) { return (i / C) * (i % C); }, BC)) != nullptr;
+    if (ok) return v;
+    vec_release(v);
+    if (!err0 && jvsip_gpu_last_error()) jvsip_gpu_clear_error();
+    return nullptr;
+}
+
+// One vector of unit stride from `in` to `out` through `scratch` (N points).
+bool launch_vec_f32(const VecPlan &v, const float2 *in, float2 *out, float2 *scratch, const float2 *lo, const float2 *hi,
+                    unsigned mask, unsigned sh, int conj_in, int conj_out, int has_scale, float scale, cudaStream_t st) {
+    const long A = v.f[0], B = v.f[1], C = v.f[2];
+    for (int i = 0; i < 3; i++) {
+        if (!v.tab[i]) continue;
+        DifArgs<float> a;
+        memset(&a, 0, sizeof a);
+        dif_fill(a, *v.tab[i]);
+        const long V = vec_tile(a.N, A * B * C);
+        a.lgv = V == 16 ? 4 : V == 8 ? 3 : 2;
+        a.vpb = (int)V;
+        a.scale = 1.f;
+        size_t smem;
+        unsigned groups = 1;
+        a.in = i == 0 ? in : scratch;
+        a.out = i == 2 ? out : scratch;
+        if (i < 2) {
+            const long cols = i == 0 ? B * C : C;
+            a.es_in = a.es_out = a.nvec = cols;
+            a.vs_in = a.vs_out = 1;
+            a.bvs_in = a.bvs_out = B * C;
+            groups = i == 0 ? 1u : (unsigned)A;
+            a.tv = (const float2 *)(i == 0 ? v.d_t1 : v.d_t2);
+            a.tv_st = (int)C;
+            a.tw_lo = lo;
+            a.tw_hi = hi;
+            a.tw_mask = mask;
+            a.tw_sh = sh;
+            a.smask_in = i == 0 && conj_in ? 0x80000000u : 0u;
+            smem = ((size_t)a.LD * V + (i == 0 ? a.N : 0)) * sizeof(float2);
+        } else {
+            a.LD |= 1;
+            a.es_in = 1;
+            a.vs_in = B * C;
+            a.bvs_in = C;
+            a.nvec = A;
+            a.es_out = A * B;
+            a.vs_out = 1;
+            a.bvs_out = A;
+            groups = (unsigned)B;
+            a.smask_out = conj_out ? 0x80000000u : 0u;
+            a.has_scale = has_scale;
+            if (has_scale) a.scale = scale;
+            smem = (size_t)a.LD * V * sizeof(float2);
+        }
+        const int nthr = (int)std::min(512L, std::max(64L, (V * a.N / 16 + 31) / 32 * 32));
+        if (!dif_vec_go(i == 0 ? DIF_VEC1 : i == 1 ? DIF_VEC2 : DIF_VECR, a, nthr, smem, st, groups)) return false;
+    }
+    return true;
 }
 
 bool dif_tile_args(const Job &j, long tuned, DifArgs<float> &a, DifCta &c) {

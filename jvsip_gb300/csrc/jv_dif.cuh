@@ -53,12 +53,19 @@ template <typename T> struct DifArgs {
     long bvs_in, bvs_out;
     const C *tw_lo, *tw_hi;
     unsigned tw_mask, tw_sh, tw_ts, tw_ys;
+    const C *tv;             // DIF_VEC1, DIF_VEC2: output k of transform t times tv[k*tv_st + t]
+    int tv_st;
     const C *thalf;          // real transforms: exp(-+ i pi k/N), k <= N
     unsigned mH;             // and the magic of the pair passes' work items per transform
     DifPass p[kDifMaxPass];
 };
 
-enum DifKind { DIF_C2C = 0, DIF_SPLIT = 1, DIF_R2C = 2, DIF_C2R = 3, DIF_STEP = 4 };
+// DIF_VEC1, DIF_VEC2, DIF_VECR: the passes over a single long vector
+// (launch_vec_f32)
+enum DifKind {
+    DIF_C2C = 0, DIF_SPLIT = 1, DIF_R2C = 2, DIF_C2R = 3, DIF_STEP = 4, DIF_VEC1 = 5, DIF_VEC2 = 6, DIF_VECR = 7
+};
+template <int KIND> constexpr bool dif_groups() { return KIND >= DIF_STEP; }
 
 template <int KIND, typename T>
 __device__ __forceinline__ typename cplx_t<T>::t dif_in(const DifArgs<T> &a, long e) {
@@ -95,7 +102,7 @@ __device__ __forceinline__ void dif_first(const DifArgs<T> &a, typename cplx_t<T
             j = b - t * S;
         }
         long e0 = (v0 + t) * a.vs_in + (COLS ? (long)j * a.es_in : (long)j);
-        if constexpr (KIND == DIF_STEP) e0 += blockIdx.y * a.bvs_in;
+        if constexpr (dif_groups<KIND>()) e0 += blockIdx.y * a.bvs_in;
         C v[R];
         if constexpr (COLS) {
             const long st = (long)S * a.es_in;
@@ -166,14 +173,17 @@ template <int KIND, bool COLS, int R, typename T>
 __device__ __forceinline__ void dif_last(const DifArgs<T> &a, const typename cplx_t<T>::t *s, int nt, long v0) {
     typedef typename cplx_t<T>::t C;
     const DifPass &p = a.p[a.np - 1];
-    const int Q = p.NR, V = COLS ? a.vpb : 1;
-    const int nb = COLS ? Q : nt * Q;
-    const int step = COLS ? (int)blockDim.x >> a.lgv : (int)blockDim.x;
-    const int ct = COLS ? ((int)threadIdx.x & (V - 1)) : 0;
-    if (COLS && ct >= nt) return;
-    for (int b = COLS ? (int)threadIdx.x >> a.lgv : (int)threadIdx.x; b < nb; b += step) {
+    // stores with consecutive threads on adjacent transforms: column tiles,
+    // and the rows of a long vector's last pass
+    constexpr bool TF = COLS || KIND == DIF_VECR;
+    const int Q = p.NR, V = TF ? a.vpb : 1;
+    const int nb = TF ? Q : nt * Q;
+    const int step = TF ? (int)blockDim.x >> a.lgv : (int)blockDim.x;
+    const int ct = TF ? ((int)threadIdx.x & (V - 1)) : 0;
+    if (TF && ct >= nt) return;
+    for (int b = TF ? (int)threadIdx.x >> a.lgv : (int)threadIdx.x; b < nb; b += step) {
         int t = ct, q = b;
-        if (!COLS && a.vpb > 1) {
+        if (!TF && a.vpb > 1) {
             t = mdiv(b, p.mNR);
             q = b - t * Q;
         }
@@ -183,16 +193,27 @@ __device__ __forceinline__ void dif_last(const DifArgs<T> &a, const typename cpl
 #pragma unroll
         for (int r = 0; r < R; r++) v[r] = COLS ? d[r * V] : d[r];
         Dft<C, R>::run(v);
-        long e0 = (v0 + t) * a.vs_out + (COLS ? (long)q * a.es_out : (long)q);
-        const long st = COLS ? (long)Q * a.es_out : (long)Q;
+        long e0 = (v0 + t) * a.vs_out + (TF ? (long)q * a.es_out : (long)q);
+        const long st = TF ? (long)Q * a.es_out : (long)Q;
+        if constexpr (dif_groups<KIND>()) e0 += blockIdx.y * a.bvs_out;
         if constexpr (KIND == DIF_STEP) {
-            e0 += blockIdx.y * a.bvs_out;
             if (a.tw_lo) {
                 const unsigned g = (unsigned)(v0 + t) * a.tw_ts + blockIdx.y * a.tw_ys;
 #pragma unroll
                 for (int r = 0; r < R; r++)
                     v[r] = cmul(v[r], tw_two_level(a.tw_lo, a.tw_hi, a.tw_mask, a.tw_sh, g * (unsigned)(q + r * Q)));
             }
+        }
+        if constexpr (KIND == DIF_VEC1) {
+            // W_N^(k (v0 + t)) = base[k] * W_N^(k t)
+            const C *base = s + a.LD * V + q, *w = a.tv + (q * V + t);
+#pragma unroll
+            for (int r = 0; r < R; r++) v[r] = cmul(v[r], cmul(base[r * Q], __ldg(w + r * Q * V)));
+        }
+        if constexpr (KIND == DIF_VEC2) {
+            const C *w = a.tv + ((long)q * a.tv_st + v0 + t);
+#pragma unroll
+            for (int r = 0; r < R; r++) v[r] = cmul(v[r], __ldg(w + r * Q * a.tv_st));
         }
 #pragma unroll
         for (int r = 0; r < R; r++)
@@ -332,6 +353,11 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_dif(const __gri
     C *s = reinterpret_cast<C *>(smem_raw);
     const long v0 = (long)blockIdx.x * a.vpb;
     const int nt = (int)min((long)a.vpb, a.nvec - v0);
+    if constexpr (KIND == DIF_VEC1) {
+        // W_N^(k v0), k < the pass's length (k v0 < N), behind the tile
+        for (int k = threadIdx.x; k < a.N; k += blockDim.x)
+            s[a.LD * a.vpb + k] = tw_two_level(a.tw_lo, a.tw_hi, a.tw_mask, a.tw_sh, (unsigned)k * (unsigned)v0);
+    }
     if constexpr (KIND == DIF_C2R) {
 #define JV_DIF_FIRST(R) (dif_first_c2r<R, T>(a, s, nt, v0))
         JV_DIF_PAIR_SWITCH(a.p[0].R, JV_DIF_FIRST)
@@ -443,5 +469,6 @@ JV_DIF_DECLARE(float, DIF_SPLIT, true)
 JV_DIF_DECLARE(float, DIF_R2C, false)
 JV_DIF_DECLARE(float, DIF_C2R, false)
 bool dif_step_go(const DifArgs<float> &a, int nthr, size_t smem, cudaStream_t st, unsigned groups);
+bool dif_vec_go(int kind, const DifArgs<float> &a, int nthr, size_t smem, cudaStream_t st, unsigned groups);
 
 }  // namespace jv

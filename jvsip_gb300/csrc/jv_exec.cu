@@ -385,6 +385,17 @@ static bool two_steps(const Job &j, LongPlan *lp, const CView &in, const CView &
     return launch_smem_f64(a, st) && launch_smem_f64(b, st);
 }
 
+// The transforms of `in` into `out`: a single vector of unit stride in the
+// plan's passes over it (launch_vec_f32) when it has them, else the two steps.
+static bool long_c2c(const Job &j, LongPlan *lp, const CView &in, const CView &out, long nv, int conj_in, int conj_out,
+                     int has_scale, double scale, char *sc, size_t esz, cudaStream_t st) {
+    if (lp->vec && nv == 1 && in.es == 1 && out.es == 1)
+        return launch_vec_f32(*lp->vec, (const float2 *)in.re + in.off, (float2 *)out.re + out.off, (float2 *)sc,
+                              (const float2 *)lp->d_lo, (const float2 *)lp->d_hi, lp->mask, lp->sh, conj_in, conj_out,
+                              has_scale, (float)scale, st);
+    return two_steps(j, lp, in, out, nv, conj_in, conj_out, has_scale, scale, sc, esz, st);
+}
+
 // A single vector of 2^n points (single precision, interleaved, unit stride)
 // as large-radix Stockham passes (LongPlan::sp_radix): pass p reads element n
 // of transform j at j + n*N/R_p, multiplies it by W_N^(n*m*N/(Ns*R_p)),
@@ -521,26 +532,21 @@ static bool run_long(Job &j, cudaStream_t st, bool *handled) {
     if (j.kind == K_R2C && !(interleaved(j.cout, esz) && real_as_complex(j.rin, j.nvec, esz, &zin))) return false;
     const long N = j.N, nv = j.nvec;
     const size_t one = (size_t)nv * N * 2 * esz;
-    // single vectors of unit stride take the Stockham passes when planned:
-    // c2c, and R2C (the half-length transform of the pairs, then the split)
-    // when it has three passes or more (measured: R2C of 2^24 points 892 GB/s
-    // in the two steps, 815 in two passes; 2^26 points 715 against 891)
-    const bool sp = !lp->sp_radix.empty() && nv == 1 && j.prec == P_F32 && j.cout.es == 1 &&
-                    ((j.kind == K_C2C && j.cin.es == 1) || (j.kind == K_R2C && lp->sp_radix.size() >= 3));
+    // single c2c vectors of unit stride take the Stockham passes when planned
+    const bool sp = !lp->sp_radix.empty() && nv == 1 && j.prec == P_F32 && j.kind == K_C2C && j.cout.es == 1 &&
+                    j.cin.es == 1;
     // the plan's call shape is fixed, so the scratch is sized once: a captured
     // call's graph holds its address, and it is never reallocated while the
     // plan lives
     *handled = true;
     if (!long_scratch(lp, long_scratch_need(j), false)) return false;
     char *sc = (char *)lp->scratch;
-    if (sp && j.kind == K_C2C) return sp_passes(j, lp, j.cin, j.cout, j.inv, j.has_scale, j.scale, sc, esz, st);
+    if (sp) return sp_passes(j, lp, j.cin, j.cout, j.inv, j.has_scale, j.scale, sc, esz, st);
     if (j.kind == K_C2C)
-        return two_steps(j, lp, j.cin, j.cout, nv, j.inv, j.inv, j.has_scale, j.scale, sc, esz, st);
+        return long_c2c(j, lp, j.cin, j.cout, nv, j.inv, j.inv, j.has_scale, j.scale, sc, esz, st);
     if (j.kind == K_R2C) {
         // Z = F(z) into the first N elements of each output vector, then the split
-        const bool ok = sp ? sp_passes(j, lp, zin, j.cout, 0, 0, 1.0, sc, esz, st)
-                           : two_steps(j, lp, zin, j.cout, nv, 0, 0, 0, 1.0, sc, esz, st);
-        if (!ok) return false;
+        if (!long_c2c(j, lp, zin, j.cout, nv, 0, 0, 0, 1.0, sc, esz, st)) return false;
         void *z = (char *)j.cout.re + (size_t)j.cout.off * 2 * esz;
         return j.prec == P_F32
                    ? launch_r2c_pairs_f32(z, j.cout.es, j.cout.vs, N, nv, j.has_scale, j.scale, j.thalf, st)
@@ -559,9 +565,9 @@ static bool run_long(Job &j, cudaStream_t st, bool *handled) {
     if (!ok) return false;
     CView xo;
     if (real_as_complex(j.rout, nv, esz, &xo))
-        return two_steps(j, lp, yv, xo, nv, 0, 1, j.has_scale, j.scale, sc, esz, st);
+        return long_c2c(j, lp, yv, xo, nv, 0, 1, j.has_scale, j.scale, sc, esz, st);
     // other real views: the steps back into the second half, then the final store
-    if (!two_steps(j, lp, yv, yv, nv, 0, 0, 0, 1.0, sc, esz, st)) return false;
+    if (!long_c2c(j, lp, yv, yv, nv, 0, 0, 0, 1.0, sc, esz, st)) return false;
     return j.prec == P_F32 ? launch_c2r_unpack_f32(j, ys, st) : launch_c2r_unpack_f64(j, ys, st);
 }
 

@@ -402,6 +402,7 @@ static void long_free(LongPlan *lp) {
             release_tables(q);
             delete q;
         }
+    vec_release(lp->vec);
     dfree(lp->d_lo);
     dfree(lp->d_hi);
     dfree(lp->scratch);
@@ -500,13 +501,10 @@ static bool build_long(Plan *p) {
         long_free(lp);
         return false;
     }
-    // single vectors of 2^n points, n >= 13 (single precision): large-radix
-    // Stockham passes of 2^6..2^12 points each, larger first -- two up to
-    // 2^23 points (fewer launches for short vectors), else ceil(n/9)
-    if (p->prec == P_F32 && (N & (N - 1)) == 0 && bits >= 13 && bits <= 31) {
-        const unsigned k = bits <= 23 ? 2 : (bits + 8) / 9;
-        std::vector<long> rad;
-        for (unsigned i = 0; i < k; i++) rad.push_back(1L << (bits / k + (i < bits % k ? 1 : 0)));
+    // single vectors of 2^n points, 13 <= n <= 20 (single precision): two
+    // large-radix Stockham passes of 2^6..2^10 points each, larger first
+    if (p->prec == P_F32 && (N & (N - 1)) == 0 && bits >= 13 && bits <= 20) {
+        const std::vector<long> rad = {1L << ((bits + 1) / 2), 1L << (bits / 2)};
         bool ok = true;
         for (long R : rad) ok = ok && R >= 64 && R <= 4096;
         for (size_t i = 0; ok && i < rad.size(); i++) {
@@ -531,6 +529,15 @@ static bool build_long(Plan *p) {
             jvsip_gpu_clear_error();
         }
     }
+    // the other single vectors: passes on the in-place mixed-radix kernel,
+    // unless both steps run on the register-resident column tiles, or one of
+    // two steps of 1536 points and more does on a vector that L2 holds
+    // (1000000 points: 16.6 us in the steps, 20.7 in the passes; 3145728: 43.9
+    // and 50.8; 1572864 = 1024 x 1536: 28.5 and 26.6; 5242880: 92 and 69)
+    const bool f1 = fast_step_len(lp->N1), f2 = fast_step_len(lp->N2);
+    const bool steps = (N & (N - 1)) != 0 && ((f1 && f2) || ((f1 || f2) && lp->N1 >= 1536 && N < (1L << 22)));
+    if (p->prec == P_F32 && p->mN == 1 && !p->no_fast && lp->sp_radix.empty() && !steps)
+        lp->vec = vec_acquire(N);
     p->lp = lp;
     return true;
 }

@@ -160,3 +160,44 @@ def test_routes_agree_with_the_general_kernels(monkeypatch, N):
                 b.destroy()
         assert rel(outs[0], outs[1]) <= tol(N), (cs, rs)
         assert np.array_equal(outs[0] == 0, outs[1] == 0)
+
+
+@pytest.mark.parametrize("N", [8748, 9000, 59049, 100842, 234375, 823543, 1953125, 1 << 21, 3 << 20, 2 * 3 ** 13])
+@pytest.mark.parametrize("inplace", [False, True])
+def test_single_vectors(N, inplace):
+    """Two and three passes over one vector, last tiles that are not full, an
+    offset, both directions; then R2C of 2N real points and C2R back."""
+    z = rnd(N + 2, N)
+    bx = J.CBlock(z.copy().view(np.float32), admit=True)
+    by = bx if inplace else J.CBlock(np.zeros(2 * (N + 2), np.float32), admit=True)
+    vx, vy = bx.vview(1, 1, N), by.vview(1, 1, N)
+    p = J.FFT(J.KIND_CCIP if inplace else J.KIND_CCOP, N, 1.0 / N, J.VSIP_FFT_INV, ntimes=1)
+    if inplace:
+        p.ccfftip(vx)
+    else:
+        p.ccfftop(vx, vy)
+    by.sync()
+    got = by.re.view(np.complex64)
+    assert rel(got[1:-1], np.fft.ifft(z[1:-1].astype(np.complex128))) <= tol(N)
+    assert np.array_equal(got[[0, -1]], z[[0, -1]] if inplace else np.zeros(2))
+    for v in (vx, vy):
+        v.destroy()
+    for b in {bx, by}:
+        b.destroy()
+    if inplace:
+        return
+    x = np.random.default_rng(N).standard_normal(2 * N).astype(np.float32)
+    out = np.zeros(2 * N, np.float32)
+    bx, bz, bo = (J.RBlock(x, admit=True), J.CBlock(np.zeros(2 * (N + 1), np.float32), admit=True),
+                  J.RBlock(out, admit=True))
+    vx, vz, vo = bx.vview(0, 1, 2 * N), bz.vview(0, 1, N + 1), bo.vview(0, 1, 2 * N)
+    J.FFT(J.KIND_RCOP, 2 * N, 1.0, ntimes=1).rcfftop(vx, vz)
+    J.FFT(J.KIND_CROP, 2 * N, 0.5 / N, ntimes=1).crfftop(vz, vo)
+    bz.sync()
+    bo.sync()
+    assert rel(bz.re.view(np.complex64), np.fft.rfft(x.astype(np.float64))) <= tol(2 * N)
+    assert rel(out, x.astype(np.float64)) <= 2 * tol(2 * N)
+    for v in (vx, vz, vo):
+        v.destroy()
+    for b in (bx, bz, bo):
+        b.destroy()
