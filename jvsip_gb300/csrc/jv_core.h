@@ -205,6 +205,7 @@ struct DifTab {
     long P1 = 0;              // shared-memory pitch of a first-pass block
     std::vector<int> two;     // start of each pass's twiddle table
     void *d_tw = nullptr;
+    const struct DifFixEntry *fix = nullptr;  // the length's compiled-in kernels (or null)
     long vpb = 1;             // CTA shape of row calls: transforms, threads
     int nthr = 128;
     int refs = 0;

@@ -125,6 +125,42 @@ bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1) {
     return true;
 }
 
+// ---------------------------------------------------------------- compiled-in schedules
+void dif_fix_c2c_1(std::vector<DifFixEntry> &out);
+void dif_fix_c2c_2(std::vector<DifFixEntry> &out);
+void dif_fix_c2c_3(std::vector<DifFixEntry> &out);
+void dif_fix_long_1(std::vector<DifFixEntry> &out);
+void dif_fix_r2c_1(std::vector<DifFixEntry> &out);
+void dif_fix_r2c_2(std::vector<DifFixEntry> &out);
+void dif_fix_c2r_1(std::vector<DifFixEntry> &out);
+void dif_fix_c2r_2(std::vector<DifFixEntry> &out);
+
+const DifFixEntry *dif_fix(long N, int cls) {
+    // built once, thread-safely, on the first call
+    static const std::vector<std::map<long, DifFixEntry>> tab = []() {
+        std::vector<std::map<long, DifFixEntry>> t(3);
+        std::vector<DifFixEntry> v[4];
+        dif_fix_c2c_1(v[0]);
+        dif_fix_c2c_2(v[0]);
+        dif_fix_c2c_3(v[0]);
+        dif_fix_r2c_1(v[1]);
+        dif_fix_r2c_2(v[1]);
+        dif_fix_c2r_1(v[2]);
+        dif_fix_c2r_2(v[2]);
+        dif_fix_long_1(v[3]);
+        for (int c = 0; c < 3; c++)
+            for (const DifFixEntry &e : v[c]) t[c][e.N] = e;
+        for (const DifFixEntry &e : v[3]) {
+            DifFixEntry &d = t[0][e.N];
+            d.step = e.step;
+            for (int i = 0; i < 3; i++) d.vec[i] = e.vec[i];
+        }
+        return t;
+    }();
+    auto it = tab[cls].find(N);
+    return it == tab[cls].end() ? nullptr : &it->second;
+}
+
 // ---------------------------------------------------------------- tables
 static std::mutex g_dif_mu;
 static std::map<std::tuple<long, int, int>, DifTab> g_dif;
@@ -215,7 +251,14 @@ const DifTab *dif_acquire(long N, int prec, int cls) {
         return &it->second;
     }
     DifTab t;
-    if (!dif_schedule(N, prec, cls, t.radix, &t.P1)) return nullptr;
+    const DifFixEntry *fix = prec == P_F32 ? dif_fix(N, cls) : nullptr;
+    if (fix) {
+        t.radix = fix->radix;
+        t.P1 = fix->P1;
+        t.fix = fix;
+    } else if (!dif_schedule(N, prec, cls, t.radix, &t.P1)) {
+        return nullptr;
+    }
     t.N = N;
     t.prec = prec;
     t.cls = cls;
@@ -225,7 +268,12 @@ const DifTab *dif_acquire(long N, int prec, int cls) {
         if (!err0 && jvsip_gpu_last_error()) jvsip_gpu_clear_error();
         return nullptr;
     }
-    row_shape(t, cls);
+    if (fix) {
+        t.vpb = fix->vpb;
+        t.nthr = fix->nthr;
+    } else {
+        row_shape(t, cls);
+    }
     t.refs = 1;
     auto &slot = g_dif[key];
     slot = t;
@@ -374,6 +422,11 @@ static bool dif_args(const Job &j, long tuned, DifArgs<T> &a, DifCta &cta) {
         const long pts = sizeof(T) == 4 ? 9600 : 4800;
         a.lgv = sizeof(T) == 4 ? 4 : 3;
         while (a.lgv > 2 && (j.N << a.lgv) > (a.lgv == 4 ? 4096 : pts)) a.lgv--;
+        if (t->fix && t->fix->vcol)
+            for (a.lgv = 0; (1 << a.lgv) < t->fix->vcol; a.lgv++) {
+            }
+        // few columns: tiles of 4, so that more SMs work on them
+        if (((j.nvec - 1) >> a.lgv) + 1 < device()->sms && j.nbatch <= 1) a.lgv = std::min(a.lgv, 2);
         if (tuned > 0)
             for (a.lgv = 0; (2L << a.lgv) <= tuned; a.lgv++) {
             }
@@ -396,6 +449,10 @@ static bool launch_dif_t(const Job &j, cudaStream_t st) {
     DifCta c;
     if (j.nbatch > 1 || j.tw_lo || !dif_args<T>(j, 0, a, c)) return false;
     if constexpr (sizeof(T) == 4) {
+        const DifFixEntry *f = j.dif->fix;
+        if (f && !c.split && c.rows && f->rows) return f->rows(a, c.smem, st, 1);
+        if (f && !c.split && !c.rows && f->cols && a.vpb == f->vcol) return f->cols(a, c.smem, st, 1);
+        if (f && !c.split && !c.rows && f->cols4 && a.vpb == 4) return f->cols4(a, c.smem, st, 1);
         if (j.kind == K_R2C) return dif_go<T, DIF_R2C, false>(a, c.nthr, c.smem, st);
         if (j.kind == K_C2R) return dif_go<T, DIF_C2R, false>(a, c.nthr, c.smem, st);
         if (c.split)
@@ -422,6 +479,8 @@ bool launch_dif_step_f32(const Job &j, cudaStream_t st) {
     a.tw_sh = j.tw_sh;
     a.tw_ts = j.tw_ts;
     a.tw_ys = j.tw_ys;
+    const DifFixEntry *f = j.dif->fix;
+    if (f && f->step && a.vpb == 16) return f->step(a, c.smem, st, (unsigned)j.nbatch);
     return dif_step_go(a, c.nthr, c.smem, st, (unsigned)j.nbatch);
 }
 
@@ -439,10 +498,14 @@ bool launch_dif_step_f32(const Job &j, cudaStream_t st) {
 static double vec_cost(long n) {
     std::vector<int> r;
     long P1;
-    if (n < 16 || n > 1024 || !dif_schedule(n, P_F32, 0, r, &P1)) return 1e30;
+    if (n < 16 || n > 1024) return 1e30;
+    const DifFixEntry *fix = dif_fix(n, 0);
+    if (fix) r = fix->radix;
+    else if (!dif_schedule(n, P_F32, 0, r, &P1)) return 1e30;
     double c = 25;  // global accesses and the pass's own twiddle
     for (int R : r) c += pass_cost(R, P_F32);
-    return n > 512 ? c * 1.3 : c;  // tiles of 8 transforms
+    if (fix && fix->vec[0]) return c;
+    return n > 512 ? c * 1.3 : c * 1.15;  // tiles of 8 transforms; no compiled-in schedule
 }
 
 // Two factors up to kVecTwoMax points where there are two, by cost otherwise
@@ -578,6 +641,11 @@ bool launch_vec_f32(const VecPlan &v, const float2 *in, float2 *out, float2 *scr
             smem = (size_t)a.LD * V * sizeof(float2);
         }
         const int nthr = (int)std::min(512L, std::max(64L, (V * a.N / 16 + 31) / 32 * 32));
+        const DifFixEntry *f = v.tab[i]->fix;
+        if (f && f->vec[i] && V == 16) {
+            if (!f->vec[i](a, smem, st, groups)) return false;
+            continue;
+        }
         if (!dif_vec_go(i == 0 ? DIF_VEC1 : i == 1 ? DIF_VEC2 : DIF_VECR, a, nthr, smem, st, groups)) return false;
     }
     return true;

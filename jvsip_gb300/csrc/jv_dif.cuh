@@ -24,12 +24,26 @@ namespace jv {
 
 constexpr int kDifMaxPass = 8;
 
+// A pass's constants, read from the arguments ...
 struct DifPass {
     int R, S;            // radix; distance of a butterfly's elements inside a k1 block
     int NR, mstep;       // butterflies per transform N/R; M - S
     int NB1, two;        // butterflies per k1 block; start of the pass's twiddle table
     unsigned mNR, mNB1;  // multiply-high magic of NR, NB1
     unsigned mS, mR;     // of S, R
+    __device__ __forceinline__ int by_NR(int x) const { return mdiv(x, mNR); }
+    __device__ __forceinline__ int by_NB1(int x) const { return mdiv(x, mNB1); }
+    __device__ __forceinline__ int by_S(int x) const { return mdiv(x, mS); }
+    __device__ __forceinline__ int by_R(int x) const { return mdiv(x, mR); }
+};
+// ... or of a schedule known at compile time (DifFix)
+template <class F, int I> struct DifFixPass {
+    static constexpr int R = F::radix(I), S = F::S(I), NR = F::N / R, mstep = F::M(I) - S, NB1 = F::N / F::radix(0) / R,
+                         two = F::two(I);
+    __device__ __forceinline__ int by_NR(int x) const { return x / NR; }
+    __device__ __forceinline__ int by_NB1(int x) const { return x / (NB1 > 0 ? NB1 : 1); }
+    __device__ __forceinline__ int by_S(int x) const { return x / S; }
+    __device__ __forceinline__ int by_R(int x) const { return x / R; }
 };
 
 template <typename T> struct DifArgs {
@@ -83,22 +97,82 @@ __device__ __forceinline__ void dif_out(const DifArgs<T> &a, long e, typename cp
     }
 }
 
+// Schedules: the passes from the arguments (any length) ...
+struct DifDyn {
+    static constexpr int V = 0;  // transforms per column tile: from the arguments
+    template <typename T> static __device__ __forceinline__ const DifPass &first(const DifArgs<T> &a) { return a.p[0]; }
+    template <typename T> static __device__ __forceinline__ const DifPass &last(const DifArgs<T> &a) {
+        return a.p[a.np - 1];
+    }
+    template <typename T> static __device__ __forceinline__ int P1(const DifArgs<T> &a) { return a.P1; }
+    // position of butterfly q = k1 + R1*(k2 + R2*(...)) of the last pass
+    template <typename T> static __device__ __forceinline__ int pos(const DifArgs<T> &a, int q) {
+        int rem = mdiv(q, a.p[0].mR);
+        int pos = (q - rem * a.p[0].R) * a.P1;
+        for (int i = 1; i + 1 < a.np; i++) {
+            const int n = mdiv(rem, a.p[i].mR);
+            pos += (rem - n * a.p[i].R) * a.p[i].S;
+            rem = n;
+        }
+        return pos;
+    }
+};
+// ... or radices Rs and block pitch P known at compile time: strides and
+// divisors are immediates and a kernel holds its own codelets only (2^24
+// points in rows: 50-52 us for lengths of three passes against 56-62).  VT:
+// transforms per column tile (1 for rows).
+template <int VT, int P, int... Rs> struct DifFix {
+    static constexpr int V = VT, np = sizeof...(Rs), N = (Rs * ...);
+    static constexpr int radix(int i) {
+        const int r[] = {Rs...};
+        return r[i];
+    }
+    static constexpr int M(int i) {
+        int m = N;
+        for (int j = 0; j < i; j++) m /= radix(j);
+        return m;
+    }
+    static constexpr int S(int i) { return M(i) / radix(i); }
+    static constexpr int two(int i) {
+        int t = 0;
+        for (int j = 0; j < i; j++) t += M(j);
+        return t;
+    }
+    template <typename T> static __device__ __forceinline__ DifFixPass<DifFix, 0> first(const DifArgs<T> &) { return {}; }
+    template <typename T> static __device__ __forceinline__ DifFixPass<DifFix, np - 1> last(const DifArgs<T> &) {
+        return {};
+    }
+    template <typename T> static __device__ __forceinline__ int P1(const DifArgs<T> &) { return P; }
+    template <int I> static __device__ __forceinline__ int digits(int rem) {
+        if constexpr (I + 1 < np) return rem % radix(I) * S(I) + digits<I + 1>(rem / radix(I));
+        else return 0;
+    }
+    template <typename T> static __device__ __forceinline__ int pos(const DifArgs<T> &, int q) {
+        return q % radix(0) * P + digits<1>(q / radix(0));
+    }
+};
+
+// x / V, V a power of two
+template <class SC, typename T> __device__ __forceinline__ int dif_by_v(const DifArgs<T> &a, int x) {
+    return SC::V ? x / (SC::V ? SC::V : 1) : x >> a.lgv;
+}
+
 // First pass.  Rows: consecutive threads on consecutive n' of one transform;
 // column tiles: on adjacent transforms (element i of transform t at i*vpb + t).
-template <int KIND, bool COLS, int R, typename T>
+template <class SC, int KIND, bool COLS, int R, typename T>
 __device__ __forceinline__ void dif_first(const DifArgs<T> &a, typename cplx_t<T>::t *s, int nt, long v0) {
     typedef typename cplx_t<T>::t C;
-    const DifPass &p = a.p[0];
-    const int S = p.S, V = COLS ? a.vpb : 1;
+    const auto &p = SC::first(a);
+    const int S = p.S, V = !COLS ? 1 : SC::V ? SC::V : a.vpb;
     const int nb = COLS ? S : nt * S;
-    const int step = COLS ? (int)blockDim.x >> a.lgv : (int)blockDim.x;
+    const int step = COLS ? dif_by_v<SC>(a, (int)blockDim.x) : (int)blockDim.x;
     const int ct = COLS ? ((int)threadIdx.x & (V - 1)) : 0;
-    const int sp = a.P1 * V;
+    const int sp = SC::P1(a) * V;
     if (COLS && ct >= nt) return;
-    for (int b = COLS ? (int)threadIdx.x >> a.lgv : (int)threadIdx.x; b < nb; b += step) {
+    for (int b = COLS ? dif_by_v<SC>(a, (int)threadIdx.x) : (int)threadIdx.x; b < nb; b += step) {
         int t = ct, j = b;
         if (!COLS && a.vpb > 1) {
-            t = mdiv(b, p.mNR);
+            t = p.by_NR(b);
             j = b - t * S;
         }
         long e0 = (v0 + t) * a.vs_in + (COLS ? (long)j * a.es_in : (long)j);
@@ -125,24 +199,24 @@ __device__ __forceinline__ void dif_first(const DifArgs<T> &a, typename cplx_t<T
 }
 
 // Middle pass.
-template <bool COLS, int R, typename T>
-__device__ __forceinline__ void dif_mid(const DifArgs<T> &a, const DifPass &p, typename cplx_t<T>::t *s, int nt) {
+template <class SC, bool COLS, int R, typename T, class PD>
+__device__ __forceinline__ void dif_mid(const DifArgs<T> &a, const PD &p, typename cplx_t<T>::t *s, int nt) {
     typedef typename cplx_t<T>::t C;
-    const int S = p.S, V = COLS ? a.vpb : 1;
+    const int S = p.S, V = !COLS ? 1 : SC::V ? SC::V : a.vpb;
     const int nb = COLS ? p.NR : nt * p.NR;
-    const int step = COLS ? (int)blockDim.x >> a.lgv : (int)blockDim.x;
+    const int step = COLS ? dif_by_v<SC>(a, (int)blockDim.x) : (int)blockDim.x;
     const int ct = COLS ? ((int)threadIdx.x & (V - 1)) : 0;
     const int sp = S * V;
     if (COLS && ct >= nt) return;
-    for (int b = COLS ? (int)threadIdx.x >> a.lgv : (int)threadIdx.x; b < nb; b += step) {
+    for (int b = COLS ? dif_by_v<SC>(a, (int)threadIdx.x) : (int)threadIdx.x; b < nb; b += step) {
         int t = ct, j = b;
         if (!COLS && a.vpb > 1) {
-            t = mdiv(b, p.mNR);
+            t = p.by_NR(b);
             j = b - t * p.NR;
         }
-        const int k1 = mdiv(j, p.mNB1), u = j - k1 * p.NB1;
-        const int c = mdiv(u, p.mS), n = u - c * S;
-        const int pos = k1 * a.P1 + u + c * p.mstep;
+        const int k1 = p.by_NB1(j), u = j - k1 * p.NB1;
+        const int c = p.by_S(u), n = u - c * S;
+        const int pos = k1 * SC::P1(a) + u + c * p.mstep;
         C *d = COLS ? s + (pos * V + t) : s + (t * a.LD + pos);
         C v[R];
 #pragma unroll
@@ -156,38 +230,26 @@ __device__ __forceinline__ void dif_mid(const DifArgs<T> &a, const DifPass &p, t
     }
 }
 
-// position of butterfly q = k1 + R1*(k2 + R2*(...)) of the last pass
-template <typename T> __device__ __forceinline__ int dif_pos(const DifArgs<T> &a, int q) {
-    int rem = mdiv(q, a.p[0].mR);
-    int pos = (q - rem * a.p[0].R) * a.P1;
-    for (int i = 1; i + 1 < a.np; i++) {
-        const int n = mdiv(rem, a.p[i].mR);
-        pos += (rem - n * a.p[i].R) * a.p[i].S;
-        rem = n;
-    }
-    return pos;
-}
-
 // Last pass: to the view.
-template <int KIND, bool COLS, int R, typename T>
+template <class SC, int KIND, bool COLS, int R, typename T>
 __device__ __forceinline__ void dif_last(const DifArgs<T> &a, const typename cplx_t<T>::t *s, int nt, long v0) {
     typedef typename cplx_t<T>::t C;
-    const DifPass &p = a.p[a.np - 1];
+    const auto &p = SC::last(a);
     // stores with consecutive threads on adjacent transforms: column tiles,
     // and the rows of a long vector's last pass
     constexpr bool TF = COLS || KIND == DIF_VECR;
-    const int Q = p.NR, V = TF ? a.vpb : 1;
+    const int Q = p.NR, V = !TF ? 1 : SC::V ? SC::V : a.vpb;
     const int nb = TF ? Q : nt * Q;
-    const int step = TF ? (int)blockDim.x >> a.lgv : (int)blockDim.x;
+    const int step = TF ? dif_by_v<SC>(a, (int)blockDim.x) : (int)blockDim.x;
     const int ct = TF ? ((int)threadIdx.x & (V - 1)) : 0;
     if (TF && ct >= nt) return;
-    for (int b = TF ? (int)threadIdx.x >> a.lgv : (int)threadIdx.x; b < nb; b += step) {
+    for (int b = TF ? dif_by_v<SC>(a, (int)threadIdx.x) : (int)threadIdx.x; b < nb; b += step) {
         int t = ct, q = b;
         if (!TF && a.vpb > 1) {
-            t = mdiv(b, p.mNR);
+            t = p.by_NR(b);
             q = b - t * Q;
         }
-        const int pos = dif_pos(a, q);
+        const int pos = SC::pos(a, q);
         const C *d = COLS ? s + (pos * V + t) : s + (t * a.LD + pos);
         C v[R];
 #pragma unroll
@@ -226,11 +288,11 @@ __device__ __forceinline__ void dif_last(const DifArgs<T> &a, const typename cpl
 // the forward passes.  A thread takes the butterflies of n' and S - n' (one of
 // them for n' = 0 and S/2), which hold each other's partners X_{N-n}, so every
 // spectrum element is loaded once; w_{N-n} = -conj w_n.
-template <int R, typename T>
+template <class SC, int R, typename T>
 __device__ __forceinline__ void dif_first_c2r(const DifArgs<T> &a, typename cplx_t<T>::t *s, int nt, long v0) {
     typedef typename cplx_t<T>::t C;
-    const DifPass &p = a.p[0];
-    const int S = p.S, H = S / 2 + 1;
+    const auto &p = SC::first(a);
+    const int S = p.S, H = S / 2 + 1, P1 = SC::P1(a);
     for (int b = threadIdx.x; b < nt * H; b += blockDim.x) {
         const int t = mdiv(b, a.mH), j = b - t * H;
         const C *x = a.in + (v0 + t) * a.vs_in;
@@ -253,7 +315,7 @@ __device__ __forceinline__ void dif_first_c2r(const DifArgs<T> &a, typename cplx
 #pragma unroll
         for (int r = 1; r < R; r++) u[r] = cmul(u[r], __ldg(tu + r * S));
 #pragma unroll
-        for (int r = 0; r < R; r++) d[r * a.P1] = u[r];
+        for (int r = 0; r < R; r++) d[r * P1] = u[r];
         if (j != 0 && 2 * j != S) {
             d += S - 2 * j;
             Dft<C, R>::run(w);
@@ -261,7 +323,7 @@ __device__ __forceinline__ void dif_first_c2r(const DifArgs<T> &a, typename cplx
 #pragma unroll
             for (int r = 1; r < R; r++) w[r] = cmul(w[r], __ldg(tw + r * S));
 #pragma unroll
-            for (int r = 0; r < R; r++) d[r * a.P1] = w[r];
+            for (int r = 0; r < R; r++) d[r * P1] = w[r];
         }
     }
 }
@@ -271,14 +333,14 @@ __device__ __forceinline__ void dif_first_c2r(const DifArgs<T> &a, typename cplx
 // (Z_k - conj Z_{N-k}))/2, w_k = exp(-i pi k/N), Z_N = Z_0, the scale applied
 // to Z first (c_VSIP_src/VI_rcfftmop_f_def.h:79-118): the spectrum leaves from
 // registers, without another trip through shared memory.
-template <int R, typename T>
+template <class SC, int R, typename T>
 __device__ __forceinline__ void dif_last_r2c(const DifArgs<T> &a, const typename cplx_t<T>::t *s, int nt, long v0) {
     typedef typename cplx_t<T>::t C;
-    const DifPass &p = a.p[a.np - 1];
+    const auto &p = SC::last(a);
     const int Q = p.NR, H = Q / 2 + 1;
     for (int b = threadIdx.x; b < nt * H; b += blockDim.x) {
         const int t = mdiv(b, a.mH), q = b - t * H;
-        const C *su = s + (t * a.LD + dif_pos(a, q)), *sw = s + (t * a.LD + dif_pos(a, q ? Q - q : 0));
+        const C *su = s + (t * a.LD + SC::pos(a, q)), *sw = s + (t * a.LD + SC::pos(a, q ? Q - q : 0));
         C u[R], w[R];
 #pragma unroll
         for (int r = 0; r < R; r++) u[r] = su[r];
@@ -346,6 +408,63 @@ constexpr int kDifPairMax = 10;
         default: CALL(2); break;      \
     }
 
+// The passes of one CTA's transforms.
+template <typename T, int KIND, bool COLS>
+__device__ __forceinline__ void dif_passes(const DifArgs<T> &a, typename cplx_t<T>::t *s, int nt, long v0) {
+    typedef DifDyn SC;
+    if constexpr (KIND == DIF_C2R) {
+#define JV_DIF_FIRST(R) (dif_first_c2r<SC, R, T>(a, s, nt, v0))
+        JV_DIF_PAIR_SWITCH(a.p[0].R, JV_DIF_FIRST)
+#undef JV_DIF_FIRST
+    } else {
+#define JV_DIF_FIRST(R) (dif_first<SC, KIND, COLS, R, T>(a, s, nt, v0))
+        JV_DIF_SWITCH(a.p[0].R, JV_DIF_FIRST)
+#undef JV_DIF_FIRST
+    }
+    __syncthreads();
+    for (int i = 1; i + 1 < a.np; i++) {
+#define JV_DIF_MID(R) (dif_mid<SC, COLS, R, T>(a, a.p[i], s, nt))
+        JV_DIF_SWITCH(a.p[i].R, JV_DIF_MID)
+#undef JV_DIF_MID
+        __syncthreads();
+    }
+    if constexpr (KIND == DIF_R2C) {
+#define JV_DIF_LAST(R) (dif_last_r2c<SC, R, T>(a, s, nt, v0))
+        JV_DIF_PAIR_SWITCH(a.p[a.np - 1].R, JV_DIF_LAST)
+#undef JV_DIF_LAST
+    } else {
+#define JV_DIF_LAST(R) (dif_last<SC, KIND, COLS, R, T>(a, s, nt, v0))
+        JV_DIF_SWITCH(a.p[a.np - 1].R, JV_DIF_LAST)
+#undef JV_DIF_LAST
+    }
+}
+template <class F, int I, typename T, bool COLS>
+__device__ __forceinline__ void dif_mids(const DifArgs<T> &a, typename cplx_t<T>::t *s, int nt) {
+    if constexpr (I + 1 < F::np) {
+        dif_mid<F, COLS, F::radix(I), T>(a, DifFixPass<F, I>(), s, nt);
+        __syncthreads();
+        dif_mids<F, I + 1, T, COLS>(a, s, nt);
+    }
+}
+template <class F, typename T, int KIND, bool COLS>
+__device__ __forceinline__ void dif_passes_fix(const DifArgs<T> &a, typename cplx_t<T>::t *s, int nt, long v0) {
+    if constexpr (KIND == DIF_C2R) dif_first_c2r<F, F::radix(0), T>(a, s, nt, v0);
+    else dif_first<F, KIND, COLS, F::radix(0), T>(a, s, nt, v0);
+    __syncthreads();
+    dif_mids<F, 1, T, COLS>(a, s, nt);
+    if constexpr (KIND == DIF_R2C) dif_last_r2c<F, F::radix(F::np - 1), T>(a, s, nt, v0);
+    else dif_last<F, KIND, COLS, F::radix(F::np - 1), T>(a, s, nt, v0);
+}
+
+template <typename T, int KIND>
+__device__ __forceinline__ void dif_prologue(const DifArgs<T> &a, typename cplx_t<T>::t *s, long v0) {
+    if constexpr (KIND == DIF_VEC1) {
+        // W_N^(k v0), k < the pass's length (k v0 < N), behind the tile
+        for (int k = threadIdx.x; k < a.N; k += blockDim.x)
+            s[a.LD * a.vpb + k] = tw_two_level(a.tw_lo, a.tw_hi, a.tw_mask, a.tw_sh, (unsigned)k * (unsigned)v0);
+    }
+}
+
 template <typename T, int KIND, bool COLS>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_dif(const __grid_constant__ DifArgs<T> a) {
     typedef typename cplx_t<T>::t C;
@@ -353,36 +472,21 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_dif(const __gri
     C *s = reinterpret_cast<C *>(smem_raw);
     const long v0 = (long)blockIdx.x * a.vpb;
     const int nt = (int)min((long)a.vpb, a.nvec - v0);
-    if constexpr (KIND == DIF_VEC1) {
-        // W_N^(k v0), k < the pass's length (k v0 < N), behind the tile
-        for (int k = threadIdx.x; k < a.N; k += blockDim.x)
-            s[a.LD * a.vpb + k] = tw_two_level(a.tw_lo, a.tw_hi, a.tw_mask, a.tw_sh, (unsigned)k * (unsigned)v0);
-    }
-    if constexpr (KIND == DIF_C2R) {
-#define JV_DIF_FIRST(R) (dif_first_c2r<R, T>(a, s, nt, v0))
-        JV_DIF_PAIR_SWITCH(a.p[0].R, JV_DIF_FIRST)
-#undef JV_DIF_FIRST
-    } else {
-#define JV_DIF_FIRST(R) (dif_first<KIND, COLS, R, T>(a, s, nt, v0))
-        JV_DIF_SWITCH(a.p[0].R, JV_DIF_FIRST)
-#undef JV_DIF_FIRST
-    }
-    __syncthreads();
-    for (int i = 1; i + 1 < a.np; i++) {
-#define JV_DIF_MID(R) (dif_mid<COLS, R, T>(a, a.p[i], s, nt))
-        JV_DIF_SWITCH(a.p[i].R, JV_DIF_MID)
-#undef JV_DIF_MID
-        __syncthreads();
-    }
-    if constexpr (KIND == DIF_R2C) {
-#define JV_DIF_LAST(R) (dif_last_r2c<R, T>(a, s, nt, v0))
-        JV_DIF_PAIR_SWITCH(a.p[a.np - 1].R, JV_DIF_LAST)
-#undef JV_DIF_LAST
-    } else {
-#define JV_DIF_LAST(R) (dif_last<KIND, COLS, R, T>(a, s, nt, v0))
-        JV_DIF_SWITCH(a.p[a.np - 1].R, JV_DIF_LAST)
-#undef JV_DIF_LAST
-    }
+    dif_prologue<T, KIND>(a, s, v0);
+    dif_passes<T, KIND, COLS>(a, s, nt, v0);
+}
+
+// The same with a schedule known at compile time, in CTAs of NT threads of
+// which MB share an SM.
+template <class F, typename T, int KIND, bool COLS, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_dif_fix(const __grid_constant__ DifArgs<T> a) {
+    typedef typename cplx_t<T>::t C;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    C *s = reinterpret_cast<C *>(smem_raw);
+    const long v0 = (long)blockIdx.x * a.vpb;
+    const int nt = (int)min((long)a.vpb, a.nvec - v0);
+    dif_prologue<T, KIND>(a, s, v0);
+    dif_passes_fix<F, T, KIND, COLS>(a, s, nt, v0);
 }
 
 // One tile of a batch of calls: nt transforms from v0 of call `call`.
@@ -405,24 +509,25 @@ __global__ void __launch_bounds__(1024) k_dif_batch(const DifArgs<float> *__rest
         reinterpret_cast<unsigned long long *>(&a)[i] =
             __ldg(reinterpret_cast<const unsigned long long *>(&calls[d.call]) + i);
     __syncthreads();
-#define JV_DIF_FIRST(R) (dif_first<DIF_C2C, COLS, R, float>(a, s, d.nt, d.v0))
-    JV_DIF_SWITCH(a.p[0].R, JV_DIF_FIRST)
-#undef JV_DIF_FIRST
-    __syncthreads();
-    for (int i = 1; i + 1 < a.np; i++) {
-#define JV_DIF_MID(R) (dif_mid<COLS, R, float>(a, a.p[i], s, d.nt))
-        JV_DIF_SWITCH(a.p[i].R, JV_DIF_MID)
-#undef JV_DIF_MID
-        __syncthreads();
-    }
-#define JV_DIF_LAST(R) (dif_last<DIF_C2C, COLS, R, float>(a, s, d.nt, d.v0))
-    JV_DIF_SWITCH(a.p[a.np - 1].R, JV_DIF_LAST)
-#undef JV_DIF_LAST
+    dif_passes<float, DIF_C2C, COLS>(a, s, d.nt, d.v0);
 }
 
 // static shared memory of k_dif_batch (the copied arguments), rounded up
 constexpr size_t kStaticArgs = 1024;
 static_assert(sizeof(DifArgs<float>) <= kStaticArgs, "arguments fit");
+
+// A length whose schedule is compiled in (jv_dif_table.h) and its launchers
+// (null: the kernel that reads the schedule from its arguments).
+typedef bool (*DifFixGo)(const DifArgs<float> &a, size_t smem, cudaStream_t st, unsigned groups);
+struct DifFixEntry {
+    int N = 0, P1 = 0;
+    int vpb = 1, nthr = 0;   // rows: transforms per CTA, threads
+    int vcol = 0;            // transforms per column tile
+    std::vector<int> radix;
+    DifFixGo rows = nullptr, cols = nullptr, cols4 = nullptr;  // cols4: tiles of 4, for few columns
+    DifFixGo step = nullptr, vec[3] = {nullptr, nullptr, nullptr};
+};
+const DifFixEntry *dif_fix(long N, int cls);  // cls 0: c2c, 1: R2C, 2: C2R; null: not in the table
 
 // CTA shape of a call
 struct DifCta {

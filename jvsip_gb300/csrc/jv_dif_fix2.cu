@@ -1,0 +1,11 @@
+// jv_dif_fix2.cu -- compiled-in schedules of the in-place mixed-radix kernel:
+// c2c rows and column tiles of 601 to 3000 points.
+#include "jv_dif_fix.cuh"
+
+namespace jv {
+void dif_fix_c2c_2(std::vector<DifFixEntry> &out) {
+#define X(...) out.push_back(dif_fix_c2c<__VA_ARGS__>());
+    JV_DIF_LENGTHS_2(X)
+#undef X
+}
+}  // namespace jv

@@ -571,17 +571,29 @@ static bool run_long(Job &j, cudaStream_t st, bool *handled) {
     return j.prec == P_F32 ? launch_c2r_unpack_f32(j, ys, st) : launch_c2r_unpack_f64(j, ys, st);
 }
 
-// One launch over whole transforms: the register-resident kernel at its
-// lengths, the in-place mixed-radix kernel at the others (lengths with factors
-// 11 and 13 among them) and where it is the faster one -- rows of 64 and 1000
-// points that fill the GPU (2^24 points: 43.1 us against 49.2, and 60 against
-// 70; 40 rows of 1000: 6.9 against 6.2).  False when neither takes the call.
+// Calls that the register-resident kernel runs faster than the in-place one
+// (us on 2^24 points in rows, 2^23 otherwise): rows of 512 / 768 / 4096 points
+// 45.2 / 49.2 / 48.9 against 47.0 / 51.2 / 49.4, when they fill the GPU (64 rows
+// of 512: 6.2 against 4.0); R2C of 512 points 28.7 against 30.8, C2R of 512 32.8
+// and 33.0 (4096 rows: 6.2 and 8.2), R2C and C2R of 8192 points 34.8 against
+// 38; columns of 4096 points 53 against 61.  At its
+// other lengths the in-place kernel is the faster one or as fast (rows of 128 /
+// 1000 / 1024 points 41.8 / 51.3 / 43.7 against 43.6 / 70.4 / 47.1; R2C of 1536
+// 32.9 against 34.1, C2R 32.9 against 35.1; columns of 1000 35.0 against 41.0).
+static bool fast_first(const Job &j) {
+    if (j.kind != K_C2C) return j.N == 256 || j.N == 4096;
+    if (j.cin.cst != 2) return true;  // split complex
+    if (j.cin.es == 1 && j.cout.es == 1)
+        return (j.N == 512 || j.N == 768 || j.N == 4096) && j.nvec * j.N >= 4096L * device()->sms;
+    return j.N == 4096;
+}
+
+// One launch over whole transforms, on the register-resident or the in-place
+// mixed-radix kernel; false when neither takes the call.
 static bool run_tiles(const Job &j, cudaStream_t st) {
     if (j.prec != P_F32) return false;
-    const bool dif_first = (j.N == 64 || j.N == 1000) && j.kind == K_C2C && j.cin.cst == 2 && j.cin.es == 1 &&
-                           j.cout.es == 1 && j.nvec * j.N >= 4096L * device()->sms;
-    if (dif_first && launch_dif_f32(j, st)) return true;
-    return launch_fast_f32(j, st) || launch_dif_f32(j, st);
+    if (fast_first(j)) return launch_fast_f32(j, st) || launch_dif_f32(j, st);
+    return launch_dif_f32(j, st) || launch_fast_f32(j, st);
 }
 
 static bool run_job(Job &j, cudaStream_t st) {

@@ -11,21 +11,27 @@ namespace jv {
 template <int RM, int FXK = 0>
 static bool launch_fast_real_t(const Job &j, cudaStream_t st) {
     switch (j.N) {
-        case 64: return launch_fast_n<64, 4, 64, RList<16, 4>, false, false, false, false, RM, FXK>(j, st);
-        case 128: return launch_fast_n<128, 8, 32, RList<16, 8>, false, false, false, false, RM, FXK>(j, st);
         case 256: return launch_fast_n<256, 16, 16, RList<16, 16>, false, false, false, false, RM, FXK>(j, st);
-        case 512: return launch_fast_n<512, 32, 8, RList<16, 16, 2>, false, false, false, false, RM, FXK>(j, st);
-        // 768 points: 4 rows per CTA, 7 CTAs per SM (measured on 4096 x 1536
-        // R2C / C2R: 21.1 / 21.6 us against 23.8 / 23.3 us for 8 rows per CTA
-        // at 3 CTAs per SM)
-        case 768: return launch_fast_n<768, 32, 4, RList<12, 8, 8>, false, false, false, false, RM, FXK>(j, st);
-        case 1000: return launch_fast_n<1000, 100, 4, RList<10, 10, 10>, false, false, false, false, RM, FXK>(j, st);
-        case 1024: return launch_fast_n<1024, 64, 4, RList<16, 16, 4>, false, false, false, false, RM, FXK>(j, st);
-        case 2048: return launch_fast_n<2048, 128, 2, RList<16, 16, 8>, false, false, false, false, RM, FXK>(j, st);
         case 4096: return launch_fast_n<4096, 256, 1, RList<16, 16, 16>, false, false, false, false, RM, FXK>(j, st);
-        case 8192: return launch_fast_n<8192, 512, 1, RList<16, 16, 16, 2>, false, false, false, false, RM, FXK>(j, st);
-        default: return false;
+        default: break;
     }
+    if constexpr (FXK != 0) {
+        switch (j.N) {
+            case 64: return launch_fast_n<64, 4, 64, RList<16, 4>, false, false, false, false, RM, FXK>(j, st);
+            case 128: return launch_fast_n<128, 8, 32, RList<16, 8>, false, false, false, false, RM, FXK>(j, st);
+            case 512: return launch_fast_n<512, 32, 8, RList<16, 16, 2>, false, false, false, false, RM, FXK>(j, st);
+            // 768 points: 4 rows per CTA, 7 CTAs per SM (measured on 4096 x 1536
+            // R2C / C2R: 21.1 / 21.6 us against 23.8 / 23.3 us for 8 rows per CTA
+            // at 3 CTAs per SM)
+            case 768: return launch_fast_n<768, 32, 4, RList<12, 8, 8>, false, false, false, false, RM, FXK>(j, st);
+            case 1000: return launch_fast_n<1000, 100, 4, RList<10, 10, 10>, false, false, false, false, RM, FXK>(j, st);
+            case 1024: return launch_fast_n<1024, 64, 4, RList<16, 16, 4>, false, false, false, false, RM, FXK>(j, st);
+            case 2048: return launch_fast_n<2048, 128, 2, RList<16, 16, 8>, false, false, false, false, RM, FXK>(j, st);
+            case 8192: return launch_fast_n<8192, 512, 1, RList<16, 16, 16, 2>, false, false, false, false, RM, FXK>(j, st);
+            default: break;
+        }
+    }
+    return false;
 }
 
 // Real rows of unit stride in a real block (not a real view of a complex

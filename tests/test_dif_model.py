@@ -2,6 +2,9 @@
 restated in numpy: positions, twiddles and output order of every pass, the
 block pitch, and the pair passes of the real transforms, against numpy's FFT
 for schedules of two to five passes in several orders (no GPU needed)."""
+import os
+import re
+
 import numpy as np
 import pytest
 
@@ -95,3 +98,53 @@ def test_c2r_pair_pass_partners(rad):
         assert max(w) <= N and all(u[r] + w[R - 1 - r] == N for r in range(R))
         done += u + (w if j and 2 * j != S else [])
     assert sorted(done) == list(range(N))
+
+
+# ---------------------------------------------------------------- compiled-in schedules
+def table():
+    src = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "jvsip_gb300", "csrc",
+                            "jv_dif_table.h")).read()
+    out = {}
+    for name, body in re.findall(r"#define (JV_DIF_\w+)\(X\) \\\n((?:    X\([\d, ]+\)(?: \\)?\n?)+)", src):
+        kind = "c2c" if "LENGTHS" in name else name.split("_")[2].lower()
+        out.setdefault(kind, []).extend([int(v) for v in row.split(",")] for row in re.findall(r"X\(([\d, ]+)\)", body))
+    return out
+
+
+def test_table_covers_its_lengths_once():
+    smooth = [n for n in range(40, 16385) if _smooth(n)]
+    t = table()
+    assert [r[0] for r in t["c2c"]] == smooth
+    for kind in ("r2c", "c2r"):
+        assert [r[0] for r in t[kind]] == [n for n in smooth if n <= 8192]
+
+
+def _smooth(n):
+    for p in (2, 3, 5):
+        while n % p == 0:
+            n //= p
+    return n == 1
+
+
+@pytest.mark.parametrize("kind", ["c2c", "r2c", "c2r"])
+def test_table_entries_fit_the_kernel(kind):
+    """Radices give the length and are codelets (pair passes at most 10), blocks
+    do not overlap, every CTA's threads and shared memory exist, and index
+    products stay below the multiply-high limit."""
+    for row in table()[kind]:
+        N, P1, T, VPB = row[:4]
+        VC, TC, TV, TL, rad = (*row[4:8], row[8:]) if kind == "c2c" else (0, 0, 0, 0, row[4:])
+        assert int(np.prod(rad)) == N and len(rad) >= 2 and all(2 <= r <= 16 for r in rad), row
+        assert N // rad[0] <= P1 < N // rad[0] + 16, row
+        if kind == "r2c":
+            assert rad[-1] <= 10, row
+        if kind == "c2r":
+            assert rad[0] <= 10, row
+        tiles = [(VPB, T)] + [(v, t) for v, t in ((VC, TC), (16, TV), (4, TL)) if v and t]
+        for v, t in tiles:
+            assert t % 32 == 0 and 64 <= t <= 1024, row
+            # the long vectors' first pass keeps N more elements behind its tile of 16
+            assert (v * (rad[0] * P1 + 1) + (N if v == 16 and t == TV else 0)) * 8 <= 227 * 1024, row
+            assert v * N // min(rad) * (N // min(rad)) < 2 ** 32, row
+        for v, t in tiles[1:]:
+            assert v & (v - 1) == 0 and t % v == 0, row
