@@ -53,7 +53,7 @@ static long bank_waves(const std::vector<int> &r, long N, long P1, int W) {
     for (int p = 1; p < np; p++) {
         const bool last = p == np - 1;
         const long S = last ? 1 : M / r[p], NR = N / r[p], NB1 = N / r[0] / r[p];
-        const long ngr = (NR + W - 1) / W, take = std::min<long>(ngr, 12);
+        const long ngr = (NR + W - 1) / W, take = std::min<long>(ngr, 6);
         for (long g = 0; g < take; g++) {
             const long b0 = g * ngr / take * W;
             int hit[16] = {0};
@@ -121,7 +121,7 @@ bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1) {
                 *P1 = S1 + pad;
             }
         }
-    } while (++tried < 60 && std::next_permutation(q.begin(), q.end()));
+    } while (++tried < 24 && std::next_permutation(q.begin(), q.end()));
     return true;
 }
 
@@ -130,6 +130,9 @@ void dif_fix_c2c_1(std::vector<DifFixEntry> &out);
 void dif_fix_c2c_2(std::vector<DifFixEntry> &out);
 void dif_fix_c2c_3(std::vector<DifFixEntry> &out);
 void dif_fix_long_1(std::vector<DifFixEntry> &out);
+void dif_fix_taper_1(std::vector<DifFixEntry> &out);
+void dif_fix_taper_2(std::vector<DifFixEntry> &out);
+void dif_fix_power_1(std::vector<DifFixEntry> &out);
 void dif_fix_r2c_1(std::vector<DifFixEntry> &out);
 void dif_fix_r2c_2(std::vector<DifFixEntry> &out);
 void dif_fix_c2r_1(std::vector<DifFixEntry> &out);
@@ -139,7 +142,7 @@ const DifFixEntry *dif_fix(long N, int cls) {
     // built once, thread-safely, on the first call
     static const std::vector<std::map<long, DifFixEntry>> tab = []() {
         std::vector<std::map<long, DifFixEntry>> t(3);
-        std::vector<DifFixEntry> v[4];
+        std::vector<DifFixEntry> v[6];
         dif_fix_c2c_1(v[0]);
         dif_fix_c2c_2(v[0]);
         dif_fix_c2c_3(v[0]);
@@ -148,6 +151,9 @@ const DifFixEntry *dif_fix(long N, int cls) {
         dif_fix_c2r_1(v[2]);
         dif_fix_c2r_2(v[2]);
         dif_fix_long_1(v[3]);
+        dif_fix_taper_1(v[4]);
+        dif_fix_taper_2(v[4]);
+        dif_fix_power_1(v[5]);
         for (int c = 0; c < 3; c++)
             for (const DifFixEntry &e : v[c]) t[c][e.N] = e;
         for (const DifFixEntry &e : v[3]) {
@@ -155,6 +161,11 @@ const DifFixEntry *dif_fix(long N, int cls) {
             d.step = e.step;
             for (int i = 0; i < 3; i++) d.vec[i] = e.vec[i];
         }
+        for (const DifFixEntry &e : v[4]) {
+            t[1][e.N].taper = e.taper;
+            t[1][e.N].vtaper = e.vtaper;
+        }
+        for (const DifFixEntry &e : v[5]) t[0][e.N].power = e.power;
         return t;
     }();
     auto it = tab[cls].find(N);
@@ -164,6 +175,9 @@ const DifFixEntry *dif_fix(long N, int cls) {
 // ---------------------------------------------------------------- tables
 static std::mutex g_dif_mu;
 static std::map<std::tuple<long, int, int>, DifTab> g_dif;
+// schedules and CTA shapes found so far (host only; one small entry per length
+// a program has planned, at most 16384 x 3): the search takes 0.1 to 0.3 ms
+static std::map<std::tuple<long, int, int>, DifTab> g_found;
 
 static void root(long m, long N, double *c, double *s) {  // exp(-2 pi i m/N)
     bool flip = false;
@@ -176,18 +190,18 @@ static void root(long m, long N, double *c, double *s) {  // exp(-2 pi i m/N)
     *s = flip ? sin(a) : -sin(a);
 }
 
-template <typename T> static void *upload_tables(const std::vector<int> &rad, long N, std::vector<int> &two) {
+template <typename T>
+static void *upload_tables(const std::vector<int> &rad, long N, const std::vector<double> &roots,
+                           std::vector<int> &two) {
     std::vector<T> tw;
     long M = N;
     for (size_t p = 0; p + 1 < rad.size(); p++) {
-        const long R = rad[p], S = M / R;
+        const long R = rad[p], S = M / R, step = N / M;
         two.push_back((int)(tw.size() / 2));
         for (long k = 0; k < R; k++)
             for (long n = 0; n < S; n++) {
-                double c, s;
-                root(k * n % M, M, &c, &s);
-                tw.push_back((T)c);
-                tw.push_back((T)s);
+                tw.push_back((T)roots[2 * (k * n * step)]);  // k*n < M
+                tw.push_back((T)roots[2 * (k * n * step) + 1]);
             }
         M = S;
     }
@@ -241,7 +255,7 @@ static void row_shape(DifTab &t, int cls) {
     }
 }
 
-const DifTab *dif_acquire(long N, int prec, int cls) {
+const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots) {
     if (prec != P_F32 || N > 16384) return nullptr;
     std::lock_guard<std::mutex> lk(g_dif_mu);
     auto key = std::make_tuple(N, prec, cls);
@@ -256,14 +270,27 @@ const DifTab *dif_acquire(long N, int prec, int cls) {
         t.radix = fix->radix;
         t.P1 = fix->P1;
         t.fix = fix;
-    } else if (!dif_schedule(N, prec, cls, t.radix, &t.P1)) {
-        return nullptr;
     }
     t.N = N;
     t.prec = prec;
     t.cls = cls;
+    if (!fix) {
+        auto seen = g_found.find(key);
+        if (seen == g_found.end()) {
+            if (dif_schedule(N, prec, cls, t.radix, &t.P1)) row_shape(t, cls);
+            seen = g_found.emplace(key, t).first;
+        }
+        if (seen->second.radix.empty()) return nullptr;  // no schedule
+        t = seen->second;
+    }
     const int err0 = jvsip_gpu_last_error();
-    t.d_tw = prec == P_F32 ? upload_tables<float>(t.radix, N, t.two) : upload_tables<double>(t.radix, N, t.two);
+    std::vector<double> own;
+    if (!roots) {
+        own = unit_roots(N);
+        roots = &own;
+    }
+    t.d_tw = prec == P_F32 ? upload_tables<float>(t.radix, N, *roots, t.two)
+                           : upload_tables<double>(t.radix, N, *roots, t.two);
     if (!t.d_tw) {  // the general kernels take the plan's calls
         if (!err0 && jvsip_gpu_last_error()) jvsip_gpu_clear_error();
         return nullptr;
@@ -271,8 +298,6 @@ const DifTab *dif_acquire(long N, int prec, int cls) {
     if (fix) {
         t.vpb = fix->vpb;
         t.nthr = fix->nthr;
-    } else {
-        row_shape(t, cls);
     }
     t.refs = 1;
     auto &slot = g_dif[key];
@@ -484,6 +509,69 @@ bool launch_dif_step_f32(const Job &j, cudaStream_t st) {
     return dif_step_go(a, c.nthr, c.smem, st, (unsigned)j.nbatch);
 }
 
+// ---------------------------------------------------------------- k-omega
+// The tapered R2C rows into a column-major spectrum (kw.c creates it so):
+// tiles of 4 to 16 rows in about 64 KB.  Row-major spectra are not taken.
+bool launch_dif_komega_r2c_f32(const Job &j, cudaStream_t st) {
+    const DifTab *t = j.dif;
+    if (!t || j.no_fast || j.no_dif || j.kind != K_R2C || j.nvec <= 1 || !j.thalf || !j.taper_n || !j.taper_t ||
+        !j.taper_back)
+        return false;
+    const CView &co = j.cout;
+    if (!real_pairs<float>(j.rin, 2 * j.N, j.nvec) || !interleaved_c<float>(co) || co.vs != 1 || co.es < j.nvec)
+        return false;
+    DifArgs<float> a;
+    memset(&a, 0, sizeof a);
+    a.in = (const float2 *)j.rin.a + j.rin.off / 2;
+    a.wb = const_cast<float2 *>(a.in);
+    a.vs_in = j.rin.vs / 2;
+    a.es_in = 1;
+    a.out = (float2 *)co.re + co.off;
+    a.es_out = co.es;
+    a.vs_out = 1;
+    a.thalf = (const float2 *)j.thalf;
+    a.nvec = j.nvec;
+    a.has_scale = j.has_scale;
+    a.scale = j.has_scale ? (float)j.scale : 1.f;
+    a.tp_n = (const float *)j.taper_n;
+    a.tp_t = (const float *)j.taper_t;
+    a.tp_n_st = j.taper_n_st;
+    a.tp_t_st = j.taper_t_st;
+    dif_fill(a, *t);
+    a.LD |= 1;
+    a.mH = magic_host((unsigned long)(a.p[a.np - 1].NR / 2 + 1));
+    const DifFixEntry *f = t->fix;
+    a.lgv = 4;
+    while (a.lgv > 2 && ((size_t)a.LD << a.lgv) * sizeof(float2) > 72 * 1024) a.lgv--;
+    if (f && f->taper)
+        for (a.lgv = 0; (1 << a.lgv) < f->vtaper; a.lgv++) {
+        }
+    // few sensors: fewer rows per tile, so that more SMs work on them
+    while (a.lgv > 0 && 2 * (((j.nvec - 1) >> a.lgv) + 1) < device()->sms) a.lgv--;
+    a.vpb = 1 << a.lgv;
+    const size_t smem = (size_t)a.LD * a.vpb * sizeof(float2);
+    if (smem > device()->smem_optin) return false;
+    if (f && f->taper && a.vpb == f->vtaper) return f->taper(a, smem, st, 1);
+    const long nthr = std::min(512L, std::max(96L, (a.vpb * j.N / 16 + 31) / 32 * 32));
+    return dif_komega_go(DIF_R2CT, a, (int)nthr, smem, st);
+}
+
+// Its transforms over the sensors, contiguous in that spectrum.
+bool launch_dif_komega_power_f32(const Job &j, cudaStream_t st) {
+    if (!j.gram) return false;
+    Job q = j;
+    q.gram = nullptr;
+    DifArgs<float> a;
+    DifCta c;
+    if (j.kind != K_C2C || !dif_args<float>(q, 0, a, c) || !c.rows || c.split) return false;
+    a.gram = (float *)j.gram;
+    a.g_es = j.gram_es;
+    a.g_vs = j.gram_vs;
+    a.g_scale = (float)j.gram_scale;
+    if (j.dif->fix && j.dif->fix->power) return j.dif->fix->power(a, c.smem, st, 1);
+    return dif_komega_go(DIF_POWER, a, c.nthr, c.smem, st);
+}
+
 // ---------------------------------------------------------------- single long vectors
 // N = A*B*C (or A*C, B = 1) points of one vector: with n = n1*BC + r and k =
 // k1 + A*(k2 + B*k3), pass 1 transforms over n1 (A points BC apart, 16
@@ -583,7 +671,7 @@ VecPlan *vec_acquire(long N) {
     bool ok = true;
     for (int i = 0; i < 3; i++) {
         v->f[i] = f[i];
-        if (f[i] > 1) ok = ok && (v->tab[i] = dif_acquire(f[i], P_F32, 0)) != nullptr;
+        if (f[i] > 1) ok = ok && (v->tab[i] = dif_acquire(f[i], P_F32, 0, nullptr)) != nullptr;
     }
     ok = ok && (v->d_t1 = upload_roots(f[0] * V, [&](long i) { return (i / V) * (i % V); }, N)) != nullptr;
     const long C = f[2];

@@ -69,17 +69,31 @@ template <typename T> struct DifArgs {
     unsigned tw_mask, tw_sh, tw_ts, tw_ys;
     const C *tv;             // DIF_VEC1, DIF_VEC2: output k of transform t times tv[k*tv_st + t]
     int tv_st;
+    // DIF_R2CT: real element n of row t times tp_n[n*tp_n_st], then times
+    // tp_t[t*tp_t_st], written back through wb; DIF_POWER: output k of transform
+    // t stores (p, Im X), p = g_scale |X|^2 added to gram[t*g_vs + k*g_es]
+    const T *tp_n, *tp_t;
+    long tp_n_st, tp_t_st;
+    C *wb;
+    T *gram;
+    long g_es, g_vs;
+    T g_scale;
     const C *thalf;          // real transforms: exp(-+ i pi k/N), k <= N
     unsigned mH;             // and the magic of the pair passes' work items per transform
     DifPass p[kDifMaxPass];
 };
 
 // DIF_VEC1, DIF_VEC2, DIF_VECR: the passes over a single long vector
-// (launch_vec_f32)
+// (launch_vec_f32).  DIF_R2CT, DIF_POWER: the k-omega pipeline's tapered R2C
+// rows into a column-major spectrum, and its transforms over the sensors with
+// the power accumulator (kw.c komega()).
 enum DifKind {
-    DIF_C2C = 0, DIF_SPLIT = 1, DIF_R2C = 2, DIF_C2R = 3, DIF_STEP = 4, DIF_VEC1 = 5, DIF_VEC2 = 6, DIF_VECR = 7
+    DIF_C2C = 0, DIF_SPLIT = 1, DIF_R2C = 2, DIF_C2R = 3, DIF_STEP = 4, DIF_VEC1 = 5, DIF_VEC2 = 6, DIF_VECR = 7,
+    DIF_R2CT = 8, DIF_POWER = 9
 };
-template <int KIND> constexpr bool dif_groups() { return KIND >= DIF_STEP; }
+template <int KIND> constexpr bool dif_groups() { return KIND >= DIF_STEP && KIND <= DIF_VECR; }
+// rows whose last pass stores with consecutive threads on adjacent transforms
+template <int KIND> constexpr bool dif_rows_tf() { return KIND == DIF_VECR || KIND == DIF_R2CT; }
 
 template <int KIND, typename T>
 __device__ __forceinline__ typename cplx_t<T>::t dif_in(const DifArgs<T> &a, long e) {
@@ -186,6 +200,17 @@ __device__ __forceinline__ void dif_first(const DifArgs<T> &a, typename cplx_t<T
 #pragma unroll
             for (int r = 0; r < R; r++) v[r] = dif_in<KIND>(a, e0 + r * S);
         }
+        if constexpr (KIND == DIF_R2CT) {
+            // kw.c: data = ts * data (VSIP_ROW), then data = arr * data (VSIP_COL)
+            const T wt = a.tp_t[(v0 + t) * a.tp_t_st];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const long n = 2L * (j + r * S);
+                v[r].x = mul_rn(mul_rn(a.tp_n[n * a.tp_n_st], v[r].x), wt);
+                v[r].y = mul_rn(mul_rn(a.tp_n[(n + 1) * a.tp_n_st], v[r].y), wt);
+                a.wb[e0 + r * S] = v[r];
+            }
+        }
 #pragma unroll
         for (int r = 0; r < R; r++) v[r].y = flip_sign(v[r].y, a.smask_in);
         Dft<C, R>::run(v);
@@ -237,7 +262,7 @@ __device__ __forceinline__ void dif_last(const DifArgs<T> &a, const typename cpl
     const auto &p = SC::last(a);
     // stores with consecutive threads on adjacent transforms: column tiles,
     // and the rows of a long vector's last pass
-    constexpr bool TF = COLS || KIND == DIF_VECR;
+    constexpr bool TF = COLS || dif_rows_tf<KIND>();
     const int Q = p.NR, V = !TF ? 1 : SC::V ? SC::V : a.vpb;
     const int nb = TF ? Q : nt * Q;
     const int step = TF ? dif_by_v<SC>(a, (int)blockDim.x) : (int)blockDim.x;
@@ -277,9 +302,26 @@ __device__ __forceinline__ void dif_last(const DifArgs<T> &a, const typename cpl
 #pragma unroll
             for (int r = 0; r < R; r++) v[r] = cmul(v[r], __ldg(w + r * Q * a.tv_st));
         }
+        if constexpr (KIND == DIF_POWER) {
+            T *g = a.gram + (v0 + t) * a.g_vs + (long)q * a.g_es;
+            T old[R];
 #pragma unroll
-        for (int r = 0; r < R; r++)
-            dif_out<KIND>(a, e0 + r * st, out_value(v[r], a.smask_out, a.has_scale != 0, a.scale));
+            for (int r = 0; r < R; r++) old[r] = g[(long)(r * Q) * a.g_es];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                // p = |X|^2 (vsip_mcmagsq_f), p *= s (vsip_smmul_f),
+                // gram = p + gram (vsip_madd_f), rounded in that order
+                const C x = out_value(v[r], a.smask_out, a.has_scale != 0, a.scale);
+                T p = add_rn(mul_rn(x.x, x.x), mul_rn(x.y, x.y));
+                p = mul_rn(a.g_scale, p);
+                g[(long)(r * Q) * a.g_es] = add_rn(p, old[r]);
+                dif_out<KIND>(a, e0 + r * st, mk<C>(p, x.y));
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                dif_out<KIND>(a, e0 + r * st, out_value(v[r], a.smask_out, a.has_scale != 0, a.scale));
+        }
     }
 }
 
@@ -333,13 +375,20 @@ __device__ __forceinline__ void dif_first_c2r(const DifArgs<T> &a, typename cplx
 // (Z_k - conj Z_{N-k}))/2, w_k = exp(-i pi k/N), Z_N = Z_0, the scale applied
 // to Z first (c_VSIP_src/VI_rcfftmop_f_def.h:79-118): the spectrum leaves from
 // registers, without another trip through shared memory.
-template <class SC, int R, typename T>
+template <class SC, int KIND, int R, typename T>
 __device__ __forceinline__ void dif_last_r2c(const DifArgs<T> &a, const typename cplx_t<T>::t *s, int nt, long v0) {
     typedef typename cplx_t<T>::t C;
     const auto &p = SC::last(a);
-    const int Q = p.NR, H = Q / 2 + 1;
-    for (int b = threadIdx.x; b < nt * H; b += blockDim.x) {
-        const int t = mdiv(b, a.mH), q = b - t * H;
+    // a column-major spectrum (DIF_R2CT) is stored with consecutive threads on
+    // adjacent rows: segments of 8 bytes times the tile's rows instead of single
+    // elements a column apart
+    constexpr bool TF = dif_rows_tf<KIND>();
+    const int Q = p.NR, H = Q / 2 + 1, V = !TF ? 1 : SC::V ? SC::V : a.vpb;
+    const int ct = TF ? ((int)threadIdx.x & (V - 1)) : 0;
+    if (TF && ct >= nt) return;
+    const int nb = TF ? H : nt * H, step = TF ? dif_by_v<SC>(a, (int)blockDim.x) : (int)blockDim.x;
+    for (int b = TF ? dif_by_v<SC>(a, (int)threadIdx.x) : (int)threadIdx.x; b < nb; b += step) {
+        const int t = TF ? ct : mdiv(b, a.mH), q = TF ? b : b - t * H;
         const C *su = s + (t * a.LD + SC::pos(a, q)), *sw = s + (t * a.LD + SC::pos(a, q ? Q - q : 0));
         C u[R], w[R];
 #pragma unroll
@@ -428,8 +477,8 @@ __device__ __forceinline__ void dif_passes(const DifArgs<T> &a, typename cplx_t<
 #undef JV_DIF_MID
         __syncthreads();
     }
-    if constexpr (KIND == DIF_R2C) {
-#define JV_DIF_LAST(R) (dif_last_r2c<SC, R, T>(a, s, nt, v0))
+    if constexpr (KIND == DIF_R2C || KIND == DIF_R2CT) {
+#define JV_DIF_LAST(R) (dif_last_r2c<SC, KIND, R, T>(a, s, nt, v0))
         JV_DIF_PAIR_SWITCH(a.p[a.np - 1].R, JV_DIF_LAST)
 #undef JV_DIF_LAST
     } else {
@@ -452,7 +501,7 @@ __device__ __forceinline__ void dif_passes_fix(const DifArgs<T> &a, typename cpl
     else dif_first<F, KIND, COLS, F::radix(0), T>(a, s, nt, v0);
     __syncthreads();
     dif_mids<F, 1, T, COLS>(a, s, nt);
-    if constexpr (KIND == DIF_R2C) dif_last_r2c<F, F::radix(F::np - 1), T>(a, s, nt, v0);
+    if constexpr (KIND == DIF_R2C || KIND == DIF_R2CT) dif_last_r2c<F, KIND, F::radix(F::np - 1), T>(a, s, nt, v0);
     else dif_last<F, KIND, COLS, F::radix(F::np - 1), T>(a, s, nt, v0);
 }
 
@@ -526,6 +575,8 @@ struct DifFixEntry {
     std::vector<int> radix;
     DifFixGo rows = nullptr, cols = nullptr, cols4 = nullptr;  // cols4: tiles of 4, for few columns
     DifFixGo step = nullptr, vec[3] = {nullptr, nullptr, nullptr};
+    DifFixGo taper = nullptr, power = nullptr;  // k-omega: R2C tiles of vtaper rows; power rows
+    int vtaper = 0;
 };
 const DifFixEntry *dif_fix(long N, int cls);  // cls 0: c2c, 1: R2C, 2: C2R; null: not in the table
 
@@ -574,6 +625,7 @@ JV_DIF_DECLARE(float, DIF_SPLIT, true)
 JV_DIF_DECLARE(float, DIF_R2C, false)
 JV_DIF_DECLARE(float, DIF_C2R, false)
 bool dif_step_go(const DifArgs<float> &a, int nthr, size_t smem, cudaStream_t st, unsigned groups);
+bool dif_komega_go(int kind, const DifArgs<float> &a, int nthr, size_t smem, cudaStream_t st);
 bool dif_vec_go(int kind, const DifArgs<float> &a, int nthr, size_t smem, cudaStream_t st, unsigned groups);
 
 }  // namespace jv

@@ -53,6 +53,24 @@ template <int N, int P1, int T, int VPB, int VC, int TC, int TV, int TL, int... 
     }
     return e;
 }
+// ... the k-omega pipeline's tapered R2C tiles (about 64 KB) and power rows ...
+constexpr int dif_taper_rows(int N) { return N <= 512 ? 16 : N <= 1024 ? 8 : 4; }
+template <int N, int P1, int T, int VPB, int... R> static DifFixEntry dif_fix_taper() {
+    DifFixEntry e;
+    e.N = N;
+    if constexpr (N <= 4096) {
+        constexpr int V = dif_taper_rows(N), W = (V * N / 16 + 31) / 32 * 32, NT = W < 96 ? 96 : W < 512 ? W : 512;
+        e.vtaper = V;
+        e.taper = dif_fix_go<DifFix<V, P1, R...>, DIF_R2CT, false, NT>;
+    }
+    return e;
+}
+template <int N, int P1, int T, int VPB, int VC, int TC, int TV, int TL, int... R> static DifFixEntry dif_fix_power() {
+    DifFixEntry e;
+    e.N = N;
+    if constexpr (N <= 4096) e.power = dif_fix_go<DifFix<1, P1, R...>, DIF_POWER, false, T>;
+    return e;
+}
 // ... and real rows.
 template <int KIND, int N, int P1, int T, int VPB, int... R> static DifFixEntry dif_fix_real() {
     static_assert((R * ...) == N, "radices give the length");

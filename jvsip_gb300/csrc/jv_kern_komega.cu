@@ -1,8 +1,11 @@
 // jv_kern_komega.cu -- the k-omega pipeline's instances of the shared-memory
 // kernel (single precision): R2C rows whose first pass tapers the real pairs
 // it loads (and writes them back), and c2c columns whose last pass stores the
-// power and accumulates it into the gram.  Views and lengths the
-// register-resident kernel takes go there first.
+// power and accumulates it into the gram.  The in-place mixed-radix kernel's
+// instances go first (a column-major spectrum), then the register-resident
+// kernel's.  4096 sensors x 4096 samples: 102 us (159 with both launches on the
+// register-resident kernel, whose R2C stores its spectrum one 8-byte element
+// per 32 KB column); 2500 x 3000: 57 us (137 on the shared-memory kernel).
 #include "jv_launch.cuh"
 
 namespace jv {
@@ -12,6 +15,8 @@ bool launch_komega_r2c_f32(const Job &j, cudaStream_t s) {
         return false;
     }
     const int e0 = jvsip_gpu_last_error();
+    if (launch_dif_komega_r2c_f32(j, s)) return true;
+    if (jvsip_gpu_last_error() != e0) return false;
     if (launch_fast_komega_r2c_f32(j, s)) return true;
     if (jvsip_gpu_last_error() != e0) return false;
     return launch_smem_t<float, KX_R2C_TAPER>(j, s);
@@ -22,6 +27,8 @@ bool launch_komega_power_f32(const Job &j, cudaStream_t s) {
         return false;
     }
     const int e0 = jvsip_gpu_last_error();
+    if (launch_dif_komega_power_f32(j, s)) return true;
+    if (jvsip_gpu_last_error() != e0) return false;
     if (launch_fast_komega_power_f32(j, s)) return true;
     if (jvsip_gpu_last_error() != e0) return false;
     return launch_smem_t<float, KX_C2C_POWER>(j, s);

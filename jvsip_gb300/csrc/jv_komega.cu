@@ -35,6 +35,8 @@ static void plan_job(Job &j, const Plan *p, int kind) {
     j.twp = p->d_twp;
     j.twg = p->d_twg;
     j.pc = p->d_pc;
+    j.dif = p->dif;
+    j.no_dif = p->no_dif;
     j.form = 0;
     j.no_fast = p->no_fast;  // JVSIP_GPU_NO_FAST: the shared-memory kernel's instances only
     j.tma_columns = p->tma_columns;

@@ -243,6 +243,17 @@ static void unit_root(long m, long N, double *c, double *s) {
     *s = flip ? sn : -sn;
 }
 
+// exp(-2 pi i m/N), m < N: every per-pass table of a length is a selection of
+// these (N/M times the exponent of a root of order M | N gives the same bits,
+// as both angles are the same quotient), so their sines are computed once
+std::vector<double> unit_roots(long N) {
+    std::vector<double> r(2 * (size_t)(N > 0 ? N : 1));
+    r[0] = 1.0;
+    r[1] = 0.0;
+    for (long m = 0; m < N; m++) unit_root(m, N, &r[2 * m], &r[2 * m + 1]);
+    return r;
+}
+
 // Device tables are shared by all plans of one (length, precision, kind):
 // a batch of thousands of plans over a few hundred lengths keeps one copy.
 struct TableSet {
@@ -263,7 +274,7 @@ static std::string sched_key(const std::vector<int> &r) {
 static int table_kind(int type) { return type == JV_RCFFTOP ? 1 : type == JV_CRFFTOP ? 2 : 0; }
 
 template <typename T>
-static bool build_tables(Plan *p);
+static bool build_tables(Plan *p, const std::vector<double> &roots);
 
 template <typename T>
 static bool make_tables(Plan *p) {
@@ -277,11 +288,12 @@ static bool make_tables(Plan *p) {
         p->d_twp = it->second.twp;
         p->d_twg = it->second.twg;
         p->d_pc = it->second.pc;
-        p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type));
+        p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type), nullptr);
         return true;
     }
-    if (!build_tables<T>(p)) return false;
-    p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type));
+    const std::vector<double> roots = unit_roots(p->MN);
+    if (!build_tables<T>(p, roots)) return false;
+    p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type), &roots);
     TableSet ts;
     ts.tw = p->d_tw;
     ts.thalf = p->d_thalf;
@@ -311,16 +323,11 @@ static void release_tables(Plan *p) {
 }
 
 template <typename T>
-static bool build_tables(Plan *p) {
+static bool build_tables(Plan *p, const std::vector<double> &roots) {
     long MN = p->MN;
     size_t n = (size_t)(MN > 0 ? MN : 1);
     std::vector<T> tw(2 * n, (T)0);
-    for (long m = 0; m < MN; m++) {
-        double c, s;
-        unit_root(m, MN, &c, &s);
-        tw[2 * m] = (T)c;
-        tw[2 * m + 1] = (T)s;
-    }
+    for (long m = 0; m < 2 * MN; m++) tw[m] = (T)roots[m];
     Device *d = device();
     if (!d) return false;
     p->d_tw = dmalloc(2 * n * sizeof(T));
@@ -333,12 +340,12 @@ static bool build_tables(Plan *p) {
         std::vector<T> tp;
         long Ns = 1;
         for (int R : radices) {
+            const long step = MN / (Ns * R);
             for (long r = 0; r < R; r++)
                 for (long m = 0; m < Ns; m++) {
-                    double c, s;
-                    unit_root((r * m) % (Ns * R), Ns * R, &c, &s);
-                    tp.push_back((T)c);
-                    tp.push_back((T)s);
+                    const T *w = &tw[2 * (r * m * step)];  // r*m < Ns*R
+                    tp.push_back(w[0]);
+                    tp.push_back(w[1]);
                 }
             Ns *= R;
         }

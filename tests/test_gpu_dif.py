@@ -201,3 +201,38 @@ def test_single_vectors(N, inplace):
         v.destroy()
     for b in (bx, bz, bo):
         b.destroy()
+
+
+@pytest.mark.parametrize("ns,nt", [(2, 8), (36, 60), (250, 500), (162, 3000), (700, 1050), (75, 8192), (1029, 128)])
+def test_komega_column_major(ns, nt):
+    """k-omega (lengths 2^a 3^b 5^c 7^d, as the call takes) in tiles that are not full, one row per tile, compiled-in schedules
+    and others: tapered data bit for bit (products rounded in order), power,
+    imaginary part and gram against numpy in 64 bits."""
+    g = np.random.default_rng(ns + nt)
+    nf = nt // 2 + 1
+    x = g.standard_normal((ns, nt)).astype(np.float32)
+    ts, arr = (g.uniform(0.5, 1.0, n).astype(np.float32) for n in (nt, ns))
+    gram = g.uniform(0, 1, (nf, ns)).astype(np.float32)
+    scale = np.float32(1.0 / (ns * nt))
+    bx, bg = J.RBlock(x.reshape(-1).copy(), admit=True), J.RBlock(gram.reshape(-1).copy(), admit=True)
+    bf = J.CBlock(np.zeros(2 * nf * ns, np.float32), admit=True)
+    bt, ba = J.RBlock(ts, admit=True), J.RBlock(arr, admit=True)
+    vx, vf, vg = bx.view(0, nt, ns, 1, nt), bf.view(0, 1, ns, ns, nf), bg.view(0, 1, ns, ns, nf)
+    vt, va = bt.vview(0, 1, nt), ba.vview(0, 1, ns)
+    rc = J.FFTM(J.KIND_RCOP, ns, nt, 1.0, J.VSIP_FFT_FWD, J.VSIP_ROW, ntimes=1)
+    cc = J.FFTM(J.KIND_CCIP, ns, nf, 1.0, J.VSIP_FFT_FWD, J.VSIP_COL, ntimes=1)
+    assert J.lib().jvsip_komega_f(rc.h, cc.h, vt.h, va.h, vx.h, vf.h, float(scale), vg.h) == 0, J.last_error()
+    for b in (bx, bf, bg):
+        b.sync()
+    tapered = (ts[None, :] * x) * arr[:, None]
+    assert np.array_equal(bx.a.reshape(ns, nt), tapered)
+    z = np.fft.fft(np.fft.rfft(tapered.astype(np.float64)).T)
+    power = float(scale) * np.abs(z) ** 2
+    f = bf.re.reshape(nf, ns, 2)
+    assert rel(f[..., 0], power) <= 2 * tol(ns * nt)
+    assert rel(f[..., 1], z.imag) <= tol(ns * nt)
+    assert rel(bg.a.reshape(nf, ns), gram.astype(np.float64) + power) <= 2 * tol(ns * nt)
+    for v in (vx, vf, vg, vt, va):
+        v.destroy()
+    for b in (bx, bf, bg, bt, ba):
+        b.destroy()
