@@ -82,28 +82,33 @@ static long bank_waves(const std::vector<int> &r, long N, long P1, int W) {
     return waves;
 }
 
-// The schedule of length N: the multiset of radices of least cost, in the
-// order and with the block pitch of the fewest shared-memory wavefronts
-// (larger first radices on ties).  Real transforms' pair pass (the last of
-// R2C, the first of C2R) takes a radix of at most kDifPairMax.  False when N
-// has a prime above 13 or fewer than two codelet factors.
-bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1) {
+// The multiset of radices of least cost with product N (empty: N has a prime
+// above 13 or fewer than two codelet factors).  Real transforms' pair pass (the
+// last of R2C, the first of C2R) takes a radix of at most kDifPairMax.
+static std::vector<int> least_cost(long N, int prec, int cls, double *cost) {
     std::vector<std::vector<int>> sets;
-    std::vector<int> cur;
-    if (N < 4 || N > 32768) return false;
+    std::vector<int> cur, pick;
+    *cost = 1e30;
+    if (N < 4 || N > 32768) return pick;
     multisets(N, 16, cur, sets);
-    if (sets.empty()) return false;
-    double best = 1e30;
-    std::vector<int> pick;
     for (const std::vector<int> &m : sets) {
         if (cls && m.back() > kDifPairMax) continue;
         double c = 0;
         for (int R : m) c += pass_cost(R, prec);
-        if (c < best) {
-            best = c;
+        if (c < *cost) {
+            *cost = c;
             pick = m;
         }
     }
+    return pick;
+}
+
+// The schedule of length N: the radices of least cost, in the order and with
+// the block pitch of the fewest shared-memory wavefronts (larger first radices
+// on ties).
+bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1) {
+    double cost;
+    const std::vector<int> pick = least_cost(N, prec, cls, &cost);
     if (pick.empty()) return false;
     const int W = prec == P_F32 ? 16 : 8;
     long bw = -1;
@@ -584,14 +589,11 @@ bool launch_dif_komega_power_f32(const Job &j, cudaStream_t st) {
 // W_N^(k1 t); pass 2: the whole table of BC entries), where the Stockham passes
 // before took two gathers per point.
 static double vec_cost(long n) {
-    std::vector<int> r;
-    long P1;
     if (n < 16 || n > 1024) return 1e30;
     const DifFixEntry *fix = dif_fix(n, 0);
-    if (fix) r = fix->radix;
-    else if (!dif_schedule(n, P_F32, 0, r, &P1)) return 1e30;
-    double c = 25;  // global accesses and the pass's own twiddle
-    for (int R : r) c += pass_cost(R, P_F32);
+    double c;
+    if (least_cost(n, P_F32, 0, &c).empty()) return 1e30;
+    c += 25;  // global accesses and the pass's own twiddle
     if (fix && fix->vec[0]) return c;
     return n > 512 ? c * 1.3 : c * 1.15;  // tiles of 8 transforms; no compiled-in schedule
 }
