@@ -41,8 +41,25 @@ struct Region {
     void *d_re = nullptr, *d_im = nullptr;
 };
 
+// The GPU reads and writes pageable host memory through the host's page tables
+// (Grace + Blackwell over NVLink-C2C).
+static bool host_access() {
+    // looked up once, thread-safely, on the first call
+    static const bool yes = []() {
+        int a = 0, b = 0;
+        Device *d = device();
+        return d && cudaDeviceGetAttribute(&a, cudaDevAttrPageableMemoryAccess, d->id) == cudaSuccess &&
+               cudaDeviceGetAttribute(&b, cudaDevAttrPageableMemoryAccessUsesHostPageTables, d->id) == cudaSuccess &&
+               a && b;
+    }();
+    return yes;
+}
+constexpr size_t kHostDirectMax = (size_t)64 << 20;
+
 struct Staging {
     std::vector<Region> regs;
+    bool inside = true;  // every staged view lies in its block
+    bool direct = false; // the kernels work on the host arrays themselves
     Region *find(const void *key) {
         for (auto &r : regs)
             if (r.key == key) return &r;
@@ -70,9 +87,33 @@ struct Staging {
         regs.push_back(n);
     }
     size_t bytes(const Region &r) const { return (size_t)(r.hi - r.lo + 1) * r.cst * r.esz; }
+    // whether the regions' host arrays are aligned, apart and small enough
+    bool apart() const {
+        std::vector<std::pair<const char *, const char *>> a;
+        size_t total = 0;
+        for (const Region &r : regs) {
+            const size_t b = bytes(r), o = (size_t)r.lo * r.cst * r.esz;
+            // a copy would start aligned, and so does every complex element here
+            if (!r.h_re || (uintptr_t)(r.h_re + o) % (2 * r.esz) || (uintptr_t)(r.h_im ? r.h_im + o : nullptr) % r.esz)
+                return false;
+            a.emplace_back(r.h_re + o, r.h_re + o + b);
+            if (r.h_im) a.emplace_back(r.h_im + o, r.h_im + o + b);
+            total += r.h_im ? 2 * b : b;
+        }
+        std::sort(a.begin(), a.end());
+        for (size_t i = 1; i < a.size(); i++)
+            if (a[i].first < a[i - 1].second) return false;
+        return total <= kHostDirectMax;
+    }
     bool upload(cudaStream_t st) {
         for (auto &r : regs) {
             size_t b = bytes(r);
+            if (direct) {
+                const size_t o = (size_t)r.lo * r.cst * r.esz;
+                r.d_re = r.h_re + o;
+                r.d_im = r.h_im ? r.h_im + o : nullptr;
+                continue;
+            }
             r.d_re = dmalloc(b);
             if (!r.d_re) return false;
             if (r.h_im) {
@@ -91,6 +132,7 @@ struct Staging {
     }
     bool download(cudaStream_t st) {
         bool ok = true;
+        if (direct) return ok;
         for (auto &r : regs) {
             if (!r.write || !r.d_re) continue;
             size_t b = bytes(r), o = (size_t)r.lo * r.cst * r.esz;
@@ -100,6 +142,7 @@ struct Staging {
         return ok;
     }
     ~Staging() {
+        if (direct) return;
         for (auto &r : regs) {
             dfree(r.d_re);
             dfree(r.d_im);
@@ -159,6 +202,7 @@ static void stage_c(Staging &s, const CRes<T, CB> &r, bool rd, bool wr) {
     bool split = (b->cstride == 1);
     char *h_re = (char *)b->R->array;
     char *h_im = split ? (char *)b->I->array : nullptr;
+    s.inside = s.inside && r.g.lo() >= 0 && r.g.hi() < (long)b->size;
     s.add(b, h_re, h_im, sizeof(T), split ? 1 : 2, r.g.lo(), r.g.hi(), rd, wr);
 }
 
@@ -216,6 +260,7 @@ static RRes<T, RB> resolve_r(const RB *b, const Geo &g) {
 template <typename T, typename RB>
 static void stage_r(Staging &s, const RRes<T, RB> &r, bool rd, bool wr) {
     if (r.dbase) return;
+    s.inside = s.inside && r.g.lo() >= 0 && r.g.hi() < (long)r.blk->size;
     s.add(r.blk, (char *)r.blk->array, nullptr, sizeof(T), r.rst, r.g.lo(), r.g.hi(), rd, wr);
 }
 
@@ -737,6 +782,19 @@ static void fill_job(Job &j, const Plan *p, int kind) {
     j.lp = p->lp;
 }
 
+// Whether a call on host blocks runs on the host arrays themselves, without
+// device copies: transforms along contiguous elements in one launch that reads
+// and writes every element once, 64 MiB in all, arrays that do not overlap.
+// The copies' calls and the half-duplex of copying in, then out, cost more than
+// the kernel's own C2C traffic (256 rows of 1000 complex floats 32 us against
+// 53 staged, 8 rows 14 against 30, 2000 x 1024 175 against 212; the first call
+// on untouched pages 52 against 77 us).  JVSIP_GPU_NO_PIPELINE keeps the copies.
+static bool host_direct(const Staging &s, const Job &j, long es_in, long es_out) {
+    if (s.regs.empty() || j.no_pipeline || j.form > JVSIP_FORM_PLAIN || es_in != 1 || es_out != 1) return false;
+    if (j.lp || !(job_in_smem(j) || (j.dif && !j.no_fast && !j.no_dif && j.N > 1))) return false;
+    return s.inside && s.apart() && host_access();
+}
+
 // Host-resident c2c call whose views are rows of unit element stride and
 // positive pitch (the common dense case): the transforms are cut into chunks
 // that flow host -> device (copy stream), kernel (library stream), device ->
@@ -851,6 +909,7 @@ static void exec_cc(Plan *p, const CMV *x, const CMV *y, bool ip) {
     cudaStream_t st = d->stream;
     stage_c(stg, rx, true, same_view);
     if (!same_view) stage_c(stg, ry, !ry.g.dense() || (y->block == x->block), true);
+    stg.direct = (same_view || x->block != y->block) && host_direct(stg, j, rx.g.es, ry.g.es);
     if (!stg.upload(st)) return;
     j.cin = dev_c(stg, rx);
     j.cout = same_view ? j.cin : dev_c(stg, ry);
@@ -957,6 +1016,7 @@ static void exec_rc(Plan *p, const RMV *x, const CMV *z) {
     cudaStream_t st = d->stream;
     stage_r(stg, rx, true, false);
     stage_c(stg, rz, !rz.g.dense(), true);
+    stg.direct = host_direct(stg, j, rx.g.es, rz.g.es);
     if (!stg.upload(st)) return;
     j.rin = dev_r(stg, rx);
     j.cout = dev_c(stg, rz);
@@ -992,6 +1052,7 @@ static void exec_cr(Plan *p, const CMV *z, const RMV *x) {
     cudaStream_t st = d->stream;
     stage_c(stg, rz, true, false);
     stage_r(stg, rx, !rx.g.dense(), true);
+    stg.direct = host_direct(stg, j, rz.g.es, rx.g.es);
     if (!stg.upload(st)) return;
     j.cin = dev_c(stg, rz);
     j.rout = dev_r(stg, rx);
