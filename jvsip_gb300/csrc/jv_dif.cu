@@ -228,7 +228,41 @@ static void *upload_tables(const std::vector<int> &rad, long N, const std::vecto
 // the best on average (us, transforms x threads): 100 points 12 x 128 45.3, 24
 // x 256 49.3, 32 x 192 49.3; 1200: 2 x 128 60.5, 4 x 256 62.6, 6 x 320 63.5;
 // 2400: 1 x 160 62.1, 2 x 320 67.8, 3 x 512 70.1.
+static double warp_rounds(long N, const std::vector<int> &rad, long v) {
+    double c = 0;
+    for (int R : rad) c += (double)((v * (N / R) + 31) / 32 * 32) * pass_cost(R, P_F64) * R;
+    return c / (double)(v * N);
+}
+// Whether double-precision rows run on this kernel rather than the
+// shared-memory kernel with schedule `smem`: by the warp rounds of both, to
+// which the times are proportional within 8 % over 58 lengths of 64-8192 points
+// (2^24 points, us: 100 1114 -> 867, 600 1470 -> 1184, 1000 1692 -> 1419, 1200
+// 1467 -> 1285; where the rounds are equal so are the times, 4096 1237 and 1225,
+// or this kernel's are longer, 1024 1021 and 1176).
+bool dif_f64_pays(const DifTab &t, const std::vector<int> &smem) {
+    return warp_rounds(t.N, smem, std::max(1L, 1024 / t.N)) >= 1.11 * warp_rounds(t.N, t.radix, t.vpb);
+}
+
+// Double precision: an FP64 instruction takes the pipe as long for one lane of
+// a warp as for 32, whatever else is resident, so the shape that fills its warps
+// best: the fewest warp rounds per point over the passes, in up to 72 KB (three
+// CTAs per SM).
+static void row_shape_f64(DifTab &t) {
+    const long ldb = t.radix[0] * t.P1 * 16;
+    double best = 1e30;
+    for (long v = 1; v == 1 || (v <= 16 && v * ldb <= 72 * 1024); v++) {
+        const double c = warp_rounds(t.N, t.radix, v);
+        const long most = v * (t.N / *std::min_element(t.radix.begin(), t.radix.end()));
+        if (c < best * 0.99) {
+            best = c;
+            t.vpb = v;
+            t.nthr = (int)std::min(256L, (most + 31) / 32 * 32);
+        }
+    }
+}
+
 static void row_shape(DifTab &t, int cls) {
+    if (t.prec == P_F64) return row_shape_f64(t);
     const long esz = t.prec == P_F32 ? 8 : 16, regs = t.prec == P_F32 ? 64 : 128, maxt = 65536 / regs;
     const long ldb = t.radix[0] * t.P1 * esz, unit = t.prec == P_F32 ? 1200 : 600;
     const size_t np = t.radix.size();
@@ -261,7 +295,7 @@ static void row_shape(DifTab &t, int cls) {
 }
 
 const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots) {
-    if (prec != P_F32 || N > 16384) return nullptr;
+    if (N > (prec == P_F32 ? 16384 : 8192) || (prec == P_F64 && cls != 0)) return nullptr;
     std::lock_guard<std::mutex> lk(g_dif_mu);
     auto key = std::make_tuple(N, prec, cls);
     auto it = g_dif.find(key);
@@ -436,11 +470,11 @@ static bool dif_args(const Job &j, long tuned, DifArgs<T> &a, DifCta &cta) {
             vpb = std::max(1L, std::min(tuned, (long)(cap / (a.LD * sizeof(C)))));
             nthr = std::min(512L, std::max(64L, (vpb * j.N / 16 + 31) / 32 * 32));
         } else if (tuned <= 0) {
-            // few transforms: smaller CTAs, so that more SMs work on them
-            while (vpb > 1 && (j.nvec + vpb - 1) / vpb < 2L * device()->sms) {
-                vpb = (vpb + 1) / 2;
-                nthr = std::max(64L, (vpb * j.N / 16 + 31) / 32 * 32);
-            }
+            // few transforms: smaller CTAs, so that more SMs work on them, with
+            // every pass in one round
+            while (vpb > 1 && (j.nvec + vpb - 1) / vpb < 2L * device()->sms) vpb = (vpb + 1) / 2;
+            if (vpb < t->vpb)
+                nthr = std::min(256L, (vpb * j.N / *std::min_element(t->radix.begin(), t->radix.end()) + 31) / 32 * 32);
         }
     } else {
         // Column tiles, 64 KB or less: 16 adjacent transforms (128-byte rows of
@@ -488,8 +522,8 @@ static bool launch_dif_t(const Job &j, cudaStream_t st) {
         if (c.split)
             return c.rows ? dif_go<T, DIF_SPLIT, false>(a, c.nthr, c.smem, st)
                           : dif_go<T, DIF_SPLIT, true>(a, c.nthr, c.smem, st);
-    } else if (c.split) {
-        return false;
+    } else if (c.split || (!c.rows && j.twg)) {
+        return false;  // columns: only lengths the shared-memory kernel has no codelets for
     }
     return c.rows ? dif_go<T, DIF_C2C, false>(a, c.nthr, c.smem, st) : dif_go<T, DIF_C2C, true>(a, c.nthr, c.smem, st);
 }
@@ -746,5 +780,6 @@ bool dif_tile_args(const Job &j, long tuned, DifArgs<float> &a, DifCta &c) {
 }
 
 bool launch_dif_f32(const Job &j, cudaStream_t st) { return launch_dif_t<float>(j, st); }
+bool launch_dif_f64(const Job &j, cudaStream_t st) { return launch_dif_t<double>(j, st); }
 
 }  // namespace jv

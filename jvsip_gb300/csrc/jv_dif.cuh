@@ -624,6 +624,8 @@ JV_DIF_DECLARE(float, DIF_SPLIT, false)
 JV_DIF_DECLARE(float, DIF_SPLIT, true)
 JV_DIF_DECLARE(float, DIF_R2C, false)
 JV_DIF_DECLARE(float, DIF_C2R, false)
+JV_DIF_DECLARE(double, DIF_C2C, false)
+JV_DIF_DECLARE(double, DIF_C2C, true)
 bool dif_step_go(const DifArgs<float> &a, int nthr, size_t smem, cudaStream_t st, unsigned groups);
 bool dif_komega_go(int kind, const DifArgs<float> &a, int nthr, size_t smem, cudaStream_t st);
 bool dif_vec_go(int kind, const DifArgs<float> &a, int nthr, size_t smem, cudaStream_t st, unsigned groups);

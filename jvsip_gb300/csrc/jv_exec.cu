@@ -636,7 +636,7 @@ static bool fast_first(const Job &j) {
 // One launch over whole transforms, on the register-resident or the in-place
 // mixed-radix kernel; false when neither takes the call.
 static bool run_tiles(const Job &j, cudaStream_t st) {
-    if (j.prec != P_F32) return false;
+    if (j.prec != P_F32) return launch_dif_f64(j, st);
     if (fast_first(j)) return launch_fast_f32(j, st) || launch_dif_f32(j, st);
     return launch_dif_f32(j, st) || launch_fast_f32(j, st);
 }

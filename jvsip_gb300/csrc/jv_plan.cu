@@ -276,6 +276,14 @@ static int table_kind(int type) { return type == JV_RCFFTOP ? 1 : type == JV_CRF
 template <typename T>
 static bool build_tables(Plan *p, const std::vector<double> &roots);
 
+static void take_dif(Plan *p, const std::vector<double> *roots) {
+    p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type), roots);
+    if (p->dif && p->prec == P_F64 && p->smooth && !dif_f64_pays(*p->dif, p->radix)) {
+        dif_release(p->dif);
+        p->dif = nullptr;
+    }
+}
+
 template <typename T>
 static bool make_tables(Plan *p) {
     auto key = std::make_tuple(p->MN, p->prec, table_kind(p->type), sched_key(p->radix));
@@ -288,12 +296,12 @@ static bool make_tables(Plan *p) {
         p->d_twp = it->second.twp;
         p->d_twg = it->second.twg;
         p->d_pc = it->second.pc;
-        p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type), nullptr);
+        take_dif(p, nullptr);
         return true;
     }
     const std::vector<double> roots = unit_roots(p->MN);
     if (!build_tables<T>(p, roots)) return false;
-    p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type), &roots);
+    take_dif(p, &roots);
     TableSet ts;
     ts.tw = p->d_tw;
     ts.thalf = p->d_thalf;

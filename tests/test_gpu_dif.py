@@ -236,3 +236,27 @@ def test_komega_column_major(ns, nt):
         v.destroy()
     for b in (bx, bf, bg, bt, ba):
         b.destroy()
+
+
+@pytest.mark.parametrize("N", [22, 81, 100, 143, 600, 1000, 2197, 5632, 6561, 8125])
+def test_double_rows_and_columns(N):
+    """Double precision: rows that fill their warps better here than in the
+    shared-memory kernel, and lengths with factors 11 and 13 (columns too).
+    Tolerance: rel-L2 1e-14 log2 N, the library's bound for double precision."""
+    g = np.random.default_rng(N)
+    for m, col in ((1, False), (37, False), (3, True)):
+        z = g.standard_normal(m * N) + 1j * g.standard_normal(m * N)
+        y = np.zeros(2 * m * N)
+        bx, by = J.CBlock(z.view(np.float64).copy(), admit=True), J.CBlock(y, admit=True)
+        shape = (0, m, N, 1, m) if col else (0, N, m, 1, N)
+        vx, vy = bx.view(*shape), by.view(*shape)
+        a, b = (N, m) if col else (m, N)
+        p = J.FFTM(J.KIND_CCOP, a, b, 1.0 / N, J.VSIP_FFT_INV, J.VSIP_COL if col else J.VSIP_ROW, dtype=np.float64)
+        p.ccfftmop(vx, vy)
+        by.sync()
+        ref = np.fft.ifft(z.reshape(a, b), axis=0 if col else 1)
+        assert rel(y.view(np.complex128).reshape(a, b), ref) <= 1e-14 * np.log2(N)
+        for v in (vx, vy):
+            v.destroy()
+        for blk in (bx, by):
+            blk.destroy()
