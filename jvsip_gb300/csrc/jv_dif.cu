@@ -135,6 +135,8 @@ void dif_fix_c2c_1(std::vector<DifFixEntry> &out);
 void dif_fix_c2c_2(std::vector<DifFixEntry> &out);
 void dif_fix_c2c_3(std::vector<DifFixEntry> &out);
 void dif_fix_long_1(std::vector<DifFixEntry> &out);
+void dif_fix_rows_1(std::vector<DifFixEntry> &out);
+void dif_fix_rows_2(std::vector<DifFixEntry> &out);
 void dif_fix_taper_1(std::vector<DifFixEntry> &out);
 void dif_fix_taper_2(std::vector<DifFixEntry> &out);
 void dif_fix_power_1(std::vector<DifFixEntry> &out);
@@ -151,6 +153,8 @@ const DifFixEntry *dif_fix(long N, int cls) {
         dif_fix_c2c_1(v[0]);
         dif_fix_c2c_2(v[0]);
         dif_fix_c2c_3(v[0]);
+        dif_fix_rows_1(v[0]);
+        dif_fix_rows_2(v[0]);
         dif_fix_r2c_1(v[1]);
         dif_fix_r2c_2(v[1]);
         dif_fix_c2r_1(v[2]);
@@ -239,7 +243,7 @@ static double warp_rounds(long N, const std::vector<int> &rad, long v) {
 // (2^24 points, us: 100 1114 -> 867, 600 1470 -> 1184, 1000 1692 -> 1419, 1200
 // 1467 -> 1285; where the rounds are equal so are the times, 4096 1237 and 1225,
 // or this kernel's are longer, 1024 1021 and 1176).
-bool dif_f64_pays(const DifTab &t, const std::vector<int> &smem) {
+static bool dif_f64_pays(const DifTab &t, const std::vector<int> &smem) {
     return warp_rounds(t.N, smem, std::max(1L, 1024 / t.N)) >= 1.11 * warp_rounds(t.N, t.radix, t.vpb);
 }
 
@@ -294,7 +298,8 @@ static void row_shape(DifTab &t, int cls) {
     }
 }
 
-const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots) {
+const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots,
+                          const std::vector<int> *other) {
     if (N > (prec == P_F32 ? 16384 : 8192) || (prec == P_F64 && cls != 0)) return nullptr;
     std::lock_guard<std::mutex> lk(g_dif_mu);
     auto key = std::make_tuple(N, prec, cls);
@@ -322,6 +327,7 @@ const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *
         if (seen->second.radix.empty()) return nullptr;  // no schedule
         t = seen->second;
     }
+    if (other && !dif_f64_pays(t, *other)) return nullptr;
     const int err0 = jvsip_gpu_last_error();
     std::vector<double> own;
     if (!roots) {
@@ -707,7 +713,7 @@ VecPlan *vec_acquire(long N) {
     bool ok = true;
     for (int i = 0; i < 3; i++) {
         v->f[i] = f[i];
-        if (f[i] > 1) ok = ok && (v->tab[i] = dif_acquire(f[i], P_F32, 0, nullptr)) != nullptr;
+        if (f[i] > 1) ok = ok && (v->tab[i] = dif_acquire(f[i], P_F32, 0, nullptr, nullptr)) != nullptr;
     }
     ok = ok && (v->d_t1 = upload_roots(f[0] * V, [&](long i) { return (i / V) * (i % V); }, N)) != nullptr;
     const long C = f[2];

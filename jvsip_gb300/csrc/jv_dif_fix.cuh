@@ -71,7 +71,7 @@ template <int N, int P1, int T, int VPB, int VC, int TC, int TV, int TL, int... 
     if constexpr (N <= 4096) e.power = dif_fix_go<DifFix<1, P1, R...>, DIF_POWER, false, T>;
     return e;
 }
-// ... and real rows.
+// ... and real rows, and the rows-only lengths.
 template <int KIND, int N, int P1, int T, int VPB, int... R> static DifFixEntry dif_fix_real() {
     static_assert((R * ...) == N, "radices give the length");
     DifFixEntry e;

@@ -277,11 +277,8 @@ template <typename T>
 static bool build_tables(Plan *p, const std::vector<double> &roots);
 
 static void take_dif(Plan *p, const std::vector<double> *roots) {
-    p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type), roots);
-    if (p->dif && p->prec == P_F64 && p->smooth && !dif_f64_pays(*p->dif, p->radix)) {
-        dif_release(p->dif);
-        p->dif = nullptr;
-    }
+    p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type), roots,
+                         p->prec == P_F64 && p->smooth ? &p->radix : nullptr);
 }
 
 template <typename T>

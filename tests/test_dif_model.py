@@ -117,6 +117,7 @@ def test_table_covers_its_lengths_once():
     assert [r[0] for r in t["c2c"]] == smooth
     for kind in ("r2c", "c2r"):
         assert [r[0] for r in t[kind]] == [n for n in smooth if n <= 8192]
+    assert [r[0] for r in t["rows"]] == [n for n in range(40, 16385) if any(n % p == 0 and _smooth(n // p) for p in (7, 11, 13))]
 
 
 def _smooth(n):
@@ -126,7 +127,7 @@ def _smooth(n):
     return n == 1
 
 
-@pytest.mark.parametrize("kind", ["c2c", "r2c", "c2r"])
+@pytest.mark.parametrize("kind", ["c2c", "r2c", "c2r", "rows"])
 def test_table_entries_fit_the_kernel(kind):
     """Radices give the length and are codelets (pair passes at most 10), blocks
     do not overlap, every CTA's threads and shared memory exist, and index
