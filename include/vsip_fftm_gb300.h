@@ -356,8 +356,8 @@ int jvsip_fftm_setform_d(vsip_fftm_d *plan, int form);
 int jvsip_fftm_getform_d(const vsip_fftm_d *plan);
 
 /* Batching form: run n independent c2c fftm calls (each plan with its own
- * input/output views; ccfftmop or ccfftmip plans) as one persistent launch fed
- * by a device work queue of (plan, row-tile) descriptors.  Equivalent to
+ * input/output views; ccfftmop or ccfftmip plans) as one launch per block size,
+ * each fed by a device work queue of (call, tile) descriptors.  Equivalent to
  * calling vsip_ccfftmop_f / vsip_ccfftmip_f for i = 0..n-1 (in-place plans
  * use in[i]; out[i] is ignored).  Views must be of admitted blocks.
  * Returns 0 on success. */

@@ -10,10 +10,11 @@
 // Columns from kColStepsMin points (adjacent, more than one) go through the
 // plain calls' two steps on eight streams of their own.  Other layouts, and
 // lengths without a schedule of two codelets, keep the general kernel's fused
-// c2c passes in CTAs of 256, 512 or 1024 threads (k_batch), each CTA asking L2
+// c2c passes in CTAs of 256, 512 or 1024 threads (k_batch; long adjacent
+// columns in 4-CTA clusters, k_batch_cols), each CTA asking L2
 // for the input of the descriptor one resident wave further down its queue.
 // The launches run side by side on forked streams.  160 instances of 64-16384
-// points (0.58 GB per buffer) on GB300: 0.60 ms against 0.79 with every tile
+// points (0.58 GB per buffer) on GB300: 0.56 ms against 0.80 with every tile
 // on the general kernel's passes and only columns from 8192 points in steps.
 // A captured batch (jvsip_fftm_batch_create_f) records the launches in a CUDA
 // graph once; jvsip_fftm_batch_run_f replays it.

@@ -151,8 +151,9 @@ struct CallGraph {
 };
 void count_launch_undo(unsigned long long n);  // launches recorded by a capture did not run
 
-// A transform of N = N1 * N2 points too long for one CTA, as two steps of the
-// shared-memory kernel: A, N1 transforms of N2 points down the columns of x
+// A transform of N = N1 * N2 points too long for one CTA, as two steps
+// (register-resident or in-place mixed-radix column tiles where the views and
+// lengths allow, else the shared-memory kernel): A, N1 transforms of N2 points down the columns of x
 // seen as an N2 x N1 row-major matrix (x[n1 + N1*n2]), each output element k2
 // multiplied by W_N^(n1*k2) and stored as row n1 of an N1 x N2 scratch
 // matrix; B, N2 transforms of N1 points down the scratch's columns, element

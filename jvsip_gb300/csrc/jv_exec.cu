@@ -441,7 +441,7 @@ static bool long_c2c(const Job &j, LongPlan *lp, const CView &in, const CView &o
     return two_steps(j, lp, in, out, nv, conj_in, conj_out, has_scale, scale, sc, esz, st);
 }
 
-// A single vector of 2^n points (single precision, interleaved, unit stride)
+// A single vector of 2^13 .. 2^20 points (single precision, interleaved, unit stride)
 // as large-radix Stockham passes (LongPlan::sp_radix): pass p reads element n
 // of transform j at j + n*N/R_p, multiplies it by W_N^(n*m*N/(Ns*R_p)),
 // m = j mod Ns, and writes output k at (j - m)*R_p + m + k*Ns, Ns = R_0...R_{p-1};
@@ -557,8 +557,8 @@ static bool long_few(const Job &j) {
 // with a decomposition from kColStepsMin points, not taken by the
 // register-resident column tiles: two steps whatever their count.  Measured on
 // 1000 columns (us), the steps on the in-place mixed-radix kernel against the
-// shared-memory kernel's: 3000 points 27.4 against 36.5, 6000: 45.2 against
-// 57.1, 12000: 83.5 against 112.5; steps of lengths that the register-resident
+// shared-memory kernel's: 3000 points 24.5 against 36.5, 6000: 45 against
+// 57, 12000: 80 against 112; steps of lengths that the register-resident
 // tiles take run there (16384 x 1000: 88).  One launch of the in-place
 // kernel's 4-column tiles instead: 3000 points 26.8, 3125: 36.9 (34.8 in the
 // steps), 4000 and longer slower.

@@ -6,8 +6,8 @@
 //    (powers of two up to the 16384-point tile limit) timed through the batch
 //    call on scratch data;
 //  * the plain calls' kernel choice (jvsip_fftm_autotune_plain_f): residency
-//    (the register-resident kernel where an instance exists, or the
-//    shared-memory kernel), the shared-memory kernel's radix schedule, its
+//    (the default route -- the register-resident or the in-place mixed-radix
+//    kernel -- or the shared-memory kernel), the shared-memory kernel's radix schedule, its
 //    transforms per CTA and its complex values per thread and pass (which sets
 //    the threads per transform), each candidate timed through vsip_ccfftmip_f
 //    on scratch data.  Plans created afterwards take the entry of their length,
