@@ -395,6 +395,13 @@ template <typename T> static void dif_fill(DifArgs<T> &a, const DifTab &t) {
     }
 }
 
+// Points of a column call from which tiles of 4 columns are too narrow.  Tiles of
+// 4 against 8 (run-time schedule) at 2^26 points, us: 1125 points 475 and 321,
+// 1350: 499 and 334, 1500: 499 and 436, 1792: 482 and 410, 1920: 441 and 336, 2048:
+// 393 and 334 (1944: 422 and 485); at 2^25 points 1500: 214 and 222, 2000: 199 and
+// 232, 2048: 150 and 168.
+constexpr long kColWidePts = 5L << 23;
+
 // The kernel's arguments for a call and its CTA: tuned > 0 asks for that many
 // transforms (a power of two for column tiles).  False when the call does not
 // qualify.
@@ -495,6 +502,11 @@ static bool dif_args(const Job &j, long tuned, DifArgs<T> &a, DifCta &cta) {
         if (t->fix && t->fix->vcol)
             for (a.lgv = 0; (1 << a.lgv) < t->fix->vcol; a.lgv++) {
             }
+        // calls far beyond L2: rows of 32 bytes, a megabyte and more apart, cost
+        // memory twice their bytes, so tiles of 8 wherever they fit
+        if (sizeof(T) == 4 && a.lgv == 2 && j.nbatch <= 1 && (j.N << 3) <= 16384 &&
+            j.nvec * j.N >= kColWidePts)
+            a.lgv = 3;
         // few columns: tiles of 4, so that more SMs work on them
         if (((j.nvec - 1) >> a.lgv) + 1 < device()->sms && j.nbatch <= 1) a.lgv = std::min(a.lgv, 2);
         if (tuned > 0)

@@ -621,7 +621,12 @@ static bool run_long(Job &j, cudaStream_t st, bool *handled) {
 // 45.2 / 49.2 / 48.9 against 47.0 / 51.2 / 49.4, when they fill the GPU (64 rows
 // of 512: 6.2 against 4.0); R2C of 512 points 28.7 against 30.8, C2R of 512 32.8
 // and 33.0 (4096 rows: 6.2 and 8.2), R2C and C2R of 8192 points 34.8 against
-// 38; columns of 4096 points 53 against 61.  At its
+// 38; columns of 4096 points 53 against 61.  Large calls on columns of powers of
+// two, whose rows of a tile lie a large stride apart, keep its 16-column and
+// wider tiles: 64 points 159 against 171 us on 2^26 points, 25.1 and 26.6 on 2^23,
+// equal on 2^20 and below; 256 points 84.2 and 85.8 on 2^25, 6.7 and 7.2 on 2^20;
+// 128 points 160.3 and 162.9 on 2^26, 26.6 and 26.6 on 2^23, 10.2 and 8.3 on 2^21;
+// 512 points 194 and 295 on 2^26, 102 and 115 on 2^25, 33.0 and 31.0 on 2^23.  At its
 // other lengths the in-place kernel is the faster one or as fast (rows of 128 /
 // 1000 / 1024 points 41.8 / 51.3 / 43.7 against 43.6 / 70.4 / 47.1; R2C of 1536
 // 32.9 against 34.1, C2R 32.9 against 35.1; columns of 1000 35.0 against 41.0).
@@ -630,7 +635,9 @@ static bool fast_first(const Job &j) {
     if (j.cin.cst != 2) return true;  // split complex
     if (j.cin.es == 1 && j.cout.es == 1)
         return (j.N == 512 || j.N == 768 || j.N == 4096) && j.nvec * j.N >= 4096L * device()->sms;
-    return j.N == 4096;
+    const long pts = j.nvec * j.N;
+    return j.N == 4096 || ((j.N == 64 || j.N == 256) && pts >= (1L << 20)) || (j.N == 512 && pts >= (1L << 24)) ||
+           (j.N == 128 && pts >= (1L << 25));
 }
 
 // One launch over whole transforms, on the register-resident or the in-place

@@ -68,6 +68,10 @@ static bool launch_fast_rows(const Job &j, cudaStream_t st) {
 template <bool SPLIT, int FXK = 0>
 static bool launch_fast_cols(const Job &j, cudaStream_t st) {
     switch (j.N) {
+        case 64: return launch_fast_n<64, 4, 64, RList<16, 4>, SPLIT, true, false, false, 0, FXK>(j, st);
+        case 256: return launch_fast_n<256, 16, 16, RList<16, 16>, SPLIT, true, false, false, 0, FXK>(j, st);
+        case 128: return launch_fast_n<128, 8, 32, RList<16, 8>, SPLIT, true, false, false, 0, FXK>(j, st);
+        case 512: return launch_fast_n<512, 32, 16, RList<16, 16, 2>, SPLIT, true, false, false, 0, FXK>(j, st);
         // 4096 points: 4 columns per 1024-thread CTA (139 KB of shared memory),
         // 2874 GB/s on 4096 x 4096 against 1807 for 2 columns per CTA and 1823
         // for the shared-memory kernel
@@ -76,10 +80,6 @@ static bool launch_fast_cols(const Job &j, cudaStream_t st) {
     }
     if constexpr (SPLIT || FXK != 0) {
         switch (j.N) {
-            case 64: return launch_fast_n<64, 4, 64, RList<16, 4>, SPLIT, true, false, false, 0, FXK>(j, st);
-            case 128: return launch_fast_n<128, 8, 32, RList<16, 8>, SPLIT, true, false, false, 0, FXK>(j, st);
-            case 256: return launch_fast_n<256, 16, 16, RList<16, 16>, SPLIT, true, false, false, 0, FXK>(j, st);
-            case 512: return launch_fast_n<512, 32, 16, RList<16, 16, 2>, SPLIT, true, false, false, 0, FXK>(j, st);
             case 1000: return launch_fast_n<1000, 100, 4, RList<10, 10, 10>, SPLIT, true, false, false, 0, FXK>(j, st);
             case 1024: return launch_fast_n<1024, 64, 8, RList<16, 16, 4>, SPLIT, true, false, false, 0, FXK>(j, st);
             case 2048: return launch_fast_n<2048, 128, 4, RList<16, 16, 8>, SPLIT, true, false, false, 0, FXK>(j, st);

@@ -99,6 +99,28 @@ def test_columns(N, cols, extra, inplace):
         b.destroy()
 
 
+# large calls: power-of-two columns go back to the register-resident tiles, tiles
+# of 4 columns become 8; ragged counts, first, middle and last columns
+@pytest.mark.parametrize("N,cols", [(64, 16391), (256, 4099), (512, 32773), (128, 262147), (1350, 24859), (1792, 18727)])
+def test_large_column_calls(N, cols):
+    z = rnd(N * cols, N)
+    bx = J.CBlock(z.copy().view(np.float32), admit=True)
+    by = J.CBlock(np.zeros(2 * N * cols, np.float32), admit=True)
+    vx, vy = bx.view(0, cols, N, 1, cols), by.view(0, cols, N, 1, cols)
+    p = J.FFTM(J.KIND_CCOP, N, cols, 1.0, J.VSIP_FFT_FWD, J.VSIP_COL, ntimes=1)
+    n0 = J.lib().jvsip_gpu_kernel_launches()
+    p.ccfftmop(vx, vy)
+    assert J.lib().jvsip_gpu_kernel_launches() - n0 == 1
+    by.sync()
+    pick = np.unique(np.r_[0:17, cols // 2 - 8:cols // 2 + 9, cols - 17:cols])
+    got, src = by.re.view(np.complex64).reshape(N, cols)[:, pick], z.reshape(N, cols)[:, pick]
+    assert rel(got, np.fft.fft(src.astype(np.complex128), axis=0)) <= tol(N)
+    for v in (vx, vy):
+        v.destroy()
+    for b in (bx, by):
+        b.destroy()
+
+
 @pytest.mark.parametrize("N", LENGTHS)
 @pytest.mark.parametrize("m,pad,colmajor", [(1, 0, False), (53, 4, False), (6, 0, True)])
 def test_real_rows(N, m, pad, colmajor):
