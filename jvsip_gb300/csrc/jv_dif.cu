@@ -232,9 +232,15 @@ static void *upload_tables(const std::vector<int> &rad, long N, const std::vecto
 // the best on average (us, transforms x threads): 100 points 12 x 128 45.3, 24
 // x 256 49.3, 32 x 192 49.3; 1200: 2 x 128 60.5, 4 x 256 62.6, 6 x 320 63.5;
 // 2400: 1 x 160 62.1, 2 x 320 67.8, 3 x 512 70.1.
-static double warp_rounds(long N, const std::vector<int> &rad, long v) {
+static double warp_rounds(long N, const std::vector<int> &rad, long v, bool dit) {
     double c = 0;
-    for (int R : rad) c += (double)((v * (N / R) + 31) / 32 * 32) * pass_cost(R, P_F64) * R;
+    for (size_t i = 0; i < rad.size(); i++) {
+        // radix 16: one instruction per point fewer where the twiddles precede
+        // the butterfly (tw_bfly), in every pass but the first
+        const int R = rad[i];
+        const double per = pass_cost(R, P_F64) - (dit && R == 16 && i > 0 ? 1.0 : 0.0);
+        c += (double)((v * (N / R) + 31) / 32 * 32) * per * R;
+    }
     return c / (double)(v * N);
 }
 // Whether double-precision rows run on this kernel rather than the
@@ -244,7 +250,7 @@ static double warp_rounds(long N, const std::vector<int> &rad, long v) {
 // 1467 -> 1285; where the rounds are equal so are the times, 4096 1237 and 1225,
 // or this kernel's are longer, 1024 1021 and 1176).
 static bool dif_f64_pays(const DifTab &t, const std::vector<int> &smem) {
-    return warp_rounds(t.N, smem, std::max(1L, 1024 / t.N)) >= 1.11 * warp_rounds(t.N, t.radix, t.vpb);
+    return warp_rounds(t.N, smem, std::max(1L, 1024 / t.N), true) >= 1.11 * warp_rounds(t.N, t.radix, t.vpb, false);
 }
 
 // Double precision: an FP64 instruction takes the pipe as long for one lane of
@@ -255,7 +261,7 @@ static void row_shape_f64(DifTab &t) {
     const long ldb = t.radix[0] * t.P1 * 16;
     double best = 1e30;
     for (long v = 1; v == 1 || (v <= 16 && v * ldb <= 72 * 1024); v++) {
-        const double c = warp_rounds(t.N, t.radix, v);
+        const double c = warp_rounds(t.N, t.radix, v, false);
         const long most = v * (t.N / *std::min_element(t.radix.begin(), t.radix.end()));
         if (c < best * 0.99) {
             best = c;
