@@ -253,6 +253,19 @@ static bool dif_f64_pays(const DifTab &t, const std::vector<int> &smem) {
     return warp_rounds(t.N, smem, std::max(1L, 1024 / t.N), true) >= 1.11 * warp_rounds(t.N, t.radix, t.vpb, false);
 }
 
+// False where no number of transforms per CTA would make it pay: known from the
+// radices alone, so that a plan whose rows stay on the shared-memory kernel is
+// made without the search for their order and pitch (0.1 to 0.3 ms).
+static bool dif_f64_may_pay(long N, const std::vector<int> &smem) {
+    double cost;
+    const std::vector<int> rad = least_cost(N, P_F64, 0, &cost);
+    if (rad.empty()) return false;
+    const double s = warp_rounds(N, smem, std::max(1L, 1024 / N), true);
+    for (long v = 1; v <= 16; v++)
+        if (s >= 1.11 * warp_rounds(N, rad, v, false)) return true;
+    return false;
+}
+
 // Double precision: an FP64 instruction takes the pipe as long for one lane of
 // a warp as for 32, whatever else is resident, so the shape that fills its warps
 // best: the fewest warp rounds per point over the passes, in up to 72 KB (three
@@ -327,6 +340,7 @@ const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *
     if (!fix) {
         auto seen = g_found.find(key);
         if (seen == g_found.end()) {
+            if (other && !dif_f64_may_pay(N, *other)) return nullptr;
             if (dif_schedule(N, prec, cls, t.radix, &t.P1)) row_shape(t, cls);
             seen = g_found.emplace(key, t).first;
         }
