@@ -589,8 +589,6 @@ static bool batch_streams() {
     return ok;
 }
 
-
-
 static bool launch_group(const DevBatch &db, const DevBatch::Group &g, cudaStream_t st) {
     return dif_batch_go(g.cols, db.calls, db.tiles + g.first, g.n, g.nthr, g.smem, st);
 }
