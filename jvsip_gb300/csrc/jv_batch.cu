@@ -33,6 +33,7 @@
 #include <cooperative_groups.h>
 
 #include "jv_dif.cuh"
+#include "jv_dif_tile.h"
 #include "jv_launch.cuh"
 
 namespace jv {
@@ -299,7 +300,7 @@ static bool dif_tiles(const Plan *p, const TileDesc &t, long nv, BatchBuild &bb)
         c.smem > device()->smem_optin - kStaticArgs)
         return false;
     // block sizes in steps of 64, so that one launch takes tiles of many lengths
-    c.nthr = (c.nthr + 63) / 64 * 64;
+    c.nthr = dif_batch_threads(c.nthr);
     DifGroup *g = nullptr;
     for (DifGroup &h : bb.groups)
         if (h.cols == !c.rows && h.nthr == c.nthr) g = &h;

@@ -13,6 +13,7 @@
 #include <tuple>
 
 #include "jv_dif.cuh"
+#include "jv_dif_tile.h"
 
 namespace jv {
 
@@ -529,13 +530,10 @@ static bool dif_args(const Job &j, long tuned, DifArgs<T> &a, DifCta &cta) {
             a.lgv = 3;
         // few columns: tiles of 4, so that more SMs work on them
         if (((j.nvec - 1) >> a.lgv) + 1 < device()->sms && j.nbatch <= 1) a.lgv = std::min(a.lgv, 2);
-        if (tuned > 0)
-            for (a.lgv = 0; (2L << a.lgv) <= tuned; a.lgv++) {
-            }
+        if (tuned > 0) a.lgv = dif_col_tuned(tuned, j.nvec);
         while (a.lgv > 0 && ((size_t)a.LD << a.lgv) * sizeof(C) > cap) a.lgv--;
         vpb = 1L << a.lgv;
-        nthr = std::max(64L, (vpb * j.N / 16 + 31) / 32 * 32);
-        if (nthr > 512) nthr = (sizeof(T) == 4 && vpb * j.N > 16384) ? std::min(1024L, nthr) : 512;
+        nthr = dif_col_threads(j.N, a.lgv, sizeof(T) == 4);
     }
     a.vpb = (int)vpb;
     cta.nthr = (int)nthr;

@@ -168,12 +168,13 @@ long batch_fft_per_tile(long N, bool vf, long rows) {
     return std::max(1L, per);
 }
 
-// the tuned FFTs per tile, 0 when the length was never tuned
+// the tuned FFTs per tile (16384 points at most, as above), 0 when the length
+// was never tuned
 long batch_tuned_per_tile(long N, bool vf) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     load_cache();
     auto it = g_tuned.find(std::make_tuple(N, (int)P_F32, vf ? 1 : 0));
-    return it != g_tuned.end() ? it->second : 0;
+    return it != g_tuned.end() ? std::min(it->second, std::max(1L, 16384 / N)) : 0;
 }
 
 long tuned_entries() {
