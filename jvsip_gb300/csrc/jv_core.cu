@@ -87,8 +87,8 @@ static int *g_ks = nullptr;
 int *kernel_status() {
     std::lock_guard<std::mutex> lk(g_ks_mu);
     if (!g_ks) {
-        g_ks = (int *)dmalloc(sizeof(int));
-        if (g_ks && cudaMemset(g_ks, 0, sizeof(int)) != cudaSuccess) g_ks = nullptr;
+        const int zero = 0;
+        g_ks = (int *)table_upload(&zero, sizeof zero, "kernel status");
     }
     return g_ks;
 }
@@ -129,7 +129,8 @@ static size_t size_class(size_t b) {
     return (b + (2u << 20) - 1) & ~((size_t)(2u << 20) - 1);
 }
 
-void *dmalloc(size_t bytes) {
+// *reused: handed out before, so queued work of the library stream may still use it
+static void *pool_take(size_t bytes, bool *reused) {
     if (!device()) return nullptr;
     size_t c = size_class(bytes ? bytes : 1);
     {
@@ -139,6 +140,7 @@ void *dmalloc(size_t bytes) {
             void *p = it->second;
             g_free.erase(it);
             g_live[p] = c;
+            *reused = true;
             return p;
         }
     }
@@ -153,6 +155,27 @@ void *dmalloc(size_t bytes) {
     std::lock_guard<std::mutex> lk(g_pool_mu);
     g_live[p] = c;
     return p;
+}
+
+void *dmalloc(size_t bytes) {
+    bool reused = false;
+    return pool_take(bytes, &reused);
+}
+
+// Buffers go back to the pool while work that reads them is queued on the
+// library stream, whose later work alone may write them: the copy into such a
+// buffer takes its turn there.  A copy into new memory waits for nothing.
+void *table_upload(const void *src, size_t bytes, const char *what) {
+    Device *d = device();
+    bool reused = false;
+    void *p = d ? pool_take(bytes, &reused) : nullptr;
+    if (!p) return nullptr;
+    const cudaStream_t st = reused ? d->stream : d->h2d;
+    if (cuda_ok(cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, st), what) &&
+        cuda_ok(cudaStreamSynchronize(st), what))
+        return p;
+    dfree(p);
+    return nullptr;
 }
 
 void dfree(void *p) {

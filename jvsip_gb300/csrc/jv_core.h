@@ -49,6 +49,9 @@ void count_launch(unsigned n = 1);
 // Caching device allocator: freed buffers are kept per exact size class and
 // reused, so repeated calls do not cudaMalloc.  Thread-safe.
 void *dmalloc(size_t bytes);
+// A buffer holding a copy of `bytes` of host memory (a table that later calls
+// read), there when this returns; nullptr with the error recorded.
+void *table_upload(const void *src, size_t bytes, const char *what);
 void dfree(void *p);
 void pool_trim();
 

@@ -216,13 +216,7 @@ static void *upload_tables(const std::vector<int> &rad, long N, const std::vecto
         M = S;
     }
     two.push_back(0);
-    void *d = dmalloc(tw.size() * sizeof(T));
-    if (!d) return nullptr;
-    if (!cuda_ok(cudaMemcpy(d, tw.data(), tw.size() * sizeof(T), cudaMemcpyHostToDevice), "twiddle upload")) {
-        dfree(d);
-        return nullptr;
-    }
-    return d;
+    return table_upload(tw.data(), tw.size() * sizeof(T), "twiddle upload");
 }
 
 // CTA shape of row calls: vpb transforms in nthr threads, chosen by the idle
@@ -708,12 +702,7 @@ template <typename F> static void *upload_roots(long n, F exponent, long N) {
         t[2 * i] = (float)c;
         t[2 * i + 1] = (float)s;
     }
-    void *d = dmalloc(t.size() * sizeof(float));
-    if (d && !cuda_ok(cudaMemcpy(d, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice), "twiddle upload")) {
-        dfree(d);
-        d = nullptr;
-    }
-    return d;
+    return table_upload(t.data(), t.size() * sizeof(float), "twiddle upload");
 }
 
 // adjacent transforms per tile: 128-byte segments, fewer while they leave SMs idle

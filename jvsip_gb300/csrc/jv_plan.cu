@@ -335,10 +335,8 @@ static bool build_tables(Plan *p, const std::vector<double> &roots) {
     for (long m = 0; m < 2 * MN; m++) tw[m] = (T)roots[m];
     Device *d = device();
     if (!d) return false;
-    p->d_tw = dmalloc(2 * n * sizeof(T));
+    p->d_tw = table_upload(tw.data(), 2 * n * sizeof(T), "twiddle upload");
     if (!p->d_tw) return false;
-    if (!cuda_ok(cudaMemcpy(p->d_tw, tw.data(), 2 * n * sizeof(T), cudaMemcpyHostToDevice), "twiddle upload"))
-        return false;
     // per-pass tables: the pass with radix R after radices of product Ns holds
     // exp(-2 pi i r m/(Ns R)) at r*Ns + m
     auto pass_tables = [&](const std::vector<int> &radices, void **dst) -> bool {
@@ -355,10 +353,8 @@ static bool build_tables(Plan *p, const std::vector<double> &roots) {
             Ns *= R;
         }
         if (tp.empty()) tp.assign(2, (T)0);
-        *dst = dmalloc(tp.size() * sizeof(T));
-        if (!*dst) return false;
-        return cuda_ok(cudaMemcpy(*dst, tp.data(), tp.size() * sizeof(T), cudaMemcpyHostToDevice),
-                       "pass twiddle upload");
+        *dst = table_upload(tp.data(), tp.size() * sizeof(T), "pass twiddle upload");
+        return *dst != nullptr;
     };
     if (p->smooth && !pass_tables(p->radix, &p->d_twg)) return false;
     if (p->smooth) {
@@ -372,11 +368,8 @@ static bool build_tables(Plan *p, const std::vector<double> &roots) {
             pc[i].mNs = magic_host(Ns);
             Ns *= (unsigned long)p->radix[i];
         }
-        p->d_pc = dmalloc(pc.size() * sizeof(PassConst));
+        p->d_pc = table_upload(pc.data(), pc.size() * sizeof(PassConst), "pass constants upload");
         if (!p->d_pc) return false;
-        if (!cuda_ok(cudaMemcpy(p->d_pc, pc.data(), pc.size() * sizeof(PassConst), cudaMemcpyHostToDevice),
-                     "pass constants upload"))
-            return false;
     }
     if (sizeof(T) == 4) {
         std::vector<int> fr = fast_radices(MN);
@@ -392,11 +385,8 @@ static bool build_tables(Plan *p, const std::vector<double> &roots) {
             th[2 * k] = (T)c;
             th[2 * k + 1] = (T)((p->type == JV_RCFFTOP) ? s : -s);
         }
-        p->d_thalf = dmalloc(2 * (n + 1) * sizeof(T));
+        p->d_thalf = table_upload(th.data(), 2 * (n + 1) * sizeof(T), "half-angle table upload");
         if (!p->d_thalf) return false;
-        if (!cuda_ok(cudaMemcpy(p->d_thalf, th.data(), 2 * (n + 1) * sizeof(T), cudaMemcpyHostToDevice),
-                     "half-angle table upload"))
-            return false;
     }
     return true;
 }
@@ -505,11 +495,9 @@ static bool build_long(Plan *p) {
         hi[2 * q] = (T)c;
         hi[2 * q + 1] = (T)s;
     }
-    lp->d_lo = dmalloc(lo.size() * sizeof(T));
-    lp->d_hi = dmalloc(hi.size() * sizeof(T));
-    if (!lp->d_lo || !lp->d_hi ||
-        !cuda_ok(cudaMemcpy(lp->d_lo, lo.data(), lo.size() * sizeof(T), cudaMemcpyHostToDevice), "twiddle upload") ||
-        !cuda_ok(cudaMemcpy(lp->d_hi, hi.data(), hi.size() * sizeof(T), cudaMemcpyHostToDevice), "twiddle upload")) {
+    lp->d_lo = table_upload(lo.data(), lo.size() * sizeof(T), "twiddle upload");
+    lp->d_hi = table_upload(hi.data(), hi.size() * sizeof(T), "twiddle upload");
+    if (!lp->d_lo || !lp->d_hi) {
         long_free(lp);
         return false;
     }
@@ -959,14 +947,8 @@ int jvsip_fftm_setform_d(vsip_fftm_d *vp, int form) {
                 }
             Ns *= R;
         }
-        void *d = dmalloc(tb.size() * sizeof(float));
-        if (!d) return E_ALLOC;
-        if (!cuda_ok(cudaMemcpy(d, tb.data(), tb.size() * sizeof(float), cudaMemcpyHostToDevice),
-                     "FP64-form twiddle upload")) {
-            dfree(d);
-            return E_CUDA;
-        }
-        p->d_twdd = d;
+        p->d_twdd = table_upload(tb.data(), tb.size() * sizeof(float), "FP64-form twiddle upload");
+        if (!p->d_twdd) return jvsip_gpu_last_error() ? jvsip_gpu_last_error() : E_ALLOC;
     }
     p->form = form;
     return 0;

@@ -444,17 +444,13 @@ static bool split_tables() {
             w16[2 * (c * 32 + bb)] = w[2 * (c * 32 + bb)] * 0.0625f;  // exact: a power of two
             w16[2 * (c * 32 + bb) + 1] = w[2 * (c * 32 + bb) + 1] * 0.0625f;
         }
-    g_bop[0] = dmalloc(SP_B_BYTES);
-    g_bop[1] = dmalloc(SP_B_BYTES);
-    g_tw[0] = dmalloc(w.size() * sizeof(float));
-    g_tw[1] = dmalloc(w.size() * sizeof(float));
-    g_status = (int *)dmalloc(sizeof(int));
-    if (!g_bop[0] || !g_bop[1] || !g_tw[0] || !g_tw[1] || !g_status) return false;
-    return cuda_ok(cudaMemcpy(g_bop[0], b16.data(), SP_B_BYTES, cudaMemcpyHostToDevice), "split tables") &&
-           cuda_ok(cudaMemcpy(g_bop[1], bbf.data(), SP_B_BYTES, cudaMemcpyHostToDevice), "split tables") &&
-           cuda_ok(cudaMemcpy(g_tw[0], w16.data(), w16.size() * sizeof(float), cudaMemcpyHostToDevice), "split tables") &&
-           cuda_ok(cudaMemcpy(g_tw[1], w.data(), w.size() * sizeof(float), cudaMemcpyHostToDevice), "split tables") &&
-           cuda_ok(cudaMemset(g_status, 0, sizeof(int)), "split status");
+    const int zero = 0;
+    if (!g_bop[0]) g_bop[0] = table_upload(b16.data(), SP_B_BYTES, "split tables");
+    if (!g_bop[1]) g_bop[1] = table_upload(bbf.data(), SP_B_BYTES, "split tables");
+    if (!g_tw[0]) g_tw[0] = table_upload(w16.data(), w16.size() * sizeof(float), "split tables");
+    if (!g_tw[1]) g_tw[1] = table_upload(w.data(), w.size() * sizeof(float), "split tables");
+    if (!g_status) g_status = (int *)table_upload(&zero, sizeof zero, "split status");
+    return g_bop[0] && g_bop[1] && g_tw[0] && g_tw[1] && g_status;
 }
 
 // true when the split form ran (or failed with an error recorded); false when
