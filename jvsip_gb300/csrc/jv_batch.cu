@@ -397,7 +397,9 @@ static bool build_tiles(size_t n, const vsip_fftm_f *const plans[], const vsip_c
         bool vf_out = labs(t.out_vs) == 1 && labs(t.out_es) != 1;
         t.vec_fast = (vf_in || vf_out) ? 1 : 0;
         t.ld = (int)tile_ld(N, t.vec_fast);
-        if (resident_long_columns_f(p, x, y)) {
+        // the plan's scratch is had now (nothing may allocate while a batch is
+        // recorded into its graph); without it the call goes in tiles
+        if (resident_long_columns_f(p, x, y) && enqueue_resident_c2c_f(p, x, y, nullptr, true)) {
             bb.steps.push_back(StepCall{p, x, y});
             bb.bytes += 16.0 * N * nv;
             continue;
@@ -481,11 +483,7 @@ struct DevBatch {
 };
 
 static bool upload(const BatchBuild &bb, DevBatch &db) {
-    // the step calls' plans get their scratch now (nothing may allocate while
-    // a batch is recorded into its graph)
     db.steps = bb.steps;
-    for (const StepCall &c : db.steps)
-        if (!enqueue_resident_c2c_f(c.p, c.x, c.y, nullptr, true)) return false;
     std::vector<TileDesc> all;
     for (int c = 0; c < kClasses; c++) {
         db.off[c] = (int)all.size();

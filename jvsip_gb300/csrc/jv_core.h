@@ -304,8 +304,9 @@ Plan *plan_of(const void *vsip_plan);   // ext_fftm_obj of a vsip_fftm_* (nullpt
 Plan *plan_of_v(const void *vsip_plan); // ext_fft_obj of a vsip_fft_* (nullptr if bad)
 // A single-precision c2c call on views of admitted interleaved blocks, enqueued
 // on `st` with no host synchronisation (the batching form's route for long
-// columns); with `prepare` only the plan's long-transform scratch is made
-// ready and nothing is launched.  False (error set) when it cannot run so.
+// columns).  False (error set) when it cannot run so.  With `prepare` nothing is
+// launched and only the plan's long-transform scratch is made ready: false, with
+// no error left, when there is no memory for it.
 bool enqueue_resident_c2c_f(Plan *p, const vsip_cmview_f *x, const vsip_cmview_f *y, cudaStream_t st, bool prepare);
 // true when such a call of plan p on these views runs as the long columns' two steps
 bool resident_long_columns_f(Plan *p, const vsip_cmview_f *x, const vsip_cmview_f *y);

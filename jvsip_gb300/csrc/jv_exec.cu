@@ -992,7 +992,7 @@ bool enqueue_resident_c2c_f(Plan *p, const vsip_cmview_f *x, const vsip_cmview_f
         set_error(E_ARG, "resident c2c call: views of admitted interleaved blocks expected");
         return false;
     }
-    if (prepare) return !j.lp || long_scratch(j.lp, long_scratch_need(j), false);
+    if (prepare) return !j.lp || long_scratch(j.lp, long_scratch_need(j), true);
     return run_job(j, st);
 }
 
