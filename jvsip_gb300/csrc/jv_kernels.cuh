@@ -216,36 +216,35 @@ template <> struct Dft<double2, 16> {
     static __device__ __forceinline__ void run(double2 *v) { dft16_fma<false>(v); }
 };
 
-// A pass's butterfly: element r times w[r*st], then the transform; `unit`: w = 1
-template <int R, typename C>
-__device__ __forceinline__ void tw_bfly(C *v, const C *__restrict__ w, int st, bool unit) {
-    if constexpr (sizeof(C) == 16 && (R == 2 || R == 4 || R == 8 || R == 16)) {
-        if (unit) {
+// A pass's butterfly in double precision, radix 2^k: element r times w[r*st],
+// then the transform; `unit`: w = 1
+template <int R> __device__ __forceinline__ void tw_bfly(double2 *v, const double2 *__restrict__ w, int st, bool unit) {
+    typedef double2 C;
+    if (unit) {
 #pragma unroll
-            for (int r = 0; r < R / 2; r++) {
-                const C a = v[r];
-                v[r] = cadd(a, v[r + R / 2]);
-                v[r + R / 2] = csub(a, v[r + R / 2]);
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < R / 2; r++) {
-                const C a = r ? cmul(v[r], __ldg(&w[r * st])) : v[0], b = v[r + R / 2], u = __ldg(&w[(r + R / 2) * st]);
-                v[r] = mk<C>(fma(-u.y, b.y, fma(u.x, b.x, a.x)), fma(u.y, b.x, fma(u.x, b.y, a.y)));
-                if constexpr (R == 16) v[r + R / 2] = mk<C>(fma(2.0, a.x, -v[r].x), fma(2.0, a.y, -v[r].y));
-                else v[r + R / 2] = mk<C>(fma(u.y, b.y, fma(-u.x, b.x, a.x)), fma(-u.y, b.x, fma(-u.x, b.y, a.y)));
-            }
+        for (int r = 0; r < R / 2; r++) {
+            const C a = v[r];
+            v[r] = cadd(a, v[r + R / 2]);
+            v[r + R / 2] = csub(a, v[r + R / 2]);
         }
-        if constexpr (R == 4) dft4_fma<true>(v[0], v[1], v[2], v[3]);
-        if constexpr (R == 8) dft8_fma<true>(v);
-        if constexpr (R == 16) dft16_fma<true>(v);
     } else {
-        if (!unit) {
 #pragma unroll
-            for (int r = 1; r < R; r++) v[r] = cmul(v[r], __ldg(&w[r * st]));
+        for (int r = 0; r < R / 2; r++) {
+            const C a = r ? cmul(v[r], __ldg(&w[r * st])) : v[0], b = v[r + R / 2], u = __ldg(&w[(r + R / 2) * st]);
+            v[r] = mk<C>(fma(-u.y, b.y, fma(u.x, b.x, a.x)), fma(u.y, b.x, fma(u.x, b.y, a.y)));
+            if constexpr (R == 16) v[r + R / 2] = mk<C>(fma(2.0, a.x, -v[r].x), fma(2.0, a.y, -v[r].y));
+            else v[r + R / 2] = mk<C>(fma(u.y, b.y, fma(-u.x, b.x, a.x)), fma(-u.y, b.x, fma(-u.x, b.y, a.y)));
         }
-        Dft<C, R>::run(v);
     }
+    if constexpr (R == 4) dft4_fma<true>(v[0], v[1], v[2], v[3]);
+    if constexpr (R == 8) dft8_fma<true>(v);
+    if constexpr (R == 16) dft16_fma<true>(v);
+}
+// Single precision multiplies in the passes themselves: through a common function
+// its c2c kernels spilled 72 and 84 bytes a thread instead of 16 and 56 (rows of
+// overlapping or strided views, 32 x 162: 8.2 us against 6.2).
+template <typename T, int R> constexpr bool tw_folds() {
+    return sizeof(T) == 8 && (R == 2 || R == 4 || R == 8 || R == 16);
 }
 
 template <typename C> struct Dft<C, 3> {
@@ -778,7 +777,15 @@ __device__ __forceinline__ void smem_pass(typename cplx_t<T>::t *s, int ld, int 
         if (b < nb) {
             int t = mdiv(b, mNR), j = b - t * NR;
             int m = (Ns == 1) ? 0 : j - Ns * mdiv(j, mNs);
-            tw_bfly<R>(v[k], tp + m, Ns, m == 0);
+            if constexpr (tw_folds<T, R>()) {
+                tw_bfly<R>(v[k], tp + m, Ns, m == 0);
+            } else {
+                if (m) {
+#pragma unroll
+                    for (int r = 1; r < R; r++) v[k][r] = cmul(v[k][r], __ldg(&tp[r * Ns + m]));
+                }
+                Dft<C, R>::run(v[k]);
+            }
             C *dst = s + t * ld;
             const int base = (j - m) * R + m;
 #pragma unroll
@@ -1009,7 +1016,15 @@ __device__ __forceinline__ void pass_last(const typename cplx_t<T>::t *s, int ld
         if (b < nb) {
             int t, j;
             tile_tj(b, io.vf_out, nt, io.mnt, NR, pc.y, t, j);
-            tw_bfly<R>(v[k], tp + j, Ns, j == 0);
+            if constexpr (tw_folds<T, R>()) {
+                tw_bfly<R>(v[k], tp + j, Ns, j == 0);
+            } else {
+                if (j) {
+#pragma unroll
+                    for (int r = 1; r < R; r++) v[k][r] = cmul(v[k][r], __ldg(&tp[r * Ns + j]));
+                }
+                Dft<C, R>::run(v[k]);
+            }
             if (io.tw_lo) {
                 // output element j + r*Ns of transform t: times W^(g*(j + r*Ns))
                 const unsigned tg = io.tw_t0 + (unsigned)t * io.tw_ts;
