@@ -418,10 +418,10 @@ template <typename T> static void dif_fill(DifArgs<T> &a, const DifTab &t) {
 constexpr long kColWidePts = 5L << 23;
 
 // The kernel's arguments for a call and its CTA: tuned > 0 asks for that many
-// transforms (a power of two for column tiles).  False when the call does not
-// qualify.
+// transforms (a power of two for column tiles); `alone`: nothing else fills the
+// SMs that the call's tiles leave idle.  False when the call does not qualify.
 template <typename T>
-static bool dif_args(const Job &j, long tuned, DifArgs<T> &a, DifCta &cta) {
+static bool dif_args(const Job &j, long tuned, bool alone, DifArgs<T> &a, DifCta &cta) {
     typedef typename cplx_t<T>::t C;
     const DifTab *t = j.dif;
     if (!t || j.no_fast || j.no_dif || j.nvec <= 0 || j.gram || j.taper_n) return false;
@@ -526,8 +526,17 @@ static bool dif_args(const Job &j, long tuned, DifArgs<T> &a, DifCta &cta) {
         if (((j.nvec - 1) >> a.lgv) + 1 < device()->sms && j.nbatch <= 1) a.lgv = std::min(a.lgv, 2);
         if (tuned > 0) a.lgv = dif_col_tuned(tuned, j.nvec);
         while (a.lgv > 0 && ((size_t)a.LD << a.lgv) * sizeof(C) > cap) a.lgv--;
+        // down to one column where SMs would be idle and no compiled-in kernel
+        // takes the tile: a tile's time is its chain of loads and passes then (us,
+        // narrow against 4 to a tile: split columns 7000 x 16 16.7 and 26.4, 5000 x 2
+        // 6.8 and 14.8, 3000 x 150 12.9 and 15.2, 7000 x 300 25.8 in twos, 34.8 in
+        // fours and 46.7 in ones, two waves; 13312 x 100 24.8 and 35.3.  Compiled in,
+        // fours stay: 1000 x 16 3.8 and 4.5 in ones)
+        const bool fixed = sizeof(T) == 4 && !split && t->fix &&
+                           ((t->fix->cols && (1 << a.lgv) == t->fix->vcol) || (t->fix->cols4 && a.lgv == 2));
+        if (alone && !fixed) a.lgv = dif_col_narrow(a.lgv, j.nvec, device()->sms);
         vpb = 1L << a.lgv;
-        nthr = dif_col_threads(j.N, a.lgv, sizeof(T) == 4);
+        nthr = dif_col_threads(j.N, a.lgv, sizeof(T) == 4, alone && ((j.nvec - 1) >> a.lgv) < device()->sms);
     }
     a.vpb = (int)vpb;
     cta.nthr = (int)nthr;
@@ -541,7 +550,7 @@ template <typename T>
 static bool launch_dif_t(const Job &j, cudaStream_t st) {
     DifArgs<T> a;
     DifCta c;
-    if (j.nbatch > 1 || j.tw_lo || !dif_args<T>(j, 0, a, c)) return false;
+    if (j.nbatch > 1 || j.tw_lo || !dif_args<T>(j, 0, true, a, c)) return false;
     if constexpr (sizeof(T) == 4) {
         const DifFixEntry *f = j.dif->fix;
         if (f && !c.split && c.rows && f->rows) return f->rows(a, c.smem, st, 1);
@@ -563,7 +572,7 @@ static bool launch_dif_t(const Job &j, cudaStream_t st) {
 bool launch_dif_step_f32(const Job &j, cudaStream_t st) {
     DifArgs<float> a;
     DifCta c;
-    if (j.kind != K_C2C || j.nbatch < 1 || j.nbatch > 65535 || !dif_args<float>(j, 0, a, c) || c.rows || c.split)
+    if (j.kind != K_C2C || j.nbatch < 1 || j.nbatch > 65535 || !dif_args<float>(j, 0, false, a, c) || c.rows || c.split)
         return false;
     a.bvs_in = j.bvs_in;
     a.bvs_out = j.bvs_out;
@@ -632,7 +641,7 @@ bool launch_dif_komega_power_f32(const Job &j, cudaStream_t st) {
     q.gram = nullptr;
     DifArgs<float> a;
     DifCta c;
-    if (j.kind != K_C2C || !dif_args<float>(q, 0, a, c) || !c.rows || c.split) return false;
+    if (j.kind != K_C2C || !dif_args<float>(q, 0, true, a, c) || !c.rows || c.split) return false;
     a.gram = (float *)j.gram;
     a.g_es = j.gram_es;
     a.g_vs = j.gram_vs;
@@ -801,7 +810,7 @@ bool launch_vec_f32(const VecPlan &v, const float2 *in, float2 *out, float2 *scr
 }
 
 bool dif_tile_args(const Job &j, long tuned, DifArgs<float> &a, DifCta &c) {
-    return j.kind == K_C2C && dif_args<float>(j, tuned, a, c) && !c.split;
+    return j.kind == K_C2C && dif_args<float>(j, tuned, false, a, c) && !c.split;
 }
 
 bool launch_dif_f32(const Job &j, cudaStream_t st) { return launch_dif_t<float>(j, st); }

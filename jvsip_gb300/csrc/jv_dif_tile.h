@@ -19,12 +19,20 @@ inline int dif_col_tuned(long tuned, long nvec) {
     return lgv;
 }
 
-// threads of a tile of 2^lgv transforms of N points: about 16 points each, 64 to
-// 512, and 1024 for single-precision tiles above 16384 points
-inline long dif_col_threads(long N, int lgv, bool f32) {
-    const long V = 1L << lgv, unit = V < 32 ? 32 : V;
-    const long most = f32 && V * N > 16384 ? 1024 : 512;
-    const long want = V * N / 16 < 64 ? 64 : V * N / 16;
+// log2 of the transforms per tile, from lgv down, while twice as many tiles still
+// have an SM each
+inline int dif_col_narrow(int lgv, long nvec, long sms) {
+    while (lgv > 0 && 2 * (((nvec - 1) >> lgv) + 1) <= sms) lgv--;
+    return lgv;
+}
+
+// threads of a tile of 2^lgv transforms of N points: about 16 points each (8 where
+// every tile has an SM to itself: `few`), 64 to 512, and 1024 for single-precision
+// tiles that ask for that many
+inline long dif_col_threads(long N, int lgv, bool f32, bool few) {
+    const long V = 1L << lgv, unit = V < 32 ? 32 : V, pts = few ? 8 : 16;
+    const long most = f32 && (few || V * N > 16384) ? 1024 : 512;
+    const long want = V * N / pts < 64 ? 64 : V * N / pts;
     const long n = (want + unit - 1) / unit * unit;
     return n < most ? n : most;
 }

@@ -19,13 +19,15 @@ def tile(tmp_path_factory):
     d = tmp_path_factory.mktemp("tile")
     (d / "t.cpp").write_text('#include "jv_dif_tile.h"\nusing namespace jv;\nextern "C" {\n'
                              "int tuned(long t, long nvec) { return dif_col_tuned(t, nvec); }\n"
-                             "long threads(long N, int lgv, int f32) { return dif_col_threads(N, lgv, f32 != 0); }\n"
+                             "long threads(long N, int lgv, int f32, int few) { return dif_col_threads(N, lgv, f32 != 0, few != 0); }\n"
+                             "int narrow(int lgv, long nvec, long sms) { return dif_col_narrow(lgv, nvec, sms); }\n"
                              "int batch(int nthr) { return dif_batch_threads(nthr); }\n}\n")
     so = str(d / "t.so")
     subprocess.check_call(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, str(d / "t.cpp"), "-o", so])
     lib = C.CDLL(so)
     lib.tuned.argtypes = [C.c_long, C.c_long]
-    lib.threads.argtypes, lib.threads.restype = [C.c_long, C.c_int, C.c_int], C.c_long
+    lib.narrow.argtypes = [C.c_int, C.c_long, C.c_long]
+    lib.threads.argtypes, lib.threads.restype = [C.c_long, C.c_int, C.c_int, C.c_int], C.c_long
     return lib
 
 
@@ -44,7 +46,8 @@ def runs_every_butterfly_once(nthr, V, nb):
 
 
 @pytest.mark.parametrize("f32", [0, 1])
-def test_every_length_and_tuned_tile(tile, f32):
+@pytest.mark.parametrize("few", [0, 1])
+def test_every_length_and_tuned_tile(tile, f32, few):
     for N in list(range(4, 65)) + [100, 256, 1000, 1024, 2187, 4096, 16384]:
         for tuned in [1 << k for k in range(15)] + [3, 100, 1 << 40, (1 << 63) - 1]:
             for nvec in (2, 5, 64, 1 << 20):
@@ -52,16 +55,24 @@ def test_every_length_and_tuned_tile(tile, f32):
                 assert 0 <= lgv <= 9 and (lgv == 0 or (1 << lgv) <= tuned)
                 while lgv > 0 and (N << lgv) > SMEM:
                     lgv -= 1
-                V, n = 1 << lgv, tile.threads(N, lgv, f32)
+                V, n = 1 << lgv, tile.threads(N, lgv, f32, few)
                 assert 64 <= n <= (1024 if f32 else 512) and n >= V and n % V == 0 and n % 32 == 0, (N, tuned, n)
                 m = tile.batch(n)
                 assert m <= 1024 and m % 64 == 0 and m % V == 0, (N, tuned, n, m)
 
 
+def test_few_columns_are_spread_over_the_sms(tile):
+    for nvec in range(2, 1300):
+        for lgv in range(5):
+            n = tile.narrow(lgv, nvec, 152)
+            tiles = [-(-nvec >> k) for k in range(lgv + 1)]
+            assert n == lgv if 2 * tiles[lgv] > 152 else tiles[n] <= 152 and (n == 0 or 2 * tiles[n] > 152), (nvec, lgv)
+
+
 @pytest.mark.parametrize("N,tuned", [(8, 128), (12, 256), (16, 1024), (20, 256), (24, 128), (36, 256), (64, 256)])
 def test_tiles_of_short_lengths_run_each_butterfly_once(tile, N, tuned):
     lgv = tile.tuned(tuned, 1 << 20)
-    V, n = 1 << lgv, tile.threads(N, lgv, 1)
+    V, n = 1 << lgv, tile.threads(N, lgv, 1, 0)
     for R in (2, 3, 4):
         if N % R == 0:
             assert runs_every_butterfly_once(n, V, N // R)
