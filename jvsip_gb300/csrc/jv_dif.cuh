@@ -213,7 +213,7 @@ __device__ __forceinline__ void dif_first(const DifArgs<T> &a, typename cplx_t<T
         }
 #pragma unroll
         for (int r = 0; r < R; r++) v[r].y = flip_sign(v[r].y, a.smask_in);
-        Dft<C, R>::run(v);
+        DftF<C, R>::run(v);
         const C *w = a.tw + j;
 #pragma unroll
         for (int r = 1; r < R; r++) v[r] = cmul(v[r], __ldg(w + r * S));
@@ -246,7 +246,7 @@ __device__ __forceinline__ void dif_mid(const DifArgs<T> &a, const PD &p, typena
         C v[R];
 #pragma unroll
         for (int r = 0; r < R; r++) v[r] = d[r * sp];
-        Dft<C, R>::run(v);
+        DftF<C, R>::run(v);
         const C *w = a.tw + (p.two + n);
 #pragma unroll
         for (int r = 1; r < R; r++) v[r] = cmul(v[r], __ldg(w + r * S));
@@ -279,7 +279,7 @@ __device__ __forceinline__ void dif_last(const DifArgs<T> &a, const typename cpl
         C v[R];
 #pragma unroll
         for (int r = 0; r < R; r++) v[r] = COLS ? d[r * V] : d[r];
-        Dft<C, R>::run(v);
+        DftF<C, R>::run(v);
         long e0 = (v0 + t) * a.vs_out + (TF ? (long)q * a.es_out : (long)q);
         const long st = TF ? (long)Q * a.es_out : (long)Q;
         if constexpr (dif_groups<KIND>()) e0 += blockIdx.y * a.bvs_out;
@@ -352,7 +352,7 @@ __device__ __forceinline__ void dif_first_c2r(const DifArgs<T> &a, typename cplx
             w[R - 1 - r] = mk<C>(f.x + g.x - c.y * d.x + c.x * d.y, -(g.y - f.y - c.y * d.y - c.x * d.x));
         }
         C *d = s + (t * a.LD + j);
-        Dft<C, R>::run(u);
+        DftF<C, R>::run(u);
         const C *tu = a.tw + j;
 #pragma unroll
         for (int r = 1; r < R; r++) u[r] = cmul(u[r], __ldg(tu + r * S));
@@ -360,7 +360,7 @@ __device__ __forceinline__ void dif_first_c2r(const DifArgs<T> &a, typename cplx
         for (int r = 0; r < R; r++) d[r * P1] = u[r];
         if (j != 0 && 2 * j != S) {
             d += S - 2 * j;
-            Dft<C, R>::run(w);
+            DftF<C, R>::run(w);
             const C *tw = a.tw + (S - j);
 #pragma unroll
             for (int r = 1; r < R; r++) w[r] = cmul(w[r], __ldg(tw + r * S));
@@ -395,8 +395,8 @@ __device__ __forceinline__ void dif_last_r2c(const DifArgs<T> &a, const typename
         for (int r = 0; r < R; r++) u[r] = su[r];
 #pragma unroll
         for (int r = 0; r < R; r++) w[r] = sw[r];
-        Dft<C, R>::run(u);
-        Dft<C, R>::run(w);
+        DftF<C, R>::run(u);
+        DftF<C, R>::run(w);
         if (a.has_scale) {
 #pragma unroll
             for (int r = 0; r < R; r++) {

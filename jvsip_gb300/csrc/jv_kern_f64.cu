@@ -5,8 +5,15 @@
 #include "jv_launch.cuh"
 
 namespace jv {
+bool launch_smem_fold_f64(const Job &j, cudaStream_t s);
+static bool radices_2k(const Job &j) {
+    for (int i = 0; i < j.npass; i++)
+        if (j.radix[i] & (j.radix[i] - 1)) return false;
+    return j.npass > 0;
+}
 bool launch_smem_f64(const Job &j, cudaStream_t s) {
     if (j.kind == K_C2C && j.cin.cst == 1 && j.cout.cst == 1) return launch_smem_split_f64(j, s);
+    if (j.kind == K_C2C && radices_2k(j)) return launch_smem_fold_f64(j, s);
     if (j.kind == K_C2C) return launch_smem_t<double, K_C2C>(j, s);
     return launch_smem_real_f64(j, s);
 }

@@ -132,12 +132,10 @@ template <typename C> struct Dft<C, 16> {
 // multiply-adds; cos(pi/8) + i sin(pi/8) is cos(pi/8) (1 + i t), t = tan(pi/8),
 // whose cosine waits for the next additions: 144 instructions for 16 points (160
 // with products), 52 for 8 (56).  With twiddles (tw_bfly) the first level is
-// a +- w b in two multiply-adds per component, which saves a rounding; at 16
-// points, which have precision to spare, a - w b is 2 a - (a + w b): 188
-// instructions with all twiddles (220): rows 16384 x 4096 4921 -> 4664 us,
-// 32.5 instead of 37.5 instructions per point.  Relative L2 error, mean of 8 inputs:
-// 2.18e-16 against 2.24e-16 with products on 4096 points (twiddles and 2 a - s on
-// every level, 192 instructions: 2.46e-16).
+// a +- w b in two multiply-adds per component, which saves a rounding: 204 for 16
+// points (220), 80 for 8 (84), in every lane.  Rows 16384 x 4096 4493 us
+// (34.5 instructions per point; 4921 with products, 37.5), 65536 x 64 146 (154).
+// Relative L2 error, mean of 8 inputs of 4096 points: 2.57e-16 against 2.63e-16 with products.
 //
 // PAIRED: the first level is done, v[r] = a_r + b_r and v[r + R/2] = a_r - b_r.
 template <bool PAIRED> __device__ __forceinline__ void dft4_fma(double2 &v0, double2 &v1, double2 &v2, double2 &v3) {
@@ -209,44 +207,38 @@ template <bool PAIRED> __device__ __forceinline__ void dft16_fma(double2 *v) {
                   mk<double2>(fma(t, x.x, x.y), fma(t, x.y, -x.x)), mk<double2>(fma(-t, y.y, -y.x), fma(t, y.x, -y.y)));
     }
 }
-template <> struct Dft<double2, 8> {
+template <typename C, int R> struct DftF : Dft<C, R> {};
+template <> struct DftF<double2, 8> {
     static __device__ __forceinline__ void run(double2 *v) { dft8_fma<false>(v); }
 };
-template <> struct Dft<double2, 16> {
+template <> struct DftF<double2, 16> {
     static __device__ __forceinline__ void run(double2 *v) { dft16_fma<false>(v); }
 };
 
 // A pass's butterfly in double precision, radix 2^k: element r times w[r*st],
-// then the transform; `unit`: w = 1
+// then the transform.  `unit` lanes (m = 0, every w is 1) take the same
+// instructions as the others, since the FP64 pipe is as busy for one lane as for
+// 32 and short rows have such a lane in every warp: they only get 0 in place of
+// the component that w's zero imaginary part multiplies, as 0 times an infinity
+// would not be 0.
 template <int R> __device__ __forceinline__ void tw_bfly(double2 *v, const double2 *__restrict__ w, int st, bool unit) {
     typedef double2 C;
-    if (unit) {
+    auto cross = [&](C a) { return unit ? mk<C>(0.0, 0.0) : a; };
 #pragma unroll
-        for (int r = 0; r < R / 2; r++) {
-            const C a = v[r];
-            v[r] = cadd(a, v[r + R / 2]);
-            v[r + R / 2] = csub(a, v[r + R / 2]);
+    for (int r = 0; r < R / 2; r++) {
+        C a = v[r];
+        if (r) {
+            const C u = __ldg(&w[r * st]), x = cross(a);
+            a = mk<C>(fma(-u.y, x.y, u.x * a.x), fma(u.y, x.x, u.x * a.y));
         }
-    } else {
-#pragma unroll
-        for (int r = 0; r < R / 2; r++) {
-            const C a = r ? cmul(v[r], __ldg(&w[r * st])) : v[0], b = v[r + R / 2], u = __ldg(&w[(r + R / 2) * st]);
-            v[r] = mk<C>(fma(-u.y, b.y, fma(u.x, b.x, a.x)), fma(u.y, b.x, fma(u.x, b.y, a.y)));
-            if constexpr (R == 16) v[r + R / 2] = mk<C>(fma(2.0, a.x, -v[r].x), fma(2.0, a.y, -v[r].y));
-            else v[r + R / 2] = mk<C>(fma(u.y, b.y, fma(-u.x, b.x, a.x)), fma(-u.y, b.x, fma(-u.x, b.y, a.y)));
-        }
+        const C b = v[r + R / 2], u = __ldg(&w[(r + R / 2) * st]), x = cross(b);
+        v[r] = mk<C>(fma(-u.y, x.y, fma(u.x, b.x, a.x)), fma(u.y, x.x, fma(u.x, b.y, a.y)));
+        v[r + R / 2] = mk<C>(fma(u.y, x.y, fma(-u.x, b.x, a.x)), fma(-u.y, x.x, fma(-u.x, b.y, a.y)));
     }
     if constexpr (R == 4) dft4_fma<true>(v[0], v[1], v[2], v[3]);
     if constexpr (R == 8) dft8_fma<true>(v);
     if constexpr (R == 16) dft16_fma<true>(v);
 }
-// Single precision multiplies in the passes themselves: through a common function
-// its c2c kernels spilled 72 and 84 bytes a thread instead of 16 and 56 (rows of
-// overlapping or strided views, 32 x 162: 8.2 us against 6.2).
-template <typename T, int R> constexpr bool tw_folds() {
-    return sizeof(T) == 8 && (R == 2 || R == 4 || R == 8 || R == 16);
-}
-
 template <typename C> struct Dft<C, 3> {
     static __device__ __forceinline__ void run(C *v) {
         typedef decltype(C::x) T;
@@ -737,12 +729,18 @@ template <typename T> struct SmemArgs {
 // pass needs ceil(EMAX/R) * blockDim >= transforms * N/R.
 __device__ __forceinline__ int spad(int i) { return i + (i >> 4); }
 
+// FX flags of the passes
+constexpr int FX_TAPER = 1;  // first pass: taper the loaded real pairs, optionally write them back
+constexpr int FX_POWER = 2;  // last pass: store (s|X|^2, Im X), gram += s|X|^2
+constexpr int FX_SPLIT = 4;  // split complex views: real and imaginary parts in separate arrays
+constexpr int FX_FOLD = 8;   // double precision, radices 2^k only: twiddles and constants folded (tw_bfly)
+
 // pass counts per codelet (order of kRadixList), 4 bits each
 __host__ __device__ __forceinline__ int pass_count(unsigned long long packed, int i) {
     return (int)((packed >> (4 * i)) & 15ull);
 }
 
-template <typename T, int R, int EMAX, int IN = 0>
+template <typename T, int R, int EMAX, int IN = 0, int FX = 0>
 __device__ __forceinline__ void smem_pass(typename cplx_t<T>::t *s, int ld, int nt, int Ns,
                                           const typename cplx_t<T>::t *__restrict__ tp, const uint4 pc, int dp = 0) {
     // IN: where the pass reads -- 0 the padded rows; 1 dense rows (t*ld + n);
@@ -753,6 +751,7 @@ __device__ __forceinline__ void smem_pass(typename cplx_t<T>::t *s, int ld, int 
     // threads of a warp (consecutive m) read consecutive entries; pc: NR = N/R,
     // the multiply-high magic numbers of NR and Ns
     typedef typename cplx_t<T>::t C;
+    if constexpr ((FX & FX_FOLD) != 0 && (R & (R - 1)) != 0) return;
     constexpr int K = pass_k(EMAX, R);
     const int NR = (int)pc.x;
     const int nb = nt * NR;
@@ -777,7 +776,7 @@ __device__ __forceinline__ void smem_pass(typename cplx_t<T>::t *s, int ld, int 
         if (b < nb) {
             int t = mdiv(b, mNR), j = b - t * NR;
             int m = (Ns == 1) ? 0 : j - Ns * mdiv(j, mNs);
-            if constexpr (tw_folds<T, R>()) {
+            if constexpr ((FX & FX_FOLD) != 0) {
                 tw_bfly<R>(v[k], tp + m, Ns, m == 0);
             } else {
                 if (m) {
@@ -799,18 +798,18 @@ __device__ __forceinline__ void smem_pass(typename cplx_t<T>::t *s, int ld, int 
 // kRadixList (the order of the plan's per-pass twiddle tables twg and pass
 // constants pc).  One loop per codelet keeps the codelets' register lifetimes
 // apart.
-template <typename T, int EMAX>
+template <typename T, int EMAX, int FX = 0>
 __device__ __forceinline__ void smem_passes_from(typename cplx_t<T>::t *s, int ld, int nt, unsigned long long packed,
                                                  const typename cplx_t<T>::t *__restrict__ &tp,
                                                  const uint4 *__restrict__ pc, int &Ns, int &p);
 
-template <typename T, int EMAX>
+template <typename T, int EMAX, int FX = 0>
 __device__ __forceinline__ void smem_passes(typename cplx_t<T>::t *s, int ld, int nt, unsigned long long packed,
                                             const typename cplx_t<T>::t *__restrict__ twg,
                                             const uint4 *__restrict__ pc) {
     int Ns = 1, p = 0;
     const typename cplx_t<T>::t *tp = twg;
-    smem_passes_from<T, EMAX>(s, ld, nt, packed, tp, pc, Ns, p);
+    smem_passes_from<T, EMAX, FX>(s, ld, nt, packed, tp, pc, Ns, p);
 }
 
 // ---------------------------------------------------------------- fused first / last passes (c2c)
@@ -874,10 +873,6 @@ template <typename T> struct TileIO {
     T *out_re, *out_im;
 };
 
-// FX flags of the fused passes
-constexpr int FX_TAPER = 1;  // first pass: taper the loaded real pairs, optionally write them back
-constexpr int FX_POWER = 2;  // last pass: store (s|X|^2, Im X), gram += s|X|^2
-constexpr int FX_SPLIT = 4;  // split complex views: real and imaginary parts in separate arrays
 
 template <int FX, typename C, typename T>
 __device__ __forceinline__ C io_load(const TileIO<T> &io, const C *src, long e) {
@@ -940,6 +935,7 @@ template <typename T, int R, int EMAX, bool LAST, int FX = 0>
 __device__ __forceinline__ void pass_first(typename cplx_t<T>::t *s, int ld, int nt, const uint4 pc,
                                            const TileIO<T> &io) {
     typedef typename cplx_t<T>::t C;
+    if constexpr ((FX & FX_FOLD) != 0 && (R & (R - 1)) != 0) return;
     constexpr int K = pass_k(EMAX, R);
     const int NR = (int)pc.x, nb = nt * NR;
     const int tid = threadIdx.x, nthr = blockDim.x;
@@ -970,7 +966,8 @@ __device__ __forceinline__ void pass_first(typename cplx_t<T>::t *s, int ld, int
         if (b < nb) {
             int t, j;
             tile_tj(b, io.vf, nt, io.mnt, NR, pc.y, t, j);
-            Dft<C, R>::run(v[k]);
+            if constexpr ((FX & FX_FOLD) != 0) DftF<C, R>::run(v[k]);
+            else Dft<C, R>::run(v[k]);
             if (LAST) {
                 // one pass: N = R, j = 0, output element r
 #pragma unroll
@@ -995,6 +992,7 @@ __device__ __forceinline__ void pass_last(const typename cplx_t<T>::t *s, int ld
                                           const typename cplx_t<T>::t *__restrict__ tp, const uint4 pc,
                                           const TileIO<T> &io) {
     typedef typename cplx_t<T>::t C;
+    if constexpr ((FX & FX_FOLD) != 0 && (R & (R - 1)) != 0) return;
     constexpr int K = pass_k(EMAX, R);
     const int NR = (int)pc.x, nb = nt * NR;
     const int tid = threadIdx.x, nthr = blockDim.x;
@@ -1016,7 +1014,7 @@ __device__ __forceinline__ void pass_last(const typename cplx_t<T>::t *s, int ld
         if (b < nb) {
             int t, j;
             tile_tj(b, io.vf_out, nt, io.mnt, NR, pc.y, t, j);
-            if constexpr (tw_folds<T, R>()) {
+            if constexpr ((FX & FX_FOLD) != 0) {
                 tw_bfly<R>(v[k], tp + j, Ns, j == 0);
             } else {
                 if (j) {
@@ -1101,7 +1099,7 @@ __device__ __forceinline__ void tile_passes(typename cplx_t<T>::t *s, int ld, in
         np--;
     }
     if (TOG && np > 0) mid -= 1ull << (4 * li);
-    smem_passes_from<T, EMAX>(s, ld, nt, mid, tp, pc, Ns, p);
+    smem_passes_from<T, EMAX, FX>(s, ld, nt, mid, tp, pc, Ns, p);
     if (TOG && np > 0) {
         const uint4 pcl = __ldg(&pc[p]);
 #define JV_LAST(R) pass_last<T, R, EMAX, FX>(s, ld, nt, Ns, tp, pcl, io)
@@ -1133,13 +1131,13 @@ __device__ __forceinline__ void staged_tile(typename cplx_t<T>::t *s, int ld, in
         }
     const uint4 pc0 = __ldg(&pc[0]);
     int Rf = 2;
-#define JV_STAGED_FIRST(R) (smem_pass<T, R, EMAX, 2>(s, ld, nt, 1, twg, pc0, dp), Rf = R)
+#define JV_STAGED_FIRST(R) (smem_pass<T, R, EMAX, 2, FX>(s, ld, nt, 1, twg, pc0, dp), Rf = R)
     JV_RADIX_SWITCH(fi, JV_STAGED_FIRST)
 #undef JV_STAGED_FIRST
     int Ns = Rf, p = 1;
     const C *tp = twg + Rf;
     const unsigned long long mid = packed - (1ull << (4 * fi)) - (1ull << (4 * li));
-    smem_passes_from<T, EMAX>(s, ld, nt, mid, tp, pc, Ns, p);
+    smem_passes_from<T, EMAX, FX>(s, ld, nt, mid, tp, pc, Ns, p);
     const uint4 pcl = __ldg(&pc[p]);
 #define JV_LAST(R) pass_last<T, R, EMAX, FX>(s, ld, nt, Ns, tp, pcl, io)
     JV_RADIX_SWITCH(li, JV_LAST)
@@ -1147,13 +1145,13 @@ __device__ __forceinline__ void staged_tile(typename cplx_t<T>::t *s, int ld, in
 }
 
 // smem_passes starting from pass p with Ns and the table pointer tp (updated)
-template <typename T, int EMAX>
+template <typename T, int EMAX, int FX>
 __device__ __forceinline__ void smem_passes_from(typename cplx_t<T>::t *s, int ld, int nt, unsigned long long packed,
                                                  const typename cplx_t<T>::t *__restrict__ &tp,
                                                  const uint4 *__restrict__ pc, int &Ns, int &p) {
 #define JV_PASS_LOOP(I, R)                                                  \
     for (int q = pass_count(packed, I); q > 0; q--, p++) {                  \
-        smem_pass<T, R, EMAX>(s, ld, nt, Ns, tp, __ldg(&pc[p]));            \
+        smem_pass<T, R, EMAX, 0, FX>(s, ld, nt, Ns, tp, __ldg(&pc[p]));     \
         tp += R * Ns;                                                       \
         Ns *= R;                                                            \
     }
@@ -1220,17 +1218,19 @@ __device__ __forceinline__ void tile_load(Walk &w, bool vf, int tot, C *s, int l
 }
 
 // Instances of the shared-memory kernel beyond the three transform kinds:
-// the k-omega pipeline's tapered R2C rows and power-accumulating c2c columns.
-constexpr int KX_R2C_TAPER = 3, KX_C2C_POWER = 4, KX_C2C_SPLIT = 5;
+// the k-omega pipeline's tapered R2C rows and power-accumulating c2c columns,
+// split complex views, schedules of radices 2^k in double precision.
+constexpr int KX_R2C_TAPER = 3, KX_C2C_POWER = 4, KX_C2C_SPLIT = 5, KX_C2C_FOLD = 6;
 
 template <typename T, int KIND0, int EMAX, int MAXT>
 __global__ void __launch_bounds__(MAXT) k_smem(const __grid_constant__ SmemArgs<T> a) {
     typedef typename cplx_t<T>::t C;
     constexpr int KIND =
-        KIND0 == KX_R2C_TAPER ? K_R2C : (KIND0 == KX_C2C_POWER || KIND0 == KX_C2C_SPLIT) ? K_C2C : KIND0;
+        KIND0 == KX_R2C_TAPER ? K_R2C : KIND0 >= KX_C2C_POWER ? K_C2C : KIND0;
     constexpr int FX = KIND0 == KX_R2C_TAPER   ? FX_TAPER
                        : KIND0 == KX_C2C_POWER ? FX_POWER
                        : KIND0 == KX_C2C_SPLIT ? FX_SPLIT
+                       : KIND0 == KX_C2C_FOLD  ? FX_FOLD
                                                : 0;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     C *s = reinterpret_cast<C *>(smem_raw);
@@ -1415,7 +1415,7 @@ __global__ void __launch_bounds__(MAXT) k_smem(const __grid_constant__ SmemArgs<
             return;
         }
         // ---------------- radix passes
-        smem_passes<T, EMAX>(s, ld, nt, a.passes, a.twg, a.pc);
+        smem_passes<T, EMAX, FX>(s, ld, nt, a.passes, a.twg, a.pc);
         }
         // ---------------- store phase
         if (KIND == K_C2C) {
