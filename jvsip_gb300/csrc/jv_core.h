@@ -216,8 +216,9 @@ struct DifTab {
 };
 std::vector<double> unit_roots(long N);  // exp(-2 pi i m/N), m < N, (re, im) pairs
 // nullptr: no schedule for N (or no memory).  roots: unit_roots(N) when the caller has them;
-// other: double precision, the shared-memory kernel's schedule to be better than (or null)
-const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots, const std::vector<int> *other);
+// other: double precision, the shared-memory kernel's schedule to be better than on nvec rows (or null)
+const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots, const std::vector<int> *other,
+                          long nvec);
 void dif_release(const DifTab *t);
 bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1);
 bool launch_dif_f32(const Job &j, cudaStream_t s);  // false when the call does not qualify

@@ -219,6 +219,94 @@ static void *upload_tables(const std::vector<int> &rad, long N, const std::vecto
     return table_upload(tw.data(), tw.size() * sizeof(T), "twiddle upload");
 }
 
+// Double precision: an FP64 instruction takes the pipe as long for one lane of a
+// warp as for 32 and the pipe serves an SM's tiles one after another, so a call's
+// time is the tiles of the fullest SM times the FP64 instructions of a tile's warps
+// (of four warps at a time where an SM has one tile: its four quarters have a pipe
+// each).  Within 5 % of the times of 1751 calls, 4-8192 points, 1 to 2^23 / N rows,
+// at 0.30 ns per instruction and lane.
+static double f64_work(const int *rad, int np, long N, long v, bool smem, int lanes) {
+    double c = 0;
+    for (int i = 0; i < np; i++) {
+        const int R = rad[i];
+        // constants folded into 52 and 144 instructions here, products there
+        double per = R == 16 && !smem ? 9.0 : R == 8 && !smem ? 6.5 : kDifCost[R];
+        if (smem ? i > 0 : i + 1 < np) per += 4.0 * (R - 1) / R;  // the twiddles of a pass
+        c += (double)((v * (N / R) + lanes - 1) / lanes * lanes) * per * R;
+    }
+    return c;
+}
+static double f64_time(const int *rad, int np, long N, long v, long nvec, bool smem) {
+    const long tiles = (nvec + v - 1) / v, k = (tiles + device()->sms - 1) / device()->sms;
+    return (double)k * f64_work(rad, np, N, v, smem, k > 1 ? 32 : 128);
+}
+
+// Transforms per tile of a double-precision row call: of the least time, in up to
+// 72 KB (three CTAs per SM), the fewest where an SM has few tiles (a tile's chain of
+// passes is shorter) and the most where it has many (381300 x 22: 16 to a tile 646
+// us, 64 to a tile 355).
+static long f64_rows_per_tile(const DifTab &t, long nvec, double *time) {
+    static const long cand[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
+    const int np = (int)t.radix.size();
+    const long ldb = t.radix[0] * t.P1 * 16;
+    double best = 1e300, e[12];
+    int n = 0;
+    for (; n < 12 && (n == 0 || cand[n] * ldb <= 72 * 1024); n++) {
+        e[n] = f64_time(t.radix.data(), np, t.N, cand[n], nvec, false);
+        best = std::min(best, e[n]);
+    }
+    int lo = 0, hi = n - 1;
+    while (e[lo] > 1.01 * best) lo++;
+    while (e[hi] > 1.01 * best) hi--;
+    const int pick = nvec >= 4 * cand[hi] * device()->sms ? hi : lo;
+    *time = e[pick];
+    return cand[pick];
+}
+
+// Whether nvec rows run on this kernel rather than the shared-memory kernel, whose
+// schedule is rad and which takes 1024 points to a CTA: by the times above, with
+// 8 % in hand (us, shared-memory kernel and this one: 2^24 points of 100 1114 and
+// 867, 600 1470 and 1184; 1000 x 216 20.2 and 23.4, 450 x 768 30.6 and 37.1 stay
+// there).  Schedules of radices 2^k do: their folded codelets take the same
+// instructions.
+static bool dif_f64_pays(const DifTab &t, const int *rad, int np, long nvec, double hand = 1.08) {
+    bool pow2 = true;
+    for (int i = 0; i < np; i++) pow2 = pow2 && (rad[i] & (rad[i] - 1)) == 0;
+    if (pow2 || np < 2) return false;
+    double time;
+    f64_rows_per_tile(t, nvec, &time);
+    return hand * time < f64_time(rad, np, t.N, std::max(1L, std::min(nvec, 1024 / t.N)), nvec, true);
+}
+
+// False where the radices alone, in whatever order, show that it would not pay: a
+// plan that stays on the shared-memory kernel is made without the search for their
+// order and pitch (0.1 to 0.3 ms).
+static bool dif_f64_may_pay(long N, const std::vector<int> &smem, long nvec) {
+    DifTab t;
+    double cost;
+    t.N = N;
+    t.radix = least_cost(N, P_F64, 0, &cost);
+    if (t.radix.empty()) return false;
+    t.P1 = N / t.radix[0];
+    return dif_f64_pays(t, smem.data(), (int)smem.size(), nvec, 1.0);
+}
+
+// Lengths without such a schedule (factors 11 and 13): whether `tiles` tiles of v
+// transforms run here rather than as passes over global memory, which spread a call
+// evenly over the SMs but cost 30 us and 17 us a pass at least (us, passes and here:
+// 1 x 5632 55 and 78, 64 x 6500 97 and 115, 161 x 6500 196 and 223; 150 x 6500 173
+// and 116, 16 x 2816 51 and 39).
+static bool dif_f64_beats_passes(const DifTab &t, long v, long nvec) {
+    const int np = (int)t.radix.size();
+    double per = 0;
+    for (int i = 0; i < np; i++) {
+        const int R = t.radix[i];
+        per += (kDifCost[R] + 4.0 * (R - 1) / R) * (R == 11 || R == 13 ? 1.13 : 1.45);
+    }
+    const double passes = 0.0003 * per * t.N * nvec / device()->sms;
+    return 0.0003 * f64_time(t.radix.data(), np, t.N, v, nvec, false) < std::max(17.0 * np, 30.0 + passes);
+}
+
 // CTA shape of row calls: vpb transforms in nthr threads, chosen by the idle
 // thread slots of the passes' last rounds, the threads and points an SM then
 // holds, and the CTA's size.  Small CTAs (1200 to 2400 points) are in
@@ -227,62 +315,9 @@ static void *upload_tables(const std::vector<int> &rad, long N, const std::vecto
 // the best on average (us, transforms x threads): 100 points 12 x 128 45.3, 24
 // x 256 49.3, 32 x 192 49.3; 1200: 2 x 128 60.5, 4 x 256 62.6, 6 x 320 63.5;
 // 2400: 1 x 160 62.1, 2 x 320 67.8, 3 x 512 70.1.
-static double warp_rounds(long N, const std::vector<int> &rad, long v, bool dit) {
-    double c = 0;
-    for (size_t i = 0; i < rad.size(); i++) {
-        // radix 16: one instruction per point fewer where the twiddles precede
-        // the butterfly (tw_bfly), in every pass but the first
-        const int R = rad[i];
-        const double per = pass_cost(R, P_F64) - (dit && R == 16 && i > 0 ? 1.0 : 0.0);
-        c += (double)((v * (N / R) + 31) / 32 * 32) * per * R;
-    }
-    return c / (double)(v * N);
-}
-// Whether double-precision rows run on this kernel rather than the
-// shared-memory kernel with schedule `smem`: by the warp rounds of both, to
-// which the times are proportional within 8 % over 58 lengths of 64-8192 points
-// (2^24 points, us: 100 1114 -> 867, 600 1470 -> 1184, 1000 1692 -> 1419, 1200
-// 1467 -> 1285; where the rounds are equal so are the times, 4096 1237 and 1225,
-// or this kernel's are longer, 1024 1021 and 1176).
-static bool dif_f64_pays(const DifTab &t, const std::vector<int> &smem) {
-    return warp_rounds(t.N, smem, std::max(1L, 1024 / t.N), true) >= 1.11 * warp_rounds(t.N, t.radix, t.vpb, false);
-}
-
-// False where no number of transforms per CTA would make it pay: known from the
-// radices alone, so that a plan whose rows stay on the shared-memory kernel is
-// made without the search for their order and pitch (0.1 to 0.3 ms).
-static bool dif_f64_may_pay(long N, const std::vector<int> &smem) {
-    double cost;
-    const std::vector<int> rad = least_cost(N, P_F64, 0, &cost);
-    if (rad.empty()) return false;
-    const double s = warp_rounds(N, smem, std::max(1L, 1024 / N), true);
-    for (long v = 1; v <= 16; v++)
-        if (s >= 1.11 * warp_rounds(N, rad, v, false)) return true;
-    return false;
-}
-
-// Double precision: an FP64 instruction takes the pipe as long for one lane of
-// a warp as for 32, whatever else is resident, so the shape that fills its warps
-// best: the fewest warp rounds per point over the passes, in up to 72 KB (three
-// CTAs per SM).
-static void row_shape_f64(DifTab &t) {
-    const long ldb = t.radix[0] * t.P1 * 16;
-    double best = 1e30;
-    for (long v = 1; v == 1 || (v <= 16 && v * ldb <= 72 * 1024); v++) {
-        const double c = warp_rounds(t.N, t.radix, v, false);
-        const long most = v * (t.N / *std::min_element(t.radix.begin(), t.radix.end()));
-        if (c < best * 0.99) {
-            best = c;
-            t.vpb = v;
-            t.nthr = (int)std::min(256L, (most + 31) / 32 * 32);
-        }
-    }
-}
-
 static void row_shape(DifTab &t, int cls) {
-    if (t.prec == P_F64) return row_shape_f64(t);
-    const long esz = t.prec == P_F32 ? 8 : 16, regs = t.prec == P_F32 ? 64 : 128, maxt = 65536 / regs;
-    const long ldb = t.radix[0] * t.P1 * esz, unit = t.prec == P_F32 ? 1200 : 600;
+    if (t.prec == P_F64) return;  // by the call (f64_rows_per_tile)
+    const long maxt = 1024, ldb = t.radix[0] * t.P1 * 8, unit = 1200;
     const size_t np = t.radix.size();
     double best = 1e30;
     t.vpb = 1;
@@ -313,12 +348,13 @@ static void row_shape(DifTab &t, int cls) {
 }
 
 const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots,
-                          const std::vector<int> *other) {
+                          const std::vector<int> *other, long nvec) {
     if (N > (prec == P_F32 ? 16384 : 8192) || (prec == P_F64 && cls != 0)) return nullptr;
     std::lock_guard<std::mutex> lk(g_dif_mu);
     auto key = std::make_tuple(N, prec, cls);
     auto it = g_dif.find(key);
     if (it != g_dif.end()) {
+        if (other && !dif_f64_pays(it->second, other->data(), (int)other->size(), nvec)) return nullptr;
         it->second.refs++;
         return &it->second;
     }
@@ -335,14 +371,14 @@ const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *
     if (!fix) {
         auto seen = g_found.find(key);
         if (seen == g_found.end()) {
-            if (other && !dif_f64_may_pay(N, *other)) return nullptr;
+            if (other && !dif_f64_may_pay(N, *other, nvec)) return nullptr;
             if (dif_schedule(N, prec, cls, t.radix, &t.P1)) row_shape(t, cls);
             seen = g_found.emplace(key, t).first;
         }
         if (seen->second.radix.empty()) return nullptr;  // no schedule
         t = seen->second;
     }
-    if (other && !dif_f64_pays(t, *other)) return nullptr;
+    if (other && !dif_f64_pays(t, other->data(), (int)other->size(), nvec)) return nullptr;
     const int err0 = jvsip_gpu_last_error();
     std::vector<double> own;
     if (!roots) {
@@ -491,7 +527,12 @@ static bool dif_args(const Job &j, long tuned, bool alone, DifArgs<T> &a, DifCta
     if (j.kind == K_C2R) a.mH = magic_host((unsigned long)(a.p[0].S / 2 + 1));
     const size_t cap = device()->smem_optin;
     long vpb, nthr;
-    if (rows) {
+    if (rows && sizeof(T) == 8) {
+        double time;
+        vpb = f64_rows_per_tile(*t, j.nvec, &time);
+        nthr = std::min(256L, (vpb * j.N / *std::min_element(t->radix.begin(), t->radix.end()) + 31) / 32 * 32);
+        if (j.twg ? !dif_f64_pays(*t, j.radix, j.npass, j.nvec) : !dif_f64_beats_passes(*t, vpb, j.nvec)) return false;
+    } else if (rows) {
         vpb = t->vpb;
         nthr = t->nthr;
         if (tuned > 0 && tuned != vpb) {
@@ -536,6 +577,13 @@ static bool dif_args(const Job &j, long tuned, bool alone, DifArgs<T> &a, DifCta
                            ((t->fix->cols && (1 << a.lgv) == t->fix->vcol) || (t->fix->cols4 && a.lgv == 2));
         if (alone && !fixed) a.lgv = dif_col_narrow(a.lgv, j.nvec, device()->sms);
         vpb = 1L << a.lgv;
+        // some columns of a long length that only this kernel takes in one launch: the
+        // passes over global memory use more of the SMs (us, here and there: 14641 x 16
+        // 30 and 22, split 13312 x 32 47 and 33, split 8788 x 32 32 and 25; 11264 x 16
+        // 24 and 25, 13312 x 4 17 and 23, x 64 28 and 38)
+        if (!j.twg && (sizeof(T) == 8 ? !dif_f64_beats_passes(*t, vpb, j.nvec)
+                                      : (split ? 2 : 1) * j.N > 13000 && j.nvec >= 8 && j.nvec <= (split ? 64 : 32)))
+            return false;
         nthr = dif_col_threads(j.N, a.lgv, sizeof(T) == 4, alone && ((j.nvec - 1) >> a.lgv) < device()->sms);
     }
     a.vpb = (int)vpb;
@@ -741,7 +789,7 @@ VecPlan *vec_acquire(long N) {
     bool ok = true;
     for (int i = 0; i < 3; i++) {
         v->f[i] = f[i];
-        if (f[i] > 1) ok = ok && (v->tab[i] = dif_acquire(f[i], P_F32, 0, nullptr, nullptr)) != nullptr;
+        if (f[i] > 1) ok = ok && (v->tab[i] = dif_acquire(f[i], P_F32, 0, nullptr, nullptr, 0)) != nullptr;
     }
     ok = ok && (v->d_t1 = upload_roots(f[0] * V, [&](long i) { return (i / V) * (i % V); }, N)) != nullptr;
     const long C = f[2];

@@ -278,7 +278,7 @@ static bool build_tables(Plan *p, const std::vector<double> &roots);
 
 static void take_dif(Plan *p, const std::vector<double> *roots) {
     p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type), roots,
-                         p->prec == P_F64 && p->smooth ? &p->radix : nullptr);
+                         p->prec == P_F64 && p->smooth ? &p->radix : nullptr, p->mN);
 }
 
 template <typename T>
