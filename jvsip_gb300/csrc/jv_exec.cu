@@ -332,13 +332,19 @@ static bool step_job(Job &q, const Job &j, const Plan *sp) {
 
 // One step: on the register-resident kernel's column tiles at its lengths
 // (groups along the grid's y), else on the in-place mixed-radix kernel's
-// (adjacent vectors), else on the shared-memory kernel.
+// (adjacent vectors), else on the shared-memory kernel.  A single vector below 2^20
+// points, which leaves SMs idle, has the shared-memory kernel's shorter chain (8
+// points a thread instead of 16; us, that and the mixed-radix tiles: strided 10000
+// points 8.2 and 10.7, 125000 11.8 and 14.8, 600000 15.8 and 19.5, 1000000 and more
+// equal; C2R of 32768 10.1 and 13.2).
 static bool long_step_f32(Job &q, cudaStream_t st) {
     if (launch_fast_step_f32(q, st)) return true;
     if (jvsip_gpu_last_error()) return false;
-    q.no_fast = false;
-    if (launch_dif_step_f32(q, st)) return true;
-    q.no_fast = true;
+    if (q.nbatch > 1 || q.nvec * q.N >= (1L << 20)) {
+        q.no_fast = false;
+        if (launch_dif_step_f32(q, st)) return true;
+        q.no_fast = true;
+    }
     return !jvsip_gpu_last_error() && launch_smem_f32(q, st);
 }
 
