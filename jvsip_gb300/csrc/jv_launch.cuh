@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "jv_kernels.cuh"
+#include "jv_tma_box.h"
 
 namespace jv {
 
@@ -114,11 +115,8 @@ static bool tma_columns(SmemArgs<T> &a, const Job &j, long vpb, long ld) {
     const T *base = (const T *)v.re + 2 * v.off;
     if (((uintptr_t)base % 16) || ((2 * v.es * (long)sizeof(T)) % 16)) return false;
     const long N = j.N;
-    const long q = std::max(1L, 128L / (vpb * 2 * (long)sizeof(T)));  // rows keeping each box 128-byte aligned
-    const long nb = (N + 255) / 256;
-    long rows = (N + nb - 1) / nb;
-    rows = (rows + q - 1) / q * q;
-    if (rows > 256 || nb * rows > ld) return false;
+    long nb, rows;
+    if (!tma_boxes(N, vpb, (long)sizeof(T), ld, &nb, &rows)) return false;
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return false;
     int *status = kernel_status();
