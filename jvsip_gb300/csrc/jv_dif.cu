@@ -846,7 +846,12 @@ bool launch_vec_f32(const VecPlan &v, const float2 *in, float2 *out, float2 *scr
             if (has_scale) a.scale = scale;
             smem = (size_t)a.LD * V * sizeof(float2);
         }
-        const int nthr = (int)std::min(512L, std::max(64L, (V * a.N / 16 + 31) / 32 * 32));
+        // up to 2^19 points the CTAs of a pass leave SMs half empty and its time is one
+        // tile's chain: 4 points a thread instead of 16 (59049 points 8.6 us, 11.9 with
+        // 16 and 10.1 in the two steps; 125000 8.8, 11.7, 11.3; 390625 12.6, 16.3, 16.9;
+        // 786432 12.8 and 11.5 with 16)
+        const long per = A * B * C <= (1L << 19) ? 4 : 16, most = per == 4 ? 1024 : 512;
+        const int nthr = (int)std::min(most, std::max(64L, (V * a.N / per + 31) / 32 * 32));
         const DifFixEntry *f = v.tab[i]->fix;
         if (f && f->vec[i] && V == 16) {
             if (!f->vec[i](a, smem, st, groups)) return false;
