@@ -678,7 +678,10 @@ bool launch_dif_komega_r2c_f32(const Job &j, cudaStream_t st) {
     const size_t smem = (size_t)a.LD * a.vpb * sizeof(float2);
     if (smem > device()->smem_optin) return false;
     if (f && f->taper && a.vpb == f->vtaper) return f->taper(a, smem, st, 1);
-    const long nthr = std::min(512L, std::max(96L, (a.vpb * j.N / 16 + 31) / 32 * 32));
+    // 8 points a thread: without a compiled-in schedule, or with fewer rows to a tile,
+    // few CTAs are there (16 x 3000 in all 15 us, 18 with 16 points; 128 x 8192 14.4
+    // and 17.9)
+    const long nthr = std::min(1024L, std::max(96L, (a.vpb * j.N / 8 + 31) / 32 * 32));
     return dif_komega_go(DIF_R2CT, a, (int)nthr, smem, st);
 }
 

@@ -9,12 +9,21 @@
 #include "jv_launch.cuh"
 
 namespace jv {
+// Few sensors: the register-resident kernel's R2C rows first, at lengths where a
+// tile's chain there is the shorter one (us, that and the in-place kernel: 2 x 4096
+// 6.1 and 9.9, 8 x 256 4.9 and 6.5, 32 x 2048 8.2 and 9.7, 4 x 512 5.0 and 5.2; the
+// other way 48 x 2048 9.1 and 7.9, 16 x 512 7.1 and 5.9, 8 x 1536 7.9 and 6.4).
+static bool few_sensors(const Job &j) {
+    return (j.nvec <= 40 && (j.N == 128 || j.N >= 1000)) || (j.nvec <= 4 && (j.N == 256 || j.N == 512));
+}
 bool launch_komega_r2c_f32(const Job &j, cudaStream_t s) {
     if (j.kind != K_R2C || !j.taper_n || !j.taper_t) {
         set_error(E_ARG, "tapered R2C without tapers");
         return false;
     }
     const int e0 = jvsip_gpu_last_error();
+    if (few_sensors(j) && launch_fast_komega_r2c_f32(j, s)) return true;
+    if (jvsip_gpu_last_error() != e0) return false;
     if (launch_dif_komega_r2c_f32(j, s)) return true;
     if (jvsip_gpu_last_error() != e0) return false;
     if (launch_fast_komega_r2c_f32(j, s)) return true;
