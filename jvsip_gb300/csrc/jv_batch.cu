@@ -7,8 +7,8 @@
 // of the in-place mixed-radix kernel (jv_dif.cuh, k_dif_batch): one queue per
 // block size, largest tiles first, one tile per CTA -- no CTA ever waits on
 // another -- whose arguments (the call's) the CTA copies into shared memory.
-// Columns from kColStepsMin points (adjacent, more than one) go through the
-// plain calls' two steps on eight streams of their own.  Other layouts, and
+// Columns from kColStepsMin points (adjacent; 32 or more below 8192 points) go
+// through the plain calls' two steps on eight streams of their own.  Other layouts, and
 // lengths without a schedule of two codelets, keep the general kernel's fused
 // c2c passes in CTAs of 256, 512 or 1024 threads (k_batch; long adjacent
 // columns in 4-CTA clusters, k_batch_cols), each CTA asking L2
@@ -248,7 +248,8 @@ struct DifGroup {
     bool cols = false;
     int nthr = 0;
     size_t smem = 0;
-    std::vector<DifTile> tiles;
+    long ntiles = 0;
+    std::vector<int> calls;  // by their index, largest tiles first
 };
 
 struct BatchBuild {
@@ -270,9 +271,9 @@ static long tile_ld(long N, bool vf) {
 long batch_fft_per_tile(long N, bool vf, long rows);
 long batch_tuned_per_tile(long N, bool vf);  // the autotuner's entry, 0: none
 
-// Cuts a call into tiles of the in-place mixed-radix kernel; false when its
-// views or length are not for it.
-static bool dif_tiles(const Plan *p, const TileDesc &t, long nv, BatchBuild &bb) {
+// Cuts a call into tiles of the in-place mixed-radix kernel that are to occupy `sms`
+// SMs; false when its views or length are not for it.
+static bool dif_tiles(const Plan *p, const TileDesc &t, long nv, long sms, BatchBuild &bb) {
     Job j;
     j.kind = K_C2C;
     j.prec = P_F32;
@@ -294,11 +295,14 @@ static bool dif_tiles(const Plan *p, const TileDesc &t, long nv, BatchBuild &bb)
     j.cout.off = t.out_off;
     j.cout.es = t.out_es;
     j.cout.vs = t.out_vs;
-    DifArgs<float> a;
+    bb.calls.emplace_back();
+    const DifArgs<float> &a = bb.calls.back();
     DifCta c;
-    if (!dif_tile_args(j, batch_tuned_per_tile(t.N, t.vec_fast != 0), a, c) ||
-        c.smem > device()->smem_optin - kStaticArgs)
+    if (!dif_tile_args(j, batch_tuned_per_tile(t.N, t.vec_fast != 0), sms, bb.calls.back(), c) ||
+        c.smem > device()->smem_optin - kStaticArgs) {
+        bb.calls.pop_back();
         return false;
+    }
     // block sizes in steps of 64, so that one launch takes tiles of many lengths
     c.nthr = dif_batch_threads(c.nthr);
     DifGroup *g = nullptr;
@@ -311,9 +315,8 @@ static bool dif_tiles(const Plan *p, const TileDesc &t, long nv, BatchBuild &bb)
         g->nthr = c.nthr;
     }
     g->smem = std::max(g->smem, c.smem);
-    for (long v0 = 0; v0 < nv; v0 += a.vpb)
-        g->tiles.push_back(DifTile{(int)bb.calls.size(), (int)std::min((long)a.vpb, nv - v0), v0});
-    bb.calls.push_back(a);
+    g->ntiles += (nv + a.vpb - 1) / a.vpb;
+    g->calls.push_back((int)bb.calls.size() - 1);
     return true;
 }
 
@@ -321,6 +324,13 @@ static bool build_tiles(size_t n, const vsip_fftm_f *const plans[], const vsip_c
                         const vsip_cmview_f *const out[], BatchBuild &bb) {
     Device *d = device();
     if (!d) return false;
+    // a call's tiles are cut for the SMs that its share of the points fills: with the
+    // whole GPU for every call each tile held one transform or four columns (64 calls
+    // of 200 rows of 64 points 6.3 us, 18.4 so; of 128 points 10.4 and 24.7)
+    double points = 0;
+    bb.calls.reserve(n);
+    for (size_t i = 0; i < n; i++)
+        if (const Plan *p = plan_of(plans[i])) points += (double)p->MN * p->mN;
     for (size_t i = 0; i < n; i++) {
         Plan *p = plan_of(plans[i]);
         if (!p || p->prec != P_F32 || (p->type != JV_CCFFTOP && p->type != JV_CCFFTIP)) {
@@ -397,14 +407,20 @@ static bool build_tiles(size_t n, const vsip_fftm_f *const plans[], const vsip_c
         bool vf_out = labs(t.out_vs) == 1 && labs(t.out_es) != 1;
         t.vec_fast = (vf_in || vf_out) ? 1 : 0;
         t.ld = (int)tile_ld(N, t.vec_fast);
+        // columns below 8192 points in steps only where there are 32 of them, or a few
+        // calls in all: a step is two launches (us, steps and tiles: 64 calls of 3000 x
+        // 3 68 and 13, 3000 x 20 92 and 31, 3000 x 200 93 and 102, 6000 x 200 87 and 122;
+        // one call 8 and 12)
+        const bool long_call = N >= kColStepsMin && (N >= kLongFewMin || nv >= 32 || n <= 4);
         // the plan's scratch is had now (nothing may allocate while a batch is
         // recorded into its graph); without it the call goes in tiles
-        if (resident_long_columns_f(p, x, y) && enqueue_resident_c2c_f(p, x, y, nullptr, true)) {
+        if (long_call && resident_long_columns_f(p, x, y) && enqueue_resident_c2c_f(p, x, y, nullptr, true)) {
             bb.steps.push_back(StepCall{p, x, y});
             bb.bytes += 16.0 * N * nv;
             continue;
         }
-        if (dif_tiles(p, t, nv, bb)) {
+        const long share = std::max(1L, (long)(d->sms * (double)N * nv / points));
+        if (dif_tiles(p, t, nv, share, bb)) {
             bb.bytes += 16.0 * N * nv;
             continue;
         }
@@ -457,8 +473,9 @@ static bool build_tiles(size_t n, const vsip_fftm_f *const plans[], const vsip_c
             return (long)a.N * a.nt > (long)b.N * b.nt;
         });
     for (DifGroup &g : bb.groups)
-        std::stable_sort(g.tiles.begin(), g.tiles.end(), [&](const DifTile &a, const DifTile &b) {
-            return (long)bb.calls[a.call].N * a.nt > (long)bb.calls[b.call].N * b.nt;
+        std::stable_sort(g.calls.begin(), g.calls.end(), [&](int x, int y) {
+            const DifArgs<float> &a = bb.calls[x], &b = bb.calls[y];
+            return (long)a.N * std::min((long)a.vpb, a.nvec) > (long)b.N * std::min((long)b.vpb, b.nvec);
         });
     // the groups of the largest CTAs are launched first
     std::stable_sort(bb.groups.begin(), bb.groups.end(), [](const DifGroup &a, const DifGroup &b) { return a.smem > b.smem; });
@@ -484,35 +501,37 @@ struct DevBatch {
 
 static bool upload(const BatchBuild &bb, DevBatch &db) {
     db.steps = bb.steps;
-    std::vector<TileDesc> all;
+    // one buffer, one copy: [tiles of the classes | calls | tiles of the groups]
+    size_t nq = 0, nt = 0;
+    for (int c = 0; c < kClasses; c++) nq += bb.tiles[c].size();
+    for (const DifGroup &g : bb.groups) nt += (size_t)g.ntiles;
+    const size_t oc = (nq * sizeof(TileDesc) + 15) / 16 * 16, ot = oc + bb.calls.size() * sizeof(DifArgs<float>),
+                 bytes = std::max<size_t>(1, ot + nt * sizeof(DifTile));
+    std::vector<unsigned char> host(bytes);
+    TileDesc *hq = (TileDesc *)host.data();
     for (int c = 0; c < kClasses; c++) {
-        db.off[c] = (int)all.size();
+        db.off[c] = db.total;
         db.n[c] = (int)bb.tiles[c].size();
         db.smem[c] = bb.smem[c];
-        all.insert(all.end(), bb.tiles[c].begin(), bb.tiles[c].end());
+        if (db.n[c]) memcpy(hq + db.total, bb.tiles[c].data(), bb.tiles[c].size() * sizeof(TileDesc));
+        db.total += db.n[c];
     }
-    db.total = (int)all.size();
-    db.q = (TileDesc *)dmalloc(std::max<size_t>(1, all.size()) * sizeof(TileDesc));
-    if (!db.q) return false;
-    Device *d = device();
-    if (!all.empty() && !cuda_ok(cudaMemcpyAsync(db.q, all.data(), all.size() * sizeof(TileDesc),
-                                                 cudaMemcpyHostToDevice, d->stream),
-                                 "batch queue upload"))
-        return false;
-    if (bb.groups.empty()) return true;
-    std::vector<DifTile> tiles;
+    if (!bb.calls.empty()) memcpy(host.data() + oc, bb.calls.data(), bb.calls.size() * sizeof(DifArgs<float>));
+    DifTile *ht = (DifTile *)(host.data() + ot);
     for (const DifGroup &g : bb.groups) {
-        db.groups.push_back({g.cols, g.nthr, (int)tiles.size(), (int)g.tiles.size(), g.smem});
-        tiles.insert(tiles.end(), g.tiles.begin(), g.tiles.end());
+        int first = db.groups.empty() ? 0 : db.groups.back().first + db.groups.back().n;
+        db.groups.push_back({g.cols, g.nthr, first, (int)g.ntiles, g.smem});
+        for (int c : g.calls) {
+            const DifArgs<float> &a = bb.calls[c];
+            for (long v0 = 0; v0 < a.nvec; v0 += a.vpb)
+                ht[first++] = DifTile{c, (int)std::min((long)a.vpb, a.nvec - v0), v0};
+        }
     }
-    db.calls = (DifArgs<float> *)dmalloc(bb.calls.size() * sizeof(DifArgs<float>));
-    db.tiles = (DifTile *)dmalloc(tiles.size() * sizeof(DifTile));
-    return db.calls && db.tiles &&
-           cuda_ok(cudaMemcpyAsync(db.calls, bb.calls.data(), bb.calls.size() * sizeof(DifArgs<float>),
-                                   cudaMemcpyHostToDevice, d->stream),
-                   "batch queue upload") &&
-           cuda_ok(cudaMemcpyAsync(db.tiles, tiles.data(), tiles.size() * sizeof(DifTile), cudaMemcpyHostToDevice,
-                                   d->stream),
+    db.q = (TileDesc *)dmalloc(bytes);
+    if (!db.q) return false;
+    db.calls = (DifArgs<float> *)((unsigned char *)db.q + oc);
+    db.tiles = (DifTile *)((unsigned char *)db.q + ot);
+    return cuda_ok(cudaMemcpyAsync(db.q, host.data(), bytes, cudaMemcpyHostToDevice, device()->stream),
                    "batch queue upload");
 }
 
@@ -641,8 +660,6 @@ static bool launch(const DevBatch &db, cudaStream_t st) {
 
 static void free_dev(DevBatch &db) {
     dfree(db.q);
-    dfree(db.calls);
-    dfree(db.tiles);
     db.q = nullptr;
     db.calls = nullptr;
     db.tiles = nullptr;

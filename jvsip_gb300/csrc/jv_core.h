@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -212,6 +213,7 @@ struct DifTab {
     const struct DifFixEntry *fix = nullptr;  // the length's compiled-in kernels (or null)
     long vpb = 1;             // CTA shape of row calls: transforms, threads
     int nthr = 128;
+    std::shared_ptr<const void> args;  // DifArgs of the schedule, views empty
     int refs = 0;
 };
 std::vector<double> unit_roots(long N);  // exp(-2 pi i m/N), m < N, (re, im) pairs

@@ -347,6 +347,39 @@ static void row_shape(DifTab &t, int cls) {
     }
 }
 
+// the schedule's part of the kernel's arguments, made once for a table
+template <typename T> static std::shared_ptr<const void> dif_fill(const DifTab &t) {
+    auto made = std::make_shared<DifArgs<T>>();
+    DifArgs<T> &a = *made;
+    memset(&a, 0, sizeof a);
+    a.N = (int)t.N;
+    a.np = (int)t.radix.size();
+    a.P1 = (int)t.P1;
+    a.LD = (int)(t.radix[0] * t.P1);
+    a.tw = (const typename cplx_t<T>::t *)t.d_tw;
+    long M = t.N;
+    for (int i = 0; i < a.np; i++) {
+        DifPass &p = a.p[i];
+        p.R = t.radix[i];
+        p.S = (int)(M / p.R);
+        p.NR = (int)(t.N / p.R);
+        p.mstep = (int)M - p.S;
+        p.NB1 = (int)(t.N / t.radix[0] / p.R);
+        p.two = t.two[i];
+        p.mNR = magic_host((unsigned long)p.NR);
+        p.mNB1 = magic_host((unsigned long)p.NB1);
+        p.mS = magic_host((unsigned long)p.S);
+        p.mR = magic_host((unsigned long)p.R);
+        M = p.S;
+    }
+    if (t.cls == 1) a.mH = magic_host((unsigned long)(a.p[a.np - 1].NR / 2 + 1));
+    if (t.cls == 2) a.mH = magic_host((unsigned long)(a.p[0].S / 2 + 1));
+    return made;
+}
+template <typename T> static const DifArgs<T> &dif_base(const DifTab &t) {
+    return *static_cast<const DifArgs<T> *>(t.args.get());
+}
+
 const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots,
                           const std::vector<int> *other, long nvec) {
     if (N > (prec == P_F32 ? 16384 : 8192) || (prec == P_F64 && cls != 0)) return nullptr;
@@ -395,6 +428,7 @@ const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *
         t.vpb = fix->vpb;
         t.nthr = fix->nthr;
     }
+    t.args = prec == P_F32 ? dif_fill<float>(t) : dif_fill<double>(t);
     t.refs = 1;
     auto &slot = g_dif[key];
     slot = t;
@@ -422,30 +456,6 @@ template <typename T> static bool real_pairs(const RView &r, long len, long nvec
            (uintptr_t)r.a % (2 * sizeof(T)) == 0;
 }
 
-// the schedule's part of the kernel's arguments
-template <typename T> static void dif_fill(DifArgs<T> &a, const DifTab &t) {
-    a.N = (int)t.N;
-    a.np = (int)t.radix.size();
-    a.P1 = (int)t.P1;
-    a.LD = (int)(t.radix[0] * t.P1);
-    a.tw = (const typename cplx_t<T>::t *)t.d_tw;
-    long M = t.N;
-    for (int i = 0; i < a.np; i++) {
-        DifPass &p = a.p[i];
-        p.R = t.radix[i];
-        p.S = (int)(M / p.R);
-        p.NR = (int)(t.N / p.R);
-        p.mstep = (int)M - p.S;
-        p.NB1 = (int)(t.N / t.radix[0] / p.R);
-        p.two = t.two[i];
-        p.mNR = magic_host((unsigned long)p.NR);
-        p.mNB1 = magic_host((unsigned long)p.NB1);
-        p.mS = magic_host((unsigned long)p.S);
-        p.mR = magic_host((unsigned long)p.R);
-        M = p.S;
-    }
-}
-
 // Points of a column call from which tiles of 4 columns are too narrow.  Tiles of
 // 4 against 8 (run-time schedule) at 2^26 points, us: 1125 points 475 and 321,
 // 1350: 499 and 334, 1500: 499 and 436, 1792: 482 and 410, 1920: 441 and 336, 2048:
@@ -454,15 +464,16 @@ template <typename T> static void dif_fill(DifArgs<T> &a, const DifTab &t) {
 constexpr long kColWidePts = 5L << 23;
 
 // The kernel's arguments for a call and its CTA: tuned > 0 asks for that many
-// transforms (a power of two for column tiles); `alone`: nothing else fills the
-// SMs that the call's tiles leave idle.  False when the call does not qualify.
+// transforms (a power of two for column tiles); the call's tiles are to occupy
+// `sms` SMs (a call of a batch has its share); column tiles become narrower than
+// four for it where `narrow`.  False when the call does not qualify.
 template <typename T>
-static bool dif_args(const Job &j, long tuned, bool alone, DifArgs<T> &a, DifCta &cta) {
+static bool dif_args(const Job &j, long tuned, long sms, bool narrow, DifArgs<T> &a, DifCta &cta) {
     typedef typename cplx_t<T>::t C;
     const DifTab *t = j.dif;
     if (!t || j.no_fast || j.no_dif || j.nvec <= 0 || j.gram || j.taper_n) return false;
     const CView &ci = j.cin, &co = j.cout;
-    memset(&a, 0, sizeof a);
+    a = dif_base<T>(*t);
     bool rows = true, split = false;
     if (j.kind == K_C2C) {
         split = ci.cst == 1 && co.cst == 1;
@@ -522,9 +533,6 @@ static bool dif_args(const Job &j, long tuned, bool alone, DifArgs<T> &a, DifCta
     a.nvec = j.nvec;
     a.has_scale = j.has_scale;
     a.scale = j.has_scale ? (T)j.scale : (T)1;
-    dif_fill(a, *t);
-    if (j.kind == K_R2C) a.mH = magic_host((unsigned long)(a.p[a.np - 1].NR / 2 + 1));
-    if (j.kind == K_C2R) a.mH = magic_host((unsigned long)(a.p[0].S / 2 + 1));
     const size_t cap = device()->smem_optin;
     long vpb, nthr;
     if (rows && sizeof(T) == 8) {
@@ -541,7 +549,7 @@ static bool dif_args(const Job &j, long tuned, bool alone, DifArgs<T> &a, DifCta
         } else if (tuned <= 0) {
             // few transforms: smaller CTAs, so that more SMs work on them, with
             // every pass in one round
-            while (vpb > 1 && (j.nvec + vpb - 1) / vpb < 2L * device()->sms) vpb = (vpb + 1) / 2;
+            while (vpb > 1 && (j.nvec + vpb - 1) / vpb < 2L * sms) vpb = (vpb + 1) / 2;
             if (vpb < t->vpb)
                 nthr = std::min(256L, (vpb * j.N / *std::min_element(t->radix.begin(), t->radix.end()) + 31) / 32 * 32);
         }
@@ -564,7 +572,7 @@ static bool dif_args(const Job &j, long tuned, bool alone, DifArgs<T> &a, DifCta
             j.nvec * j.N >= kColWidePts)
             a.lgv = 3;
         // few columns: tiles of 4, so that more SMs work on them
-        if (((j.nvec - 1) >> a.lgv) + 1 < device()->sms && j.nbatch <= 1) a.lgv = std::min(a.lgv, 2);
+        if (((j.nvec - 1) >> a.lgv) + 1 < sms && j.nbatch <= 1) a.lgv = std::min(a.lgv, 2);
         if (tuned > 0) a.lgv = dif_col_tuned(tuned, j.nvec);
         while (a.lgv > 0 && ((size_t)a.LD << a.lgv) * sizeof(C) > cap) a.lgv--;
         // down to one column where SMs would be idle and no compiled-in kernel
@@ -575,7 +583,7 @@ static bool dif_args(const Job &j, long tuned, bool alone, DifArgs<T> &a, DifCta
         // fours stay: 1000 x 16 3.8 and 4.5 in ones)
         const bool fixed = sizeof(T) == 4 && !split && t->fix &&
                            ((t->fix->cols && (1 << a.lgv) == t->fix->vcol) || (t->fix->cols4 && a.lgv == 2));
-        if (alone && !fixed) a.lgv = dif_col_narrow(a.lgv, j.nvec, device()->sms);
+        if (narrow && !fixed) a.lgv = dif_col_narrow(a.lgv, j.nvec, sms);
         vpb = 1L << a.lgv;
         // some columns of a long length that only this kernel takes in one launch: the
         // passes over global memory use more of the SMs (us, here and there: 14641 x 16
@@ -584,7 +592,7 @@ static bool dif_args(const Job &j, long tuned, bool alone, DifArgs<T> &a, DifCta
         if (!j.twg && (sizeof(T) == 8 ? !dif_f64_beats_passes(*t, vpb, j.nvec)
                                       : (split ? 2 : 1) * j.N > 13000 && j.nvec >= 8 && j.nvec <= (split ? 64 : 32)))
             return false;
-        nthr = dif_col_threads(j.N, a.lgv, sizeof(T) == 4, alone && ((j.nvec - 1) >> a.lgv) < device()->sms);
+        nthr = dif_col_threads(j.N, a.lgv, sizeof(T) == 4, narrow && ((j.nvec - 1) >> a.lgv) < sms);
     }
     a.vpb = (int)vpb;
     cta.nthr = (int)nthr;
@@ -598,7 +606,7 @@ template <typename T>
 static bool launch_dif_t(const Job &j, cudaStream_t st) {
     DifArgs<T> a;
     DifCta c;
-    if (j.nbatch > 1 || j.tw_lo || !dif_args<T>(j, 0, true, a, c)) return false;
+    if (j.nbatch > 1 || j.tw_lo || !dif_args<T>(j, 0, device()->sms, true, a, c)) return false;
     if constexpr (sizeof(T) == 4) {
         const DifFixEntry *f = j.dif->fix;
         if (f && !c.split && c.rows && f->rows) return f->rows(a, c.smem, st, 1);
@@ -620,7 +628,7 @@ static bool launch_dif_t(const Job &j, cudaStream_t st) {
 bool launch_dif_step_f32(const Job &j, cudaStream_t st) {
     DifArgs<float> a;
     DifCta c;
-    if (j.kind != K_C2C || j.nbatch < 1 || j.nbatch > 65535 || !dif_args<float>(j, 0, false, a, c) || c.rows || c.split)
+    if (j.kind != K_C2C || j.nbatch < 1 || j.nbatch > 65535 || !dif_args<float>(j, 0, device()->sms, false, a, c) || c.rows || c.split)
         return false;
     a.bvs_in = j.bvs_in;
     a.bvs_out = j.bvs_out;
@@ -646,8 +654,7 @@ bool launch_dif_komega_r2c_f32(const Job &j, cudaStream_t st) {
     const CView &co = j.cout;
     if (!real_pairs<float>(j.rin, 2 * j.N, j.nvec) || !interleaved_c<float>(co) || co.vs != 1 || co.es < j.nvec)
         return false;
-    DifArgs<float> a;
-    memset(&a, 0, sizeof a);
+    DifArgs<float> a = dif_base<float>(*t);
     a.in = (const float2 *)j.rin.a + j.rin.off / 2;
     a.wb = const_cast<float2 *>(a.in);
     a.vs_in = j.rin.vs / 2;
@@ -663,9 +670,7 @@ bool launch_dif_komega_r2c_f32(const Job &j, cudaStream_t st) {
     a.tp_t = (const float *)j.taper_t;
     a.tp_n_st = j.taper_n_st;
     a.tp_t_st = j.taper_t_st;
-    dif_fill(a, *t);
     a.LD |= 1;
-    a.mH = magic_host((unsigned long)(a.p[a.np - 1].NR / 2 + 1));
     const DifFixEntry *f = t->fix;
     a.lgv = 4;
     while (a.lgv > 2 && ((size_t)a.LD << a.lgv) * sizeof(float2) > 72 * 1024) a.lgv--;
@@ -692,7 +697,7 @@ bool launch_dif_komega_power_f32(const Job &j, cudaStream_t st) {
     q.gram = nullptr;
     DifArgs<float> a;
     DifCta c;
-    if (j.kind != K_C2C || !dif_args<float>(q, 0, true, a, c) || !c.rows || c.split) return false;
+    if (j.kind != K_C2C || !dif_args<float>(q, 0, device()->sms, true, a, c) || !c.rows || c.split) return false;
     a.gram = (float *)j.gram;
     a.g_es = j.gram_es;
     a.g_vs = j.gram_vs;
@@ -809,9 +814,7 @@ bool launch_vec_f32(const VecPlan &v, const float2 *in, float2 *out, float2 *scr
     const long A = v.f[0], B = v.f[1], C = v.f[2];
     for (int i = 0; i < 3; i++) {
         if (!v.tab[i]) continue;
-        DifArgs<float> a;
-        memset(&a, 0, sizeof a);
-        dif_fill(a, *v.tab[i]);
+        DifArgs<float> a = dif_base<float>(*v.tab[i]);
         const long V = vec_tile(a.N, A * B * C);
         a.lgv = V == 16 ? 4 : V == 8 ? 3 : 2;
         a.vpb = (int)V;
@@ -865,8 +868,8 @@ bool launch_vec_f32(const VecPlan &v, const float2 *in, float2 *out, float2 *scr
     return true;
 }
 
-bool dif_tile_args(const Job &j, long tuned, DifArgs<float> &a, DifCta &c) {
-    return j.kind == K_C2C && dif_args<float>(j, tuned, false, a, c) && !c.split;
+bool dif_tile_args(const Job &j, long tuned, long sms, DifArgs<float> &a, DifCta &c) {
+    return j.kind == K_C2C && dif_args<float>(j, tuned, sms, true, a, c) && !c.split;
 }
 
 bool launch_dif_f32(const Job &j, cudaStream_t st) { return launch_dif_t<float>(j, st); }

@@ -586,7 +586,8 @@ struct DifCta {
     size_t smem = 0;
     bool rows = true, split = false;
 };
-bool dif_tile_args(const Job &j, long tuned, DifArgs<float> &a, DifCta &c);  // batch tiles; false: not for k_dif
+// batch tiles that are to occupy `sms` SMs; false: not for k_dif
+bool dif_tile_args(const Job &j, long tuned, long sms, DifArgs<float> &a, DifCta &c);
 bool dif_batch_go(bool cols, const DifArgs<float> *calls, const DifTile *q, int ntiles, int nthr, size_t smem,
                   cudaStream_t st);
 

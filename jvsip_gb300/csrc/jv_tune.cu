@@ -173,6 +173,7 @@ long batch_fft_per_tile(long N, bool vf, long rows) {
 long batch_tuned_per_tile(long N, bool vf) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     load_cache();
+    if (g_tuned.empty()) return 0;
     auto it = g_tuned.find(std::make_tuple(N, (int)P_F32, vf ? 1 : 0));
     return it != g_tuned.end() ? std::min(it->second, std::max(1L, 16384 / N)) : 0;
 }
