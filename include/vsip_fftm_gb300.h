@@ -428,6 +428,9 @@ int jvsip_gpu_test_wait_expiry(int on);
 void *jvsip_gpu_stream(void);
 /* Number of kernels this library has launched since it was loaded. */
 unsigned long jvsip_gpu_kernel_launches(void);
+/* Number of calls on host blocks that ran on the host arrays themselves,
+ * without device copies, since the library was loaded. */
+unsigned long jvsip_gpu_host_direct_calls(void);
 /* Plan introspection: the device pass radices (returns their count) and the
  * reference's digit-reversal map of the plan length (c_VSIP_src/VI_jofk.h),
  * kept for parity checks (returns the map length). */

@@ -51,7 +51,7 @@ EXPORTS = [
     "jvsip_fftm_setform_f", "jvsip_fftm_getform_f",
     "jvsip_fftm_batch_f", "jvsip_fftm_batch_create_f", "jvsip_fftm_batch_run_f", "jvsip_fftm_batch_destroy_f",
     "jvsip_gpu_build_info", "jvsip_gpu_synchronize", "jvsip_gpu_stream", "jvsip_fftm_passes", "jvsip_fftm_jofk", "jvsip_fftm_graphs",
-    "jvsip_gpu_kernel_launches", "jvsip_ccfftm_noalloc_f", "jvsip_fftm_autotune_f",
+    "jvsip_gpu_kernel_launches", "jvsip_gpu_host_direct_calls", "jvsip_ccfftm_noalloc_f", "jvsip_fftm_autotune_f",
     "jvsip_fftm_autotune_entries",
     "vsip_ccfftop_create_f", "vsip_ccfftip_create_f", "vsip_rcfftop_create_f", "vsip_crfftop_create_f",
     "vsip_ccfftop_create_d", "vsip_ccfftip_create_d", "vsip_rcfftop_create_d", "vsip_crfftop_create_d",
@@ -190,6 +190,7 @@ def lib(load_only: bool = False):
     L.jvsip_gpu_build_info.restype = C.c_char_p
     L.jvsip_gpu_stream.restype = vp
     L.jvsip_gpu_kernel_launches.restype = C.c_ulong
+    L.jvsip_gpu_host_direct_calls.restype = C.c_ulong
     L.jvsip_gpu_test_wait_expiry.argtypes = [C.c_int]
     L.jvsip_ccfftm_noalloc_f.argtypes = [vp, vp, C.c_long, vp, C.c_long]
     L.jvsip_fftm_autotune_f.argtypes = [C.c_size_t, vp, C.c_int]

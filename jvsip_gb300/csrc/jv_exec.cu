@@ -15,9 +15,11 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <vector>
 
 #include "jv_core.h"
+#include "jv_host_rule.h"
 
 namespace jv {
 
@@ -797,15 +799,21 @@ static void fill_job(Job &j, const Plan *p, int kind) {
 
 // Whether a call on host blocks runs on the host arrays themselves, without
 // device copies: transforms along contiguous elements in one launch that reads
-// and writes every element once, 64 MiB in all, arrays that do not overlap.
+// and writes every element once, 64 MiB in all, arrays that do not overlap, rows
+// that are not too short for their number (host_rows_pay).
 // The copies' calls and the half-duplex of copying in, then out, cost more than
 // the kernel's own C2C traffic (256 rows of 1000 complex floats 32 us against
 // 53 staged, 8 rows 14 against 30, 2000 x 1024 175 against 212; the first call
 // on untouched pages 52 against 77 us).  JVSIP_GPU_NO_PIPELINE keeps the copies.
-static bool host_direct(const Staging &s, const Job &j, long es_in, long es_out) {
-    if (s.regs.empty() || j.no_pipeline || j.form > JVSIP_FORM_PLAIN || es_in != 1 || es_out != 1) return false;
+static std::atomic<unsigned long> g_host_direct{0};  // calls that did (introspection)
+static bool host_direct(const Staging &s, const Job &j, const Geo &in, const Geo &out) {
+    if (s.regs.empty() || j.no_pipeline || j.form > JVSIP_FORM_PLAIN || in.es != 1 || out.es != 1) return false;
     if (j.lp || !(job_in_smem(j) || (j.dif && !j.no_fast && !j.no_dif && j.N > 1))) return false;
-    return s.inside && s.apart() && host_access();
+    const size_t moved = (size_t)j.N * j.nvec * (j.prec == P_F32 ? 16 : 32);
+    if (!host_rows_pay(j.N, in.len, in.vs, j.nvec, j.prec != P_F32, moved)) return false;
+    if (!s.inside || !s.apart() || !host_access()) return false;
+    g_host_direct.fetch_add(1, std::memory_order_relaxed);
+    return true;
 }
 
 // Host-resident c2c call whose views are rows of unit element stride and
@@ -922,7 +930,7 @@ static void exec_cc(Plan *p, const CMV *x, const CMV *y, bool ip) {
     cudaStream_t st = d->stream;
     stage_c(stg, rx, true, same_view);
     if (!same_view) stage_c(stg, ry, !ry.g.dense() || (y->block == x->block), true);
-    stg.direct = (same_view || x->block != y->block) && host_direct(stg, j, rx.g.es, ry.g.es);
+    stg.direct = (same_view || x->block != y->block) && host_direct(stg, j, rx.g, ry.g);
     if (!stg.upload(st)) return;
     j.cin = dev_c(stg, rx);
     j.cout = same_view ? j.cin : dev_c(stg, ry);
@@ -1029,7 +1037,7 @@ static void exec_rc(Plan *p, const RMV *x, const CMV *z) {
     cudaStream_t st = d->stream;
     stage_r(stg, rx, true, false);
     stage_c(stg, rz, !rz.g.dense(), true);
-    stg.direct = host_direct(stg, j, rx.g.es, rz.g.es);
+    stg.direct = host_direct(stg, j, rx.g, rz.g);
     if (!stg.upload(st)) return;
     j.rin = dev_r(stg, rx);
     j.cout = dev_c(stg, rz);
@@ -1065,7 +1073,7 @@ static void exec_cr(Plan *p, const CMV *z, const RMV *x) {
     cudaStream_t st = d->stream;
     stage_c(stg, rz, true, false);
     stage_r(stg, rx, !rx.g.dense(), true);
-    stg.direct = host_direct(stg, j, rz.g.es, rx.g.es);
+    stg.direct = host_direct(stg, j, rz.g, rx.g);
     if (!stg.upload(st)) return;
     j.cin = dev_c(stg, rz);
     j.rout = dev_r(stg, rx);
@@ -1207,6 +1215,8 @@ void vsip_crfftop_d(const vsip_fft_d *p, const vsip_cvview_d *z, const vsip_vvie
     exec_cr<double, vsip_cmview_d, vsip_mview_d, vsip_cblock_d, vsip_block_d>(plan_of_v(p), z ? &mz : nullptr,
                                                                              x ? &mx : nullptr);
 }
+
+unsigned long jvsip_gpu_host_direct_calls(void) { return g_host_direct.load(std::memory_order_relaxed); }
 
 const char *jvsip_gpu_build_info(void) {
     static thread_local char buf[256];  // valid until the calling thread's next call
