@@ -627,7 +627,9 @@ static bool run_long(Job &j, cudaStream_t st, bool *handled) {
 // Calls that the register-resident kernel runs faster than the in-place one
 // (us on 2^24 points in rows, 2^23 otherwise): rows of 512 / 768 / 4096 points
 // 45.2 / 49.2 / 48.9 against 47.0 / 51.2 / 49.4, when they fill the GPU (64 rows
-// of 512: 6.2 against 4.0); R2C of 512 points 28.7 against 30.8, C2R of 512 32.8
+// of 512: 6.2 against 4.0; 4096 points at any count, 64 rows 3.2 and 3.4); R2C from
+// 5 * 2^20 points: 12001 x 512 19.7 and 21.4, 16384 x 512 28.4 and 30.6, 8192 x 2048
+// 53.8 and 56.0, 16384 x 1024 51.7 and 53.9; R2C of 512 real points 28.7 against 30.8, C2R of 512 32.8
 // and 33.0 (4096 rows: 6.2 and 8.2), R2C and C2R of 8192 points 34.8 against
 // 38; columns of 4096 points 53 against 61.  Large calls on columns of powers of
 // two, whose rows of a tile lie a large stride apart, keep its 16-column and
@@ -639,10 +641,11 @@ static bool run_long(Job &j, cudaStream_t st, bool *handled) {
 // 1000 / 1024 points 41.8 / 51.3 / 43.7 against 43.6 / 70.4 / 47.1; R2C of 1536
 // 32.9 against 34.1, C2R 32.9 against 35.1; columns of 1000 35.0 against 41.0).
 static bool fast_first(const Job &j) {
+    if (j.kind == K_R2C && (j.N == 512 || j.N == 1024 || j.N == 2048) && j.nvec * j.N >= 5L << 20) return true;
     if (j.kind != K_C2C) return j.N == 256 || j.N == 4096;
     if (j.cin.cst != 2) return true;  // split complex
     if (j.cin.es == 1 && j.cout.es == 1)
-        return (j.N == 512 || j.N == 768 || j.N == 4096) && j.nvec * j.N >= 4096L * device()->sms;
+        return j.N == 4096 || ((j.N == 512 || j.N == 768) && j.nvec * j.N >= 4096L * device()->sms);
     const long pts = j.nvec * j.N;
     return j.N == 4096 || ((j.N == 64 || j.N == 256) && pts >= (1L << 20)) || (j.N == 512 && pts >= (1L << 24)) ||
            (j.N == 128 && pts >= (1L << 25));

@@ -15,6 +15,14 @@ static bool launch_fast_real_t(const Job &j, cudaStream_t st) {
         case 4096: return launch_fast_n<4096, 256, 1, RList<16, 16, 16>, false, false, false, false, RM, FXK>(j, st);
         default: break;
     }
+    if constexpr (FXK == 0 && RM == 1) {  // large R2C calls (fast_first)
+        switch (j.N) {
+            case 512: return launch_fast_n<512, 32, 8, RList<16, 16, 2>, false, false, false, false, RM, FXK>(j, st);
+            case 1024: return launch_fast_n<1024, 64, 4, RList<16, 16, 4>, false, false, false, false, RM, FXK>(j, st);
+            case 2048: return launch_fast_n<2048, 128, 2, RList<16, 16, 8>, false, false, false, false, RM, FXK>(j, st);
+            default: break;
+        }
+    }
     if constexpr (FXK != 0) {
         switch (j.N) {
             case 64: return launch_fast_n<64, 4, 64, RList<16, 4>, false, false, false, false, RM, FXK>(j, st);
