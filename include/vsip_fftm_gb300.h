@@ -366,7 +366,8 @@ int jvsip_fftm_batch_f(size_t n, const vsip_fftm_f *const plans[],
 
 /* A captured batch: the descriptor queue is built and uploaded once and the
  * launch is recorded in a CUDA graph; jvsip_fftm_batch_run_f replays it.
- * The views' blocks must stay admitted (device addresses are baked in). */
+ * The views' blocks must stay admitted and the plans alive (device addresses
+ * are baked in). */
 typedef struct jvsip_fftm_batchplan_s jvsip_fftm_batchplan_f;
 jvsip_fftm_batchplan_f *jvsip_fftm_batch_create_f(size_t n, const vsip_fftm_f *const plans[],
                                               const vsip_cmview_f *const in[],

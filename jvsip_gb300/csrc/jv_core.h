@@ -216,13 +216,13 @@ struct DifTab {
     std::shared_ptr<const void> args;  // DifArgs of the schedule, views empty
     int refs = 0;
 };
+void unit_root(long m, long N, double *c, double *s);  // exp(-2 pi i m/N), the angle reduced to [0, pi]
 std::vector<double> unit_roots(long N);  // exp(-2 pi i m/N), m < N, (re, im) pairs
 // nullptr: no schedule for N (or no memory).  roots: unit_roots(N) when the caller has them;
 // other: double precision, the shared-memory kernel's schedule to be better than on nvec rows (or null)
 const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots, const std::vector<int> *other,
                           long nvec);
 void dif_release(const DifTab *t);
-bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1);
 bool launch_dif_f32(const Job &j, cudaStream_t s);  // false when the call does not qualify
 bool launch_dif_f64(const Job &j, cudaStream_t s);
 bool launch_dif_komega_r2c_f32(const Job &j, cudaStream_t s);    // k-omega tapered R2C rows

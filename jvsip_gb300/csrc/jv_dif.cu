@@ -1,5 +1,5 @@
 // jv_dif.cu -- host side of the in-place mixed-radix kernel (jv_dif.cuh): the
-// radix schedule and shared-memory pitch of a length (dif_shape), its twiddle
+// radix schedule and shared-memory pitch of a length (dif_schedule), its twiddle
 // tables (shared by all plans of the length) and the launchers.
 #include <math.h>
 #include <stdio.h>
@@ -107,7 +107,7 @@ static std::vector<int> least_cost(long N, int prec, int cls, double *cost) {
 // The schedule of length N: the radices of least cost, in the order and with
 // the block pitch of the fewest shared-memory wavefronts (larger first radices
 // on ties).
-bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1) {
+static bool dif_schedule(long N, int prec, int cls, std::vector<int> &rad, long *P1) {
     double cost;
     const std::vector<int> pick = least_cost(N, prec, cls, &cost);
     if (pick.empty()) return false;
@@ -188,17 +188,6 @@ static std::map<std::tuple<long, int, int>, DifTab> g_dif;
 // schedules and CTA shapes found so far (host only; one small entry per length
 // a program has planned, at most 16384 x 3): the search takes 0.1 to 0.3 ms
 static std::map<std::tuple<long, int, int>, DifTab> g_found;
-
-static void root(long m, long N, double *c, double *s) {  // exp(-2 pi i m/N)
-    bool flip = false;
-    if (2 * m > N) {
-        m = N - m;
-        flip = true;
-    }
-    const double a = 2.0 * 3.14159265358979323846264338327950288 * ((double)m / (double)N);
-    *c = cos(a);
-    *s = flip ? sin(a) : -sin(a);
-}
 
 template <typename T>
 static void *upload_tables(const std::vector<int> &rad, long N, const std::vector<double> &roots,
@@ -763,7 +752,7 @@ template <typename F> static void *upload_roots(long n, F exponent, long N) {
     std::vector<float> t(2 * n);
     for (long i = 0; i < n; i++) {
         double c, s;
-        root(exponent(i) % N, N, &c, &s);
+        unit_root(exponent(i) % N, N, &c, &s);
         t[2 * i] = (float)c;
         t[2 * i + 1] = (float)s;
     }

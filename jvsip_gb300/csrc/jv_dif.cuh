@@ -15,7 +15,7 @@
 // k_smem hold every butterfly of a thread in registers between two barriers),
 // a butterfly's addresses are computed once, and any thread count serves any
 // radix.  The pitch P1 of the k1 blocks is the one of 16 paddings whose
-// accesses collide least in the shared-memory banks (dif_shape).
+// accesses collide least in the shared-memory banks (dif_schedule).
 #pragma once
 
 #include "jv_kernels.cuh"

@@ -230,7 +230,7 @@ std::vector<std::vector<int>> schedule_candidates(long N, long maxt, size_t limi
 }
 
 // exp(-2 pi i m/N) in double with the angle reduced to [0, pi] by symmetry
-static void unit_root(long m, long N, double *c, double *s) {
+void unit_root(long m, long N, double *c, double *s) {
     bool flip = false;
     if (2 * m > N) {
         m = N - m;
@@ -519,7 +519,7 @@ static bool build_long(Plan *p) {
     if (p->prec == P_F32 && (N & (N - 1)) == 0 && bits >= 13 && bits <= 20) {
         const std::vector<long> rad = {1L << ((bits + 1) / 2), 1L << (bits / 2)};
         bool ok = true;
-        for (long R : rad) ok = ok && R >= 64 && R <= 4096;
+        for (long R : rad) ok = ok && R >= 64 && R <= 1024;
         for (size_t i = 0; ok && i < rad.size(); i++) {
             Plan *q = step_plan<T>(rad[i], p->prec);
             if (!q || !q->d_twp) {
