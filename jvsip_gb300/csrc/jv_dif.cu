@@ -212,8 +212,7 @@ static void *upload_tables(const std::vector<int> &rad, long N, const std::vecto
 // warp as for 32 and the pipe serves an SM's tiles one after another, so a call's
 // time is the tiles of the fullest SM times the FP64 instructions of a tile's warps
 // (of four warps at a time where an SM has one tile: its four quarters have a pipe
-// each).  Within 5 % of the times of 1751 calls, 4-8192 points, 1 to 2^23 / N rows,
-// at 0.30 ns per instruction and lane.
+// each), at 0.30 ns per instruction and lane, and 1 us a pass.
 static double f64_work(const int *rad, int np, long N, long v, bool smem, int lanes) {
     double c = 0;
     for (int i = 0; i < np; i++) {
@@ -227,44 +226,55 @@ static double f64_work(const int *rad, int np, long N, long v, bool smem, int la
 }
 static double f64_time(const int *rad, int np, long N, long v, long nvec, bool smem) {
     const long tiles = (nvec + v - 1) / v, k = (tiles + device()->sms - 1) / device()->sms;
-    return (double)k * f64_work(rad, np, N, v, smem, k > 1 ? 32 : 128);
+    double us = 0.0003 * k * f64_work(rad, np, N, v, smem, k > 1 ? 32 : 128) + 1.0 * np;
+    const int most = *std::max_element(rad, rad + np);
+    // passes of fewer than three warps leave quarters of the SM idle
+    if (!smem && k > 1 && v * (N / most) < 96) us *= 1.2;
+    if (smem && std::find(rad, rad + np, 7) != rad + np) us *= 1.4;  // 64 x 343 23.7 us, 11 here
+    return us;
 }
 
 // Transforms per tile of a double-precision row call: of the least time, in up to
-// 72 KB (three CTAs per SM), the fewest where an SM has few tiles (a tile's chain of
-// passes is shorter) and the most where it has many (381300 x 22: 16 to a tile 646
-// us, 64 to a tile 355).
+// 72 KB (three CTAs per SM).  Where several have it, the fewest if an SM has few
+// tiles (a tile's chain of passes is shorter), else the fewest that give every pass
+// four warps, one for each quarter of the SM (381300 x 22: 16 to a tile 646 us, 64 to
+// a tile 355; 103563 x 81: 32 to a tile 423, 64 to a tile 454).
 static long f64_rows_per_tile(const DifTab &t, long nvec, double *time) {
-    static const long cand[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
+    static const long cand[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 16, 20, 24, 28, 32, 40, 48, 56, 64};
+    constexpr int kCand = sizeof cand / sizeof cand[0];
     const int np = (int)t.radix.size();
     const long ldb = t.radix[0] * t.P1 * 16;
-    double best = 1e300, e[12];
+    double best = 1e300, e[kCand];
     int n = 0;
-    for (; n < 12 && (n == 0 || cand[n] * ldb <= 72 * 1024); n++) {
+    for (; n < kCand && (n == 0 || cand[n] * ldb <= 72 * 1024); n++) {
         e[n] = f64_time(t.radix.data(), np, t.N, cand[n], nvec, false);
         best = std::min(best, e[n]);
     }
-    int lo = 0, hi = n - 1;
-    while (e[lo] > 1.01 * best) lo++;
-    while (e[hi] > 1.01 * best) hi--;
-    const int pick = nvec >= 4 * cand[hi] * device()->sms ? hi : lo;
+    const long least = t.N / *std::max_element(t.radix.begin(), t.radix.end());
+    int pick = 0, last = n - 1;
+    while (e[pick] > 1.01 * best) pick++;
+    while (e[last] > 1.01 * best) last--;
+    if (nvec >= 4 * cand[last] * device()->sms)
+        while (pick < last && (cand[pick] * least < 128 || e[pick] > 1.01 * best)) pick++;
     *time = e[pick];
     return cand[pick];
 }
 
 // Whether nvec rows run on this kernel rather than the shared-memory kernel, whose
-// schedule is rad and which takes 1024 points to a CTA: by the times above, with
-// 8 % in hand (us, shared-memory kernel and this one: 2^24 points of 100 1114 and
-// 867, 600 1470 and 1184; 1000 x 216 20.2 and 23.4, 450 x 768 30.6 and 37.1 stay
-// there).  Schedules of radices 2^k do: their folded codelets take the same
-// instructions.
-static bool dif_f64_pays(const DifTab &t, const int *rad, int np, long nvec, double hand = 1.08) {
+// schedule is rad and which takes 1024 points to a CTA: where every tile has an SM,
+// or by the times above.  Of 1756 calls (4-8192 points, 1 to 2^23 / N rows) 11 are 3 %
+// or more slower than there and the average is 1.20x faster (us, there and here: 2^24
+// points of 100 1114 and 867, 600 1470 and 1184; 16 x 343 23.7 and 11.0; 1000 x 972
+// and 450 x 1620 stay there).  Schedules of radices 2^k do: their folded codelets take
+// the same instructions.
+static bool dif_f64_pays(const DifTab &t, const int *rad, int np, long nvec, double hand = 1.0) {
     bool pow2 = true;
     for (int i = 0; i < np; i++) pow2 = pow2 && (rad[i] & (rad[i] - 1)) == 0;
     if (pow2 || np < 2) return false;
     double time;
-    f64_rows_per_tile(t, nvec, &time);
-    return hand * time < f64_time(rad, np, t.N, std::max(1L, std::min(nvec, 1024 / t.N)), nvec, true);
+    const long v = f64_rows_per_tile(t, nvec, &time);
+    return (nvec + v - 1) / v <= device()->sms ||
+           hand * time < f64_time(rad, np, t.N, std::max(1L, std::min(nvec, 1024 / t.N)), nvec, true);
 }
 
 // False where the radices alone, in whatever order, show that it would not pay: a
@@ -277,23 +287,24 @@ static bool dif_f64_may_pay(long N, const std::vector<int> &smem, long nvec) {
     t.radix = least_cost(N, P_F64, 0, &cost);
     if (t.radix.empty()) return false;
     t.P1 = N / t.radix[0];
-    return dif_f64_pays(t, smem.data(), (int)smem.size(), nvec, 1.0);
+    return dif_f64_pays(t, smem.data(), (int)smem.size(), nvec, 0.95);
 }
 
 // Lengths without such a schedule (factors 11 and 13): whether `tiles` tiles of v
 // transforms run here rather than as passes over global memory, which spread a call
-// evenly over the SMs but cost 30 us and 17 us a pass at least (us, passes and here:
-// 1 x 5632 55 and 78, 64 x 6500 97 and 115, 161 x 6500 196 and 223; 150 x 6500 173
-// and 116, 16 x 2816 51 and 39).
+// evenly over the SMs but cost 30 us and 17 us a pass at least, 21 for one of 13 (us,
+// passes and here: 1 x 5632 55 and 78, 64 x 6500 97 and 115, 161 x 6500 196 and 223;
+// 150 x 6500 173 and 116, 16 x 2816 51 and 39, 16 x 2197 76 and 45).
 static bool dif_f64_beats_passes(const DifTab &t, long v, long nvec) {
     const int np = (int)t.radix.size();
-    double per = 0;
+    double per = 0, floor = 0;
     for (int i = 0; i < np; i++) {
         const int R = t.radix[i];
+        floor += R == 13 ? 21.0 : 17.0;
         per += (kDifCost[R] + 4.0 * (R - 1) / R) * (R == 11 || R == 13 ? 1.13 : 1.45);
     }
     const double passes = 0.0003 * per * t.N * nvec / device()->sms;
-    return 0.0003 * f64_time(t.radix.data(), np, t.N, v, nvec, false) < std::max(17.0 * np, 30.0 + passes);
+    return f64_time(t.radix.data(), np, t.N, v, nvec, false) < std::max(floor, 30.0 + passes);
 }
 
 // CTA shape of row calls: vpb transforms in nthr threads, chosen by the idle
