@@ -527,6 +527,7 @@ static bool upload(const BatchBuild &bb, DevBatch &db) {
                 ht[first++] = DifTile{c, (int)std::min((long)a.vpb, a.nvec - v0), v0};
         }
     }
+    if (nq + nt == 0) return true;
     db.q = (TileDesc *)dmalloc(bytes);
     if (!db.q) return false;
     db.calls = (DifArgs<float> *)((unsigned char *)db.q + oc);

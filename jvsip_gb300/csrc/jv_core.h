@@ -116,6 +116,8 @@ struct Job {
     bool no_fast = false;      // JVSIP_GPU_NO_FAST at plan creation: general kernels only
     bool no_dif = false;       // the plan's tuned schedule or shape belongs to the shared-memory kernel
     bool no_pipeline = false;  // JVSIP_GPU_NO_PIPELINE at plan creation: one staging copy each way
+    bool host = false;         // the views are host arrays
+    long dif_rows = -1, dif_rows_of = -1;  // double precision: Plan::dif_rows and the count it is for
     int tuned_vpb = 0, tuned_emax = 0;  // the plan's tuned shared-memory kernel shape (0: automatic)
     int tma_columns = -1;      // JVSIP_GPU_TMA_COLUMNS at plan creation: 1 / 0 force TMA-staged
                                // column tiles on / off, -1 (unset) automatic
@@ -222,6 +224,9 @@ std::vector<double> unit_roots(long N);  // exp(-2 pi i m/N), m < N, (re, im) pa
 // other: double precision, the shared-memory kernel's schedule to be better than on nvec rows (or null)
 const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *roots, const std::vector<int> *other,
                           long nvec);
+// double precision: transforms per tile of nvec rows, 0 where they run on the shared-
+// memory kernel (schedule rad) or, without one (rad null), as global passes
+long dif_f64_rows(const DifTab &t, const int *rad, int np, long nvec);
 void dif_release(const DifTab *t);
 bool launch_dif_f32(const Job &j, cudaStream_t s);  // false when the call does not qualify
 bool launch_dif_f64(const Job &j, cudaStream_t s);
@@ -296,6 +301,7 @@ struct Plan {
     void *d_pc = nullptr;     // per-pass constants of that schedule (PassConst, one per pass)
     void *d_twdd = nullptr;   // per-pass double-float tables of the FP64 form (built by setform_d)
     const DifTab *dif = nullptr;  // the in-place mixed-radix kernel's schedule and tables (or null)
+    long dif_rows = -1;       // double precision: its transforms per tile for mN rows, 0: another kernel's
     std::vector<unsigned long> jofk;  // reference digit-reversal map (kept for parity checks)
     std::vector<CallGraph> graphs;    // captured calls (ntimes == 0), most recent last
     bool single = false;      // a single-FFT plan (vsip_fft_*: one row, vector views)

@@ -224,8 +224,8 @@ static double f64_work(const int *rad, int np, long N, long v, bool smem, int la
     }
     return c;
 }
-static double f64_time(const int *rad, int np, long N, long v, long nvec, bool smem) {
-    const long tiles = (nvec + v - 1) / v, k = (tiles + device()->sms - 1) / device()->sms;
+static double f64_time(const int *rad, int np, long N, long v, long nvec, bool smem, long sms) {
+    const long tiles = (nvec + v - 1) / v, k = (tiles + sms - 1) / sms;
     double us = 0.0003 * k * f64_work(rad, np, N, v, smem, k > 1 ? 32 : 128) + 1.0 * np;
     const int most = *std::max_element(rad, rad + np);
     // passes of fewer than three warps leave quarters of the SM idle
@@ -243,38 +243,39 @@ static long f64_rows_per_tile(const DifTab &t, long nvec, double *time) {
     static const long cand[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 16, 20, 24, 28, 32, 40, 48, 56, 64};
     constexpr int kCand = sizeof cand / sizeof cand[0];
     const int np = (int)t.radix.size();
-    const long ldb = t.radix[0] * t.P1 * 16;
+    const long ldb = t.radix[0] * t.P1 * 16, sms = device()->sms;
     double best = 1e300, e[kCand];
     int n = 0;
     for (; n < kCand && (n == 0 || cand[n] * ldb <= 72 * 1024); n++) {
-        e[n] = f64_time(t.radix.data(), np, t.N, cand[n], nvec, false);
+        e[n] = f64_time(t.radix.data(), np, t.N, cand[n], nvec, false, sms);
         best = std::min(best, e[n]);
     }
     const long least = t.N / *std::max_element(t.radix.begin(), t.radix.end());
     int pick = 0, last = n - 1;
     while (e[pick] > 1.01 * best) pick++;
     while (e[last] > 1.01 * best) last--;
-    if (nvec >= 4 * cand[last] * device()->sms)
+    if (nvec >= 4 * cand[last] * sms)
         while (pick < last && (cand[pick] * least < 128 || e[pick] > 1.01 * best)) pick++;
     *time = e[pick];
     return cand[pick];
 }
 
-// Whether nvec rows run on this kernel rather than the shared-memory kernel, whose
-// schedule is rad and which takes 1024 points to a CTA: where every tile has an SM,
+// The tile of nvec rows, 0 where they run on the shared-memory kernel, whose schedule
+// is rad and which takes 1024 points to a CTA: on this one where every tile has an SM,
 // or by the times above.  Of 1756 calls (4-8192 points, 1 to 2^23 / N rows) 11 are 3 %
 // or more slower than there and the average is 1.20x faster (us, there and here: 2^24
 // points of 100 1114 and 867, 600 1470 and 1184; 16 x 343 23.7 and 11.0; 1000 x 972
 // and 450 x 1620 stay there).  Schedules of radices 2^k do: their folded codelets take
 // the same instructions.
-static bool dif_f64_pays(const DifTab &t, const int *rad, int np, long nvec, double hand = 1.0) {
+static long f64_rows_or_smem(const DifTab &t, const int *rad, int np, long nvec, double hand = 1.0) {
     bool pow2 = true;
     for (int i = 0; i < np; i++) pow2 = pow2 && (rad[i] & (rad[i] - 1)) == 0;
-    if (pow2 || np < 2) return false;
+    if (pow2 || np < 2) return 0;
     double time;
-    const long v = f64_rows_per_tile(t, nvec, &time);
-    return (nvec + v - 1) / v <= device()->sms ||
-           hand * time < f64_time(rad, np, t.N, std::max(1L, std::min(nvec, 1024 / t.N)), nvec, true);
+    const long v = f64_rows_per_tile(t, nvec, &time), sms = device()->sms;
+    const bool pays = (nvec + v - 1) / v <= sms ||
+                      hand * time < f64_time(rad, np, t.N, std::max(1L, std::min(nvec, 1024 / t.N)), nvec, true, sms);
+    return pays ? v : 0;
 }
 
 // False where the radices alone, in whatever order, show that it would not pay: a
@@ -287,7 +288,7 @@ static bool dif_f64_may_pay(long N, const std::vector<int> &smem, long nvec) {
     t.radix = least_cost(N, P_F64, 0, &cost);
     if (t.radix.empty()) return false;
     t.P1 = N / t.radix[0];
-    return dif_f64_pays(t, smem.data(), (int)smem.size(), nvec, 0.95);
+    return f64_rows_or_smem(t, smem.data(), (int)smem.size(), nvec, 0.95) > 0;
 }
 
 // Lengths without such a schedule (factors 11 and 13): whether `tiles` tiles of v
@@ -303,8 +304,16 @@ static bool dif_f64_beats_passes(const DifTab &t, long v, long nvec) {
         floor += R == 13 ? 21.0 : 17.0;
         per += (kDifCost[R] + 4.0 * (R - 1) / R) * (R == 11 || R == 13 ? 1.13 : 1.45);
     }
-    const double passes = 0.0003 * per * t.N * nvec / device()->sms;
-    return f64_time(t.radix.data(), np, t.N, v, nvec, false) < std::max(floor, 30.0 + passes);
+    const long sms = device()->sms;
+    const double passes = 0.0003 * per * t.N * nvec / sms;
+    return f64_time(t.radix.data(), np, t.N, v, nvec, false, sms) < std::max(floor, 30.0 + passes);
+}
+
+long dif_f64_rows(const DifTab &t, const int *rad, int np, long nvec) {
+    if (rad) return f64_rows_or_smem(t, rad, np, nvec);
+    double time;
+    const long v = f64_rows_per_tile(t, nvec, &time);
+    return dif_f64_beats_passes(t, v, nvec) ? v : 0;
 }
 
 // CTA shape of row calls: vpb transforms in nthr threads, chosen by the idle
@@ -387,7 +396,7 @@ const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *
     auto key = std::make_tuple(N, prec, cls);
     auto it = g_dif.find(key);
     if (it != g_dif.end()) {
-        if (other && !dif_f64_pays(it->second, other->data(), (int)other->size(), nvec)) return nullptr;
+        if (other && !f64_rows_or_smem(it->second, other->data(), (int)other->size(), nvec)) return nullptr;
         it->second.refs++;
         return &it->second;
     }
@@ -411,7 +420,7 @@ const DifTab *dif_acquire(long N, int prec, int cls, const std::vector<double> *
         if (seen->second.radix.empty()) return nullptr;  // no schedule
         t = seen->second;
     }
-    if (other && !dif_f64_pays(t, other->data(), (int)other->size(), nvec)) return nullptr;
+    if (other && !f64_rows_or_smem(t, other->data(), (int)other->size(), nvec)) return nullptr;
     const int err0 = jvsip_gpu_last_error();
     std::vector<double> own;
     if (!roots) {
@@ -536,10 +545,12 @@ static bool dif_args(const Job &j, long tuned, long sms, bool narrow, DifArgs<T>
     const size_t cap = device()->smem_optin;
     long vpb, nthr;
     if (rows && sizeof(T) == 8) {
-        double time;
-        vpb = f64_rows_per_tile(*t, j.nvec, &time);
+        vpb = j.nvec == j.dif_rows_of ? j.dif_rows : dif_f64_rows(*t, j.twg ? j.radix : nullptr, j.npass, j.nvec);
+        if (vpb < 1) return false;
+        // rows on the host arrays: more, smaller CTAs keep the link busy (1000 x 1000 168
+        // us, 196 with the tile of device rows)
+        while (j.host && vpb > 1 && (j.nvec + vpb - 1) / vpb < 2L * sms) vpb = (vpb + 1) / 2;
         nthr = std::min(256L, (vpb * j.N / *std::min_element(t->radix.begin(), t->radix.end()) + 31) / 32 * 32);
-        if (j.twg ? !dif_f64_pays(*t, j.radix, j.npass, j.nvec) : !dif_f64_beats_passes(*t, vpb, j.nvec)) return false;
     } else if (rows) {
         vpb = t->vpb;
         nthr = t->nthr;

@@ -788,6 +788,8 @@ static void fill_job(Job &j, const Plan *p, int kind) {
     j.pc = p->d_pc;
     j.twdd = p->d_twdd;
     j.dif = p->dif;
+    j.dif_rows = p->dif_rows;
+    j.dif_rows_of = p->mN;
     j.no_dif = p->no_dif;
     j.form = p->form;
     j.no_fast = p->no_fast;
@@ -813,7 +815,10 @@ static bool host_direct(const Staging &s, const Job &j, const Geo &in, const Geo
     if (s.regs.empty() || j.no_pipeline || j.form > JVSIP_FORM_PLAIN || in.es != 1 || out.es != 1) return false;
     if (j.lp || !(job_in_smem(j) || (j.dif && !j.no_fast && !j.no_dif && j.N > 1))) return false;
     const size_t moved = (size_t)j.N * j.nvec * (j.prec == P_F32 ? 16 : 32);
-    if (!host_rows_pay(j.N, in.len, in.vs, j.nvec, j.prec != P_F32, moved)) return false;
+    size_t staged = 0;  // in, and out again what is written
+    for (const Region &r : s.regs) staged += s.bytes(r) * (r.h_im ? 2 : 1) * ((r.read ? 1 : 0) + (r.write ? 1 : 0));
+    const int kind = j.kind == K_R2C ? 1 : j.kind == K_C2R ? 2 : 0;
+    if (!host_rows_pay(kind, j.N, in.len, in.vs, j.nvec, j.prec != P_F32, moved, staged)) return false;
     if (!s.inside || !s.apart() || !host_access()) return false;
     g_host_direct.fetch_add(1, std::memory_order_relaxed);
     return true;
@@ -934,6 +939,7 @@ static void exec_cc(Plan *p, const CMV *x, const CMV *y, bool ip) {
     stage_c(stg, rx, true, same_view);
     if (!same_view) stage_c(stg, ry, !ry.g.dense() || (y->block == x->block), true);
     stg.direct = (same_view || x->block != y->block) && host_direct(stg, j, rx.g, ry.g);
+    j.host = stg.direct;
     if (!stg.upload(st)) return;
     j.cin = dev_c(stg, rx);
     j.cout = same_view ? j.cin : dev_c(stg, ry);
@@ -1041,6 +1047,7 @@ static void exec_rc(Plan *p, const RMV *x, const CMV *z) {
     stage_r(stg, rx, true, false);
     stage_c(stg, rz, !rz.g.dense(), true);
     stg.direct = host_direct(stg, j, rx.g, rz.g);
+    j.host = stg.direct;
     if (!stg.upload(st)) return;
     j.rin = dev_r(stg, rx);
     j.cout = dev_c(stg, rz);
@@ -1077,6 +1084,7 @@ static void exec_cr(Plan *p, const CMV *z, const RMV *x) {
     stage_c(stg, rz, true, false);
     stage_r(stg, rx, !rx.g.dense(), true);
     stg.direct = host_direct(stg, j, rz.g, rx.g);
+    j.host = stg.direct;
     if (!stg.upload(st)) return;
     j.cin = dev_c(stg, rz);
     j.rout = dev_r(stg, rx);

@@ -279,6 +279,8 @@ static bool build_tables(Plan *p, const std::vector<double> &roots);
 static void take_dif(Plan *p, const std::vector<double> *roots) {
     p->dif = dif_acquire(p->MN, p->prec, table_kind(p->type), roots,
                          p->prec == P_F64 && p->smooth ? &p->radix : nullptr, p->mN);
+    if (p->prec == P_F64 && p->dif)
+        p->dif_rows = dif_f64_rows(*p->dif, p->smooth ? p->radix.data() : nullptr, (int)p->radix.size(), p->mN);
 }
 
 template <typename T>

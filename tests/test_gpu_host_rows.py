@@ -1,7 +1,7 @@
 """Which calls on host blocks run on the host arrays themselves: long rows and small
-calls do (where the GPU reaches pageable memory through the host's page tables),
-many short rows, rows that overlap in bulk, unaligned and overlapping arrays keep
-the copies -- and every call's result matches numpy in 64 bits (rel-L2 1e-6 log2 N,
+calls do (where the GPU reaches pageable memory through the host's page tables), and
+pitched rows; many short rows, rows that overlap in bulk, unaligned and overlapping
+arrays keep the copies -- and every call's result matches numpy in 64 bits (rel-L2 1e-6 log2 N,
 double 1e-14 log2 N)."""
 import numpy as np
 import pytest
@@ -40,10 +40,11 @@ def run(N, m, dtype=np.float32, pitch=None, skew=0):
 
 @pytest.mark.parametrize("N,m,dtype,pitch,skew,direct", [
     (1000, 256, np.float32, None, 0, 1), (200, 20000, np.float32, None, 0, 1), (64, 1000, np.float32, None, 0, 1),
-    (64, 20000, np.float32, None, 0, 0), (128, 1024, np.float32, None, 0, 1), (128, 1025, np.float32, None, 0, 0),
+    (64, 20000, np.float32, None, 0, 0), (128, 4096, np.float32, None, 0, 1), (128, 4097, np.float32, None, 0, 0),
     (16, 4096, np.float64, None, 0, 1), (16, 4097, np.float64, None, 0, 0), (24, 20000, np.float64, None, 0, 1),
-    (1000, 200, np.float32, 250, 0, 1), (1000, 400, np.float32, 250, 0, 0), (8, 20000, np.float32, 2, 0, 0),
-    (1000, 256, np.float32, None, 1, 0), (1500, 40, np.float64, 1502, 0, 1)])
+    (1000, 400, np.float32, 250, 0, 1), (1000, 530, np.float32, 250, 0, 0),
+    (960, 700, np.float32, 240, 0, 1), (8, 20000, np.float32, 2, 0, 0),
+    (64, 20000, np.float32, 256, 0, 1), (1000, 256, np.float32, None, 1, 0), (1500, 40, np.float64, 1502, 0, 1)])
 def test_route_and_result(N, m, dtype, pitch, skew, direct):
     if not host_access():
         direct = 0
