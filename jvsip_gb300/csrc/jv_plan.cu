@@ -312,6 +312,17 @@ static bool make_tables(Plan *p) {
     return true;
 }
 
+// Gathered tables (build_tables) lie inside d_tw's buffer, which goes back last: while
+// it is the plan's, no pointer into it can be another thread's new buffer, and dfree
+// passes over it.
+static void free_tables(Plan *p) {
+    dfree(p->d_thalf);
+    dfree(p->d_twp);
+    dfree(p->d_twg);
+    dfree(p->d_pc);
+    dfree(p->d_tw);
+}
+
 static void release_tables(Plan *p) {
     dif_release(p->dif);
     p->dif = nullptr;
@@ -322,11 +333,7 @@ static void release_tables(Plan *p) {
         if (--it->second.refs > 0) return;
         g_tabs.erase(it);
     }
-    dfree(p->d_tw);
-    dfree(p->d_thalf);
-    dfree(p->d_twp);
-    dfree(p->d_twg);
-    dfree(p->d_pc);
+    free_tables(p);
 }
 
 template <typename T>
@@ -440,11 +447,7 @@ static Plan *step_plan(long n, int prec) {
     q->radix = pass_radices(n, &q->smooth, prec == P_F32 ? 1024 : 512);
     if (!q->smooth || q->radix.empty() || !make_tables<T>(q)) {
         if (q->smooth && !q->radix.empty()) {
-            dfree(q->d_tw);
-            dfree(q->d_thalf);
-            dfree(q->d_twp);
-            dfree(q->d_twg);
-            dfree(q->d_pc);
+            free_tables(q);
         }
         delete q;
         return nullptr;
@@ -689,11 +692,7 @@ static Plan *new_plan(int type, vsip_length M, vsip_length N, double scale, int 
         for (long i = 0; i < p->MN; i++) p->jofk[i] = ref_jofk((unsigned long)i, pn, p0, pF[ns - 1], ns);
     }
     if (!make_tables<T>(p)) {
-        dfree(p->d_tw);
-        dfree(p->d_thalf);
-        dfree(p->d_twp);
-        dfree(p->d_twg);
-        dfree(p->d_pc);
+        free_tables(p);
         delete p;
         return nullptr;
     }
