@@ -428,9 +428,9 @@ __device__ __forceinline__ void dif_last_r2c(const DifArgs<T> &a, const typename
         case 16: CALL(16); break;    \
         case 15: CALL(15); break;    \
         case 14: CALL(14); break;    \
-        case 13: CALL(13); break;    \
+        case 13: if constexpr (P13) CALL(13); break; \
         case 12: CALL(12); break;    \
-        case 11: CALL(11); break;    \
+        case 11: if constexpr (P13) CALL(11); break; \
         case 10: CALL(10); break;    \
         case 9: CALL(9); break;      \
         case 8: CALL(8); break;      \
@@ -457,8 +457,13 @@ constexpr int kDifPairMax = 10;
         default: CALL(2); break;      \
     }
 
-// The passes of one CTA's transforms.
-template <typename T, int KIND, bool COLS>
+// The passes of one CTA's transforms.  P13: with the codelets 11 and 13, which the
+// lengths of batches and k-omega (2^a 3^b 5^c 7^d) do not reach.  Without them the
+// batch kernels spill 156 and 296 bytes (208 and 384 with; a batch of 60 calls 143 us,
+// 149, of 160 538 and 544).  k-omega's kernels keep them: without, the tapered rows
+// spill less (4 bytes, 88) but 343 sensors x 2058 samples take 20.4 us (17.9), and the
+// power columns spill more (556, 464; 448 x 2800 22.0 us, 21.1).
+template <typename T, int KIND, bool COLS, bool P13>
 __device__ __forceinline__ void dif_passes(const DifArgs<T> &a, typename cplx_t<T>::t *s, int nt, long v0) {
     typedef DifDyn SC;
     if constexpr (KIND == DIF_C2R) {
@@ -522,7 +527,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_dif(const __gri
     const long v0 = (long)blockIdx.x * a.vpb;
     const int nt = (int)min((long)a.vpb, a.nvec - v0);
     dif_prologue<T, KIND>(a, s, v0);
-    dif_passes<T, KIND, COLS>(a, s, nt, v0);
+    dif_passes<T, KIND, COLS, true>(a, s, nt, v0);
 }
 
 // The same with a schedule known at compile time, in CTAs of NT threads of
@@ -558,7 +563,7 @@ __global__ void __launch_bounds__(1024) k_dif_batch(const DifArgs<float> *__rest
         reinterpret_cast<unsigned long long *>(&a)[i] =
             __ldg(reinterpret_cast<const unsigned long long *>(&calls[d.call]) + i);
     __syncthreads();
-    dif_passes<float, DIF_C2C, COLS>(a, s, d.nt, d.v0);
+    dif_passes<float, DIF_C2C, COLS, false>(a, s, d.nt, d.v0);
 }
 
 // static shared memory of k_dif_batch (the copied arguments), rounded up
