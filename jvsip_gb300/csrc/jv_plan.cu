@@ -342,10 +342,12 @@ static bool build_tables(Plan *p, const std::vector<double> &roots) {
     size_t n = (size_t)(MN > 0 ? MN : 1);
     std::vector<T> tw(2 * n, (T)0);
     for (long m = 0; m < 2 * MN; m++) tw[m] = (T)roots[m];
-    // tables of up to 64K points go to one buffer in one copy (d_tw is its start, the
+    // tables of up to 1024 points go to one buffer in one copy (d_tw is its start, the
     // only one to be freed): a copy of its own for each was a third of a small plan's
-    // making (16 points 21 us, 31 with the in-place kernel's table as a fifth copy)
-    const bool gather = n <= 65536;
+    // making (16 points 21 us, 31 with the in-place kernel's table as a fifth copy).
+    // Longer plans keep a buffer for each (2400 points 121 us, 105 gathered): with the
+    // tables elsewhere 6001 x 2400 in place took 0.2 to 2.5 % longer, by where its data lay
+    const bool gather = n <= 1024;
     std::vector<unsigned char> host;
     std::vector<std::pair<void **, size_t>> at;
     auto put = [&](void **dst, const void *src, size_t bytes) -> bool {
